@@ -661,7 +661,7 @@ int grid_reserve(Grid& g, int capacity)
     g.keys_a = g.vals_a = g.keys_b = g.vals_b = g.point_cells = g.point_ids = nullptr;
     g.hist = nullptr;
     g.capacity = 0;
-    const size_t sz = sizeof(int) * (size_t)capacity;
+    const size_t sz = sizeof(int) * (size_t)capacity + 1024;  // the raycast's tree nodes round up past n ints
     cudaError_t e = cudaSuccess;
     if (e == cudaSuccess) e = cudaMalloc(&g.keys_a, sz);
     if (e == cudaSuccess) e = cudaMalloc(&g.vals_a, sz);
@@ -753,6 +753,27 @@ int build_passes(Grid& g, const float* points, int n, float cell_inv, const Gath
     return NSPH_OK;
 }
 
+template <int kItems>
+int sort_keys(Grid& g, int n, int bits, cudaStream_t stream)
+{
+    const int ntiles = ntiles_of(n, kItems);
+    unsigned* digit_tot = g.hist + (size_t)kRadix * hist_tiles(g.capacity);
+    int *kin = g.keys_a, *vin = g.vals_a, *kout = g.keys_b, *vout = g.vals_b;
+    for (int shift = 0; shift < bits; shift += kRadixBits) {
+        const int mask = (1 << std::min(kRadixBits, bits - shift)) - 1;
+        k_upsweep<kItems><<<ntiles, kSortThreads, 0, stream>>>(kin, n, shift, mask, g.hist, ntiles);
+        NSPH_LAUNCH_CHECK("k_upsweep");
+        k_scan_rows<<<kRadix, kScanThreads, 0, stream>>>(g.hist, ntiles, digit_tot);
+        NSPH_LAUNCH_CHECK("k_scan_rows");
+        k_downsweep<false, kItems><<<ntiles, kSortThreads, sizeof(DownsweepSmem<kItems>), stream>>>(
+            kin, vin, kout, vout, n, shift, mask, g.hist, ntiles, digit_tot, GatherArgs{});
+        NSPH_LAUNCH_CHECK("k_downsweep");
+        std::swap(kin, kout);
+        std::swap(vin, vout);
+    }
+    return NSPH_OK;
+}
+
 // the counting build (see k_cc_count): 5 launches
 int count_build(Grid& g, const float* points, int n, float cell_inv, const GatherArgs* gather, unsigned int* status,
                 cudaStream_t stream, int& nl, int prev_n)
@@ -778,6 +799,14 @@ int count_build(Grid& g, const float* points, int n, float cell_inv, const Gathe
 }
 
 }  // namespace
+
+int grid_sort_keys(Grid& g, int n, int bits, cudaStream_t stream)
+{
+    if (n > g.capacity) return fail(NSPH_ERR_CAPACITY, "sort: more keys than reserved");
+    if (n <= 0) return NSPH_OK;
+    return items_for(n) == kSmallItems ? sort_keys<kSmallItems>(g, n, bits, stream)
+                                       : sort_keys<kSortItems>(g, n, bits, stream);
+}
 
 int grid_build(Grid& g, const float* points, int n, float cell_width, float cell_inv, const GatherArgs* gather,
                unsigned int* status, cudaStream_t stream, int* launches, const int* world)
@@ -859,7 +888,7 @@ extern "C" int nsph_grid_reserve(nsph_grid* grid, int num_points)
     grid->mirror = nullptr;
     grid->mirror_cap = 0;
     const size_t c = (size_t)std::max(1, grid->g.capacity);
-    if (cudaMalloc(&grid->mirror, sizeof(float4) * 2 * c) != cudaSuccess) {
+    if (cudaMalloc(&grid->mirror, mirror_bytes((int)c)) != cudaSuccess) {
         cudaGetLastError();
         grid->mirror = nullptr;
         return fail(NSPH_ERR_OUT_OF_MEMORY, "grid reserve: contact mirror allocation failed");

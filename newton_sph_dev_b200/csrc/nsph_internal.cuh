@@ -311,11 +311,23 @@ void grid_free(Grid& g);
 int grid_build(Grid& g, const float* points, int n, float cell_width, float cell_inv, const GatherArgs* gather,
                unsigned int* status, cudaStream_t stream, int* launches = nullptr, const int* world = nullptr);
 
+// Sorts the n (key, value) pairs in keys_a / vals_a by the low `bits` bits of
+// the keys (stable; the grid's build scratch, free between builds). `bits` of
+// an odd number of 8-bit digits: the result is in keys_b / vals_b.
+int grid_sort_keys(Grid& g, int n, int bits, cudaStream_t stream);
+
 }  // namespace nsph
 
 // the opaque handle of the nsph_grid_* C ABI (a HashGrid object)
 struct nsph_grid {
     nsph::Grid g;
-    float4* mirror = nullptr;  // contact scratch: 2 x mirror_cap sorted float4 ((x, r), (v, inv_mass))
+    // scratch of the contact and raycast kernels: 2 x mirror_cap sorted float4
+    // ((x, r), (v, inv_mass); or the spheres in grid and in tree order), then
+    // the raycast's bounds
+    float4* mirror = nullptr;
     int mirror_cap = 0;
 };
+
+namespace nsph {
+constexpr size_t mirror_bytes(int capacity) { return sizeof(float4) * 2 * (size_t)capacity + 256; }
+}  // namespace nsph

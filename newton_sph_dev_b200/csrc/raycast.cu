@@ -7,22 +7,35 @@
 // ray_intersect_particle_sphere (raycast.py:123-156), and the final
 // clamp_no_hits_kernel (sensor_raycast.py:18-23).
 //
-// One thread per pixel marches its ray from the camera in steps of
+// Reference semantics: each pixel marches its ray from the camera in steps of
 // march_step. At every sample it queries the grid (Warp's query box around
-// the sample, radius search_radius) and intersects the ray with the sphere
-// of every candidate, keeping the nearest hit; it stops after max_steps
-// samples, beyond max_distance, or beyond the nearest hit so far. The depth
-// is the minimum over the candidates of the samples taken, which does not
-// depend on the order they are tested in.
+// the sample, radius search_radius) and intersects the ray with the sphere of
+// every candidate, keeping the nearest hit; it stops after max_steps samples,
+// beyond max_distance, or beyond the nearest hit so far. The depth is the
+// minimum over the candidates of the samples taken, which does not depend on
+// the order they are tested in.
 //
-// Each cell is tested once per ray. Along every axis the sample coordinate
-// is monotone in t, and so are both ends of the query box, so a cell of this
-// sample's box that was in any earlier box was in the previous one. The
-// cells of the box that the previous box did not hold are therefore exactly
-// the cells no earlier sample tested; testing only those gives the same
-// running minimum after every sample, hence the same samples and the same
-// result as the reference's per-sample query, at about a sixth of the cell
-// visits for a march step of half a cell.
+// Two facts make most of the march unnecessary:
+// 1. Every hit is at least M, the nearest computed hit over ALL spheres. A
+//    ray without any computed hit leaves its pixel as it is, whatever cells
+//    its march would visit. M comes from a bounding-box tree over the spheres
+//    (k_ray_leaves, k_ray_upper), whose boxes are inflated by a bound on the
+//    rounding of the sphere test, so it misses no computed hit.
+// 2. Every sample with t <= M is taken (nothing stops the march before). So
+//    when the box of such a sample holds the nearest sphere's cell, the depth
+//    is M. Otherwise the march is run, but only over the samples whose box
+//    overlaps (modulo the grid's dims) the cells that can hold a sphere hit
+//    before M + window: spheres hit later cannot stop the march inside the
+//    window, and those that can are tested at these samples only. A march
+//    that leaves the window without a hit is repeated with a wider one, in
+//    the end the reference's whole march.
+// The march itself tests each cell once per ray: along every axis both ends
+// of the query box are monotone in t, so a cell that an earlier sample tested
+// and that this box still holds was in the previous box.
+//
+// The march alone was bound by instruction issue: most rays miss, and each
+// missing ray took every sample up to max_distance through cells that the
+// grid's 128 cells per axis alias onto the scene.
 //
 // fp32, every operation rounded as written (explicit _rn intrinsics, dot
 // products ((x + y) + z)), so the depth image matches the CPU restatement
@@ -36,22 +49,210 @@ namespace nsph {
 NSPH_BOUNDS_READER(raycast)
 namespace {
 
-constexpr int kRayTileX = 32;  // a warp: 32 consecutive pixels of a row
-constexpr int kRayTileY = 4;
-
 __device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, float by, float bz)
 {
     return __fadd_rn(__fadd_rn(__fmul_rn(ax, bx), __fmul_rn(ay, by)), __fmul_rn(az, bz));
 }
 
-// sorted mirror (x, y, z, radius) of the grid's points
+// float -> unsigned, increasing, 0 below every float (the bounds start at 0)
+__device__ __forceinline__ unsigned ordered(float f)
+{
+    const unsigned u = __float_as_uint(f);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+
+__device__ __forceinline__ float unordered(unsigned u)
+{
+    return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
+}
+
+// Radius that bounds the centres of spheres whose COMPUTED test can hit,
+// around the ray, at distances up to d from the camera: the discriminant
+// proj^2 - (|o|^2 - r^2) carries at most 20 roundings (2^-24) of d^2, the
+// direction's length included; 2^-18 (64 roundings) is taken.
+__device__ __forceinline__ float reach(float r, float d) { return sqrtf(fmaf(3.8147e-6f * d, d, r * r)) * 1.0001f; }
+
+// whether sphere q can be hit within max_distance of the camera at all (its
+// coordinates and radius finite, the radius positive)
+__device__ __forceinline__ bool in_reach(float4 q, const nsph_raycast_camera& c)
+{
+    if (!(q.w > 0.f && isfinite(q.w) && fabsf(q.x) < 1e18f && fabsf(q.y) < 1e18f && fabsf(q.z) < 1e18f)) return false;
+    const float ox = q.x - c.position[0], oy = q.y - c.position[1], oz = q.z - c.position[2];
+    const float d = sqrtf(ox * ox + oy * oy + oz * oz);
+    return !(d * 0.99999f - reach(q.w, d) > c.max_distance);
+}
+
+// sorted mirror (x, y, z, radius) of the grid's points, and the bounds of the
+// spheres in reach: bounds[a] = max of ordered(x_a), bounds[3 + a] = max of
+// ordered(-x_a), both 0 at first
 __global__ void k_raycast_gather(const int* __restrict__ ids, const float* __restrict__ x,
-                                 const float* __restrict__ radius, int n, float4* __restrict__ m)
+                                 const float* __restrict__ radius, int n, const nsph_raycast_camera cam,
+                                 float4* __restrict__ m, unsigned* __restrict__ bounds)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned b[6] = {0u, 0u, 0u, 0u, 0u, 0u};
+    if (k < n) {
+        const size_t i = (size_t)ids[k];
+        const float4 q = make_float4(x[3 * i], x[3 * i + 1], x[3 * i + 2], radius[i]);
+        m[k] = q;
+        if (in_reach(q, cam)) {
+            b[0] = ordered(q.x);
+            b[1] = ordered(q.y);
+            b[2] = ordered(q.z);
+            b[3] = ordered(-q.x);
+            b[4] = ordered(-q.y);
+            b[5] = ordered(-q.z);
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < 6; ++a) {
+        const unsigned v = __reduce_max_sync(0xffffffffu, b[a]);
+        if ((threadIdx.x & 31) == a && v > bounds[a]) atomicMax(bounds + a, v);
+    }
+}
+
+__device__ __forceinline__ unsigned spread8(unsigned v)  // bits 0..7 to bits 0, 3, .., 21
+{
+    v = (v | (v << 8)) & 0x00f00fu;
+    v = (v | (v << 4)) & 0x0c30c3u;
+    return (v | (v << 2)) & 0x249249u;
+}
+
+// 24-bit Morton key of each sphere inside the bounds (spheres out of reach
+// last), and its position in the sorted mirror
+__global__ void k_ray_keys(const float4* __restrict__ m, int n, const nsph_raycast_camera cam,
+                           const unsigned* __restrict__ bounds, int* __restrict__ keys, int* __restrict__ vals)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    const size_t i = (size_t)ids[k];
-    m[k] = make_float4(x[3 * i], x[3 * i + 1], x[3 * i + 2], radius[i]);
+    const float4 q = m[k];
+    unsigned key = 0xffffffu;
+    if (in_reach(q, cam)) {
+        const float lo[3] = {-unordered(bounds[3]), -unordered(bounds[4]), -unordered(bounds[5])};
+        const float x[3] = {q.x, q.y, q.z};
+        float ext = 0.f;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) ext = fmaxf(ext, unordered(bounds[a]) - lo[a]);
+        const float scale = ext > 0.f ? 255.f / ext : 0.f;
+        key = 0u;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) key |= spread8((unsigned)min(255, max(0, (int)((x[a] - lo[a]) * scale)))) << a;
+    }
+    keys[k] = (int)key;
+    vals[k] = k;
+}
+
+// ---- the tree: nodes of eight consecutive children, leaves of eight spheres -----
+// A node is two float4: (min of the centres, largest radius), (max of the
+// centres, -); an empty one has min > max. Level 0 (the leaves) lies in its
+// own array, the levels above it one after another in `upper`.
+constexpr int kRayArity = 8;
+constexpr int kRayLevels = 12;
+
+struct RayTree {
+    float4* leaves;
+    float4* upper;
+    int levels;                // level levels - 1 holds one node
+    int count[kRayLevels];     // nodes per level
+    int offset[kRayLevels];    // first node of a level >= 1 in `upper`
+    __host__ __device__ float4* node(int level, int i) const
+    {
+        return level == 0 ? leaves + 2 * (size_t)i : upper + 2 * ((size_t)offset[level] + i);
+    }
+};
+
+struct RayBox {
+    float lo[3], hi[3], r;
+};
+
+__device__ __forceinline__ RayBox empty_box()
+{
+    RayBox b;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        b.lo[a] = INFINITY;
+        b.hi[a] = -INFINITY;
+    }
+    b.r = 0.f;
+    return b;
+}
+
+// union over the eight lanes of an aligned group, in every lane of it
+__device__ __forceinline__ RayBox join8(RayBox b)
+{
+#pragma unroll
+    for (int o = 1; o < kRayArity; o <<= 1) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            b.lo[a] = fminf(b.lo[a], __shfl_xor_sync(0xffffffffu, b.lo[a], o));
+            b.hi[a] = fmaxf(b.hi[a], __shfl_xor_sync(0xffffffffu, b.hi[a], o));
+        }
+        b.r = fmaxf(b.r, __shfl_xor_sync(0xffffffffu, b.r, o));
+    }
+    return b;
+}
+
+__device__ __forceinline__ void store_box(float4* node, const RayBox& b)
+{
+    node[0] = make_float4(b.lo[0], b.lo[1], b.lo[2], b.r);
+    node[1] = make_float4(b.hi[0], b.hi[1], b.hi[2], 0.f);
+}
+
+// the spheres in Morton order (radius -1 out of reach) and the leaves
+__global__ void __launch_bounds__(256) k_ray_leaves(const float4* __restrict__ m, const int* __restrict__ order,
+                                                    int n, const nsph_raycast_camera cam, float4* __restrict__ sorted,
+                                                    const __grid_constant__ RayTree tree)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    RayBox b = empty_box();
+    if (k < n) {
+        float4 q = m[order[k]];
+        if (in_reach(q, cam)) {
+            b.lo[0] = b.hi[0] = q.x;
+            b.lo[1] = b.hi[1] = q.y;
+            b.lo[2] = b.hi[2] = q.z;
+            b.r = q.w;
+        } else {
+            q.w = -1.f;
+        }
+        sorted[k] = q;
+    }
+    b = join8(b);
+    if (k < n && (threadIdx.x & (kRayArity - 1)) == 0) store_box(tree.node(0, k / kRayArity), b);
+}
+
+// levels 1 .. levels - 1, each from the one below
+__global__ void __launch_bounds__(256) k_ray_upper(const __grid_constant__ RayTree tree, int level)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;  // child
+    RayBox b = empty_box();
+    if (i < tree.count[level - 1]) {
+        const float4* c = tree.node(level - 1, i);
+        const float4 lo = c[0], hi = c[1];
+        b = RayBox{{lo.x, lo.y, lo.z}, {hi.x, hi.y, hi.z}, lo.w};
+    }
+    b = join8(b);
+    if (i < tree.count[level - 1] && (threadIdx.x & (kRayArity - 1)) == 0) store_box(tree.node(level, i / kRayArity), b);
+}
+
+// the levels from `first` up, in one block (the first has at most 256 x 8 children)
+__global__ void __launch_bounds__(1024) k_ray_top(const __grid_constant__ RayTree tree, int first)
+{
+    for (int level = first; level < tree.levels; ++level) {
+        const int children = tree.count[level - 1];
+        for (int base = 0; base < children; base += blockDim.x) {
+            const int i = base + threadIdx.x;
+            RayBox b = empty_box();
+            if (i < children) {
+                const float4* c = tree.node(level - 1, i);
+                const float4 lo = c[0], hi = c[1];
+                b = RayBox{{lo.x, lo.y, lo.z}, {hi.x, hi.y, hi.z}, lo.w};
+            }
+            b = join8(b);
+            if (i < children && (threadIdx.x & (kRayArity - 1)) == 0) store_box(tree.node(level, i / kRayArity), b);
+        }
+        __syncthreads();  // the next level reads this one
+    }
 }
 
 struct Ray {
@@ -129,29 +330,46 @@ __device__ __forceinline__ void box_axis(float p, float r, float inv, int dim, i
     hi = (int)b;
 }
 
-__global__ void __launch_bounds__(kRayTileX* kRayTileY) k_raycast(GridDev g, const float4* __restrict__ m,
-                                                                   const nsph_raycast_camera cam, float search_radius,
-                                                                   float march_step, int max_steps,
-                                                                   float* __restrict__ depth)
+// Cells that can hold a sphere hit before the window's end: a box of virtual
+// cells [lo, lo + span] per axis, as physical coordinates. `all`: every cell.
+struct RayRegion {
+    int first[3], span[3];
+    bool all;
+};
+
+__device__ __forceinline__ int wrap_dim(unsigned v, int dim)
 {
-    const int px = blockIdx.x * kRayTileX + threadIdx.x;
-    const int py = blockIdx.y * kRayTileY + threadIdx.y;
-    if (px >= cam.width || py >= cam.height) return;
-    const Ray r = ray_for_pixel(cam, px, py);
-    float* out = depth + (size_t)py * cam.width + px;
-    float best = *out;
-    if (best < 0.f) best = cam.max_distance;
+    return (int)((dim & (dim - 1)) == 0 ? v & (unsigned)(dim - 1) : v % (unsigned)dim);
+}
+
+// whether the physical cells of the virtual run [lo, hi] meet those of the region's axis a
+__device__ __forceinline__ bool axis_meets(const RayRegion& g, int a, int lo, int hi, int dim)
+{
+    if ((long long)lo + kOrigin < 0 || g.span[a] + (hi - lo) + 2 > dim) return true;
+    const int p = wrap_dim((unsigned)(lo + (int)kOrigin), dim);
+    const int d = p >= g.first[a] ? p - g.first[a] : p - g.first[a] + dim;  // from the region's first to lo
+    return d <= g.span[a] || dim - d <= hi - lo;
+}
+
+// the march over the samples whose box meets the region, testing each cell
+// once; `best` as the buffer had it on entry. Returns whether anything was hit.
+__device__ __noinline__ bool march(const GridDev& g, const float4* __restrict__ m, const Ray& r, float max_distance,
+                                   float search_radius, float march_step, int max_steps, const RayRegion& region,
+                                   float stop, float& best)
+{
     bool hit = false;
     // previous query box, empty at first (every cell then counts as new)
     int pxl = 0, pxh = -1, pyl = 0, pyh = -1, pzl = 0, pzh = -1;
     int s = 0;
     float t = 0.f;
-    while (s < max_steps && t <= cam.max_distance && t <= best) {
+    while (s < max_steps && t <= max_distance && t <= best && t <= stop) {
         int xl, xh, yl, yh, zl, zh;
         box_axis(__fadd_rn(r.ox, __fmul_rn(r.dx, t)), search_radius, g.inv, g.dx, xl, xh);
         box_axis(__fadd_rn(r.oy, __fmul_rn(r.dy, t)), search_radius, g.inv, g.dy, yl, yh);
         box_axis(__fadd_rn(r.oz, __fmul_rn(r.dz, t)), search_radius, g.inv, g.dz, zl, zh);
-        if (xl != pxl || xh != pxh || yl != pyl || yh != pyh || zl != pzl || zh != pzh) {
+        const bool meets = region.all || (axis_meets(region, 0, xl, xh, g.dx) && axis_meets(region, 1, yl, yh, g.dy) &&
+                                          axis_meets(region, 2, zl, zh, g.dz));
+        if (meets && (xl != pxl || xh != pxh || yl != pyl || yh != pyh || zl != pzl || zh != pzh)) {
             const AxisWalk ax = axis_walk(xl, g.dx), ay = axis_walk(yl, g.dy), az = axis_walk(zl, g.dz);
             const int nx = xh - xl + 1, ny = yh - yl + 1, nz = zh - zl + 1;
             for (int iz = 0; iz < nz; ++iz) {
@@ -171,7 +389,7 @@ __global__ void __launch_bounds__(kRayTileX* kRayTileY) k_raycast(GridDev g, con
                             if (q.w <= 0.f) continue;
                             const float th = ray_sphere(r, q);
                             if (th < 0.f) continue;
-                            if (th > cam.max_distance) continue;
+                            if (th > max_distance) continue;
                             if (th < best) {
                                 best = th;
                                 hit = true;
@@ -190,7 +408,165 @@ __global__ void __launch_bounds__(kRayTileX* kRayTileY) k_raycast(GridDev g, con
         ++s;
         t = __fadd_rn(t, march_step);
     }
-    if (hit) *out = best;
+    return hit;
+}
+
+// nearest computed hit of the warp's rays over all spheres: a depth-first walk
+// of the tree shared by the warp, nearest child first. `best` is the bound on
+// entry; returns the sphere's Morton position or -1.
+__device__ __forceinline__ int nearest_hit(const RayTree& tree, const float4* __restrict__ sorted, int n,
+                                           const Ray& r, bool live, float max_distance, float& best, int2* stack)
+{
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    int who = -1;
+    if (!live) best = -1.f;
+    // a zero component would give 0 x inf on a box face
+    auto inverse = [](float d) { return 1.f / (fabsf(d) < 1e-12f ? copysignf(1e-12f, d) : d); };
+    const float ix = inverse(r.dx), iy = inverse(r.dy), iz = inverse(r.dz);
+    int sp = 0;
+    if (lane == 0) stack[0] = make_int2((int)((unsigned)(tree.levels - 1) << 28), 0);
+    sp = 1;
+    __syncwarp();
+    while (sp > 0) {
+        const int2 top = stack[--sp];
+        __syncwarp();
+        const float far = __uint_as_float(__reduce_max_sync(kAll, __float_as_uint(fmaxf(best, 0.f))));
+        if (__int_as_float(top.y) > far) continue;
+        const int level = (int)((unsigned)top.x >> 28), first = kRayArity * (top.x & 0x0fffffff);
+        if (level == 0) {
+#pragma unroll
+            for (int c = 0; c < kRayArity; ++c) {
+                if (first + c >= n) break;
+                const float4 q = __ldg(sorted + first + c);
+                if (!(q.w > 0.f)) continue;
+                const float th = ray_sphere(r, q);
+                if (th >= 0.f && th <= max_distance && th < best) {
+                    best = th;
+                    who = first + c;
+                }
+            }
+            continue;
+        }
+        unsigned key = 0xffffffffu;  // lane c < 8: child c's nearest entry over the warp's rays
+        const int children = min(kRayArity, tree.count[level - 1] - first);
+        for (int c = 0; c < children; ++c) {
+            const float4* node = tree.node(level - 1, first + c);
+            const float4 lo = __ldg(node), hi = __ldg(node + 1);
+            float entry = INFINITY;
+            if (lo.x <= hi.x) {
+                // the farthest point of the box from the camera bounds the rounding of its spheres' tests
+                const float fx = fmaxf(fabsf(lo.x - r.ox), fabsf(hi.x - r.ox));
+                const float fy = fmaxf(fabsf(lo.y - r.oy), fabsf(hi.y - r.oy));
+                const float fz = fmaxf(fabsf(lo.z - r.oz), fabsf(hi.z - r.oz));
+                const float w = reach(lo.w, sqrtf(fx * fx + fy * fy + fz * fz) * 1.0001f);
+                const float ax = (lo.x - w - r.ox) * ix, bx = (hi.x + w - r.ox) * ix;
+                const float ay = (lo.y - w - r.oy) * iy, by = (hi.y + w - r.oy) * iy;
+                const float az = (lo.z - w - r.oz) * iz, bz = (hi.z + w - r.oz) * iz;
+                const float tn = fmaxf(fmaxf(fminf(ax, bx), fminf(ay, by)), fminf(az, bz));
+                const float tf = fminf(fminf(fmaxf(ax, bx), fmaxf(ay, by)), fmaxf(az, bz));
+                // the ray's nearest point to a centre lies in the inflated
+                // box; the hit may lie up to w before it (or, from inside a
+                // sphere, after it)
+                const float near = fmaxf(tn - w, 0.f);
+                if (tn <= tf && tf >= -2.f * w && near <= best) entry = near;
+            }
+            const unsigned e = __reduce_min_sync(kAll, __float_as_uint(entry));
+            if (lane == c) key = e;
+        }
+        const bool take = lane < children && key < 0x7f800000u;
+        const unsigned taken = __ballot_sync(kAll, take);
+        int rank = 0;  // farthest first, so that the nearest is popped next
+        for (int c = 0; c < children; ++c) {
+            const unsigned other = __shfl_sync(kAll, key, c);
+            if (((taken >> c) & 1u) && (other > key || (other == key && c > lane))) ++rank;
+        }
+        if (take) stack[sp + rank] = make_int2((int)(((unsigned)(level - 1) << 28) | (unsigned)(first + lane)), (int)key);
+        sp += __popc(taken);
+        __syncwarp();
+    }
+    return who;
+}
+
+constexpr int kRayStack = kRayLevels * kRayArity;
+
+// a warp takes a tile of 8 x 4 pixels, a block one of 16 x 8
+__global__ void __launch_bounds__(128) k_raycast(const __grid_constant__ GridDev g, const float4* __restrict__ m,
+                                                 const float4* __restrict__ sorted, const __grid_constant__ RayTree tree,
+                                                 int n, const __grid_constant__ nsph_raycast_camera cam,
+                                                 float search_radius, float march_step, int max_steps,
+                                                 float* __restrict__ depth)
+{
+    __shared__ int2 stacks[4][kRayStack];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int px = blockIdx.x * 16 + (warp & 1) * 8 + (lane & 7);
+    const int py = blockIdx.y * 8 + (warp >> 1) * 4 + (lane >> 3);
+    const bool live = px < cam.width && py < cam.height;
+    const Ray r = ray_for_pixel(cam, min(px, cam.width - 1), min(py, cam.height - 1));
+    float* out = depth + (live ? (size_t)py * cam.width + px : 0);
+    const float had = live ? (*out < 0.f ? cam.max_distance : *out) : 0.f;
+    float best = had;
+    const int who = nearest_hit(tree, sorted, n, r, live, cam.max_distance, best, stacks[warp]);
+    if (!live || who < 0) return;
+
+    // the samples with t <= best are all taken: does one of the last of them
+    // hold the sphere's cell?
+    const float4 q = sorted[who];
+    const int cx = phys_axis(trunc_sat(__fmul_rn(q.x, g.inv)), g.dx), cy = phys_axis(trunc_sat(__fmul_rn(q.y, g.inv)), g.dy),
+              cz = phys_axis(trunc_sat(__fmul_rn(q.z, g.inv)), g.dz);
+    auto holds = [](int lo, int hi, int c, int dim) {
+        if ((long long)lo + kOrigin < 0) return false;  // clamped cells: left to the march
+        int d = c - wrap_dim((unsigned)(lo + (int)kOrigin), dim);
+        if (d < 0) d += dim;
+        return d <= hi - lo;
+    };
+    int s = 0;
+    float t = 0.f;
+    while (s < max_steps && t <= cam.max_distance && t <= best) {
+        if (t + 4.f * march_step > best) {
+            int xl, xh, yl, yh, zl, zh;
+            box_axis(__fadd_rn(r.ox, __fmul_rn(r.dx, t)), search_radius, g.inv, g.dx, xl, xh);
+            box_axis(__fadd_rn(r.oy, __fmul_rn(r.dy, t)), search_radius, g.inv, g.dy, yl, yh);
+            box_axis(__fadd_rn(r.oz, __fmul_rn(r.dz, t)), search_radius, g.inv, g.dz, zl, zh);
+            if (holds(xl, xh, cx, g.dx) && holds(yl, yh, cy, g.dy) && holds(zl, zh, cz, g.dz)) {
+                *out = best;
+                return;
+            }
+        }
+        ++s;
+        t = __fadd_rn(t, march_step);
+    }
+
+    const float nearest = best, rmax = tree.node(tree.levels - 1, 0)->w;
+    const float cell = 1.f / g.inv;
+    for (float window = 4.f * (search_radius + march_step);; window *= 4.f) {
+        // centres of spheres hit in [nearest, until]: within `w` of the ray's
+        // points at [nearest - w, until + w]
+        const float until = nearest + window;
+        const float w = 1.001f * reach(rmax, until + 2.f * rmax) + 1e-5f * until;
+        RayRegion region;
+        region.all = !(until < cam.max_distance && max_steps < (1 << 24) && window < 1e6f * cell);
+        const float o[3] = {r.ox, r.oy, r.oz}, d[3] = {r.dx, r.dy, r.dz};
+        const int dims[3] = {g.dx, g.dy, g.dz};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const float p0 = o[a] + d[a] * (nearest - w), p1 = o[a] + d[a] * (until + w);
+            const float lo = (fminf(p0, p1) - w) * g.inv, hi = (fmaxf(p0, p1) + w) * g.inv;
+            const bool fits = fabsf(lo) < 1e6f && fabsf(hi) < 1e6f;
+            const int vlo = fits ? (int)floorf(lo) - 1 : 0, vhi = fits ? (int)ceilf(hi) + 1 : 0;
+            region.span[a] = vhi - vlo;
+            region.first[a] = wrap_dim((unsigned)(vlo + (int)kOrigin), dims[a]);
+            region.all |= !fits;
+        }
+        best = had;
+        const bool hit = march(g, m, r, cam.max_distance, search_radius, march_step, max_steps, region,
+                               region.all ? INFINITY : until, best);
+        // a march that ended on a hit inside the window is the reference's
+        if (region.all || (hit && best <= until)) {
+            if (hit) *out = best;
+            return;
+        }
+    }
 }
 
 __global__ void k_clamp_no_hits(float* __restrict__ depth, int count, float max_distance)
@@ -232,15 +608,47 @@ extern "C" int nsph_raycast_particles(nsph_grid* grid, const float* x, const flo
         cudaFree(grid->mirror);
         grid->mirror = nullptr;
         grid->mirror_cap = 0;
-        NSPH_CUDA_TRY(cudaMalloc(&grid->mirror, sizeof(float4) * 2 * (size_t)g.capacity));
+        NSPH_CUDA_TRY(cudaMalloc(&grid->mirror, mirror_bytes(g.capacity)));
         grid->mirror_cap = g.capacity;
     }
     cudaStream_t cs = (cudaStream_t)stream;
-    k_raycast_gather<<<(n + 255) / 256, 256, 0, cs>>>(g.point_ids, x, radius, n, grid->mirror);
+    float4* m = grid->mirror;
+    float4* sorted = grid->mirror + grid->mirror_cap;
+    unsigned* bounds = reinterpret_cast<unsigned*>(grid->mirror + 2 * (size_t)grid->mirror_cap);
+    NSPH_CUDA_TRY(cudaMemsetAsync(bounds, 0, 6 * sizeof(unsigned), cs));
+    const int blocks_n = (n + 255) / 256;
+    k_raycast_gather<<<blocks_n, 256, 0, cs>>>(g.point_ids, x, radius, n, c, m, bounds);
     NSPH_LAUNCH_CHECK("k_raycast_gather");
-    const dim3 block(kRayTileX, kRayTileY);
-    const dim3 blocks((c.width + kRayTileX - 1) / kRayTileX, (c.height + kRayTileY - 1) / kRayTileY);
-    k_raycast<<<blocks, block, 0, cs>>>(g.view(), grid->mirror, c, search_radius, march_step, max_steps, depth);
+    // the tree: Morton order by the grid's sort buffers (free after its
+    // build), then the nodes into the same buffers
+    k_ray_keys<<<blocks_n, 256, 0, cs>>>(m, n, c, bounds, g.keys_a, g.vals_a);
+    NSPH_LAUNCH_CHECK("k_ray_keys");
+    const int st = grid_sort_keys(g, n, 24, cs);
+    if (st != NSPH_OK) return st;
+    RayTree tree;
+    tree.leaves = reinterpret_cast<float4*>(g.keys_a);
+    tree.upper = reinterpret_cast<float4*>(g.vals_a);
+    tree.count[0] = (n + kRayArity - 1) / kRayArity;
+    tree.offset[0] = 0;
+    tree.levels = 1;
+    for (int used = 0; tree.count[tree.levels - 1] > 1; ++tree.levels) {
+        tree.count[tree.levels] = (tree.count[tree.levels - 1] + kRayArity - 1) / kRayArity;
+        tree.offset[tree.levels] = used;
+        used += tree.count[tree.levels];
+    }
+    k_ray_leaves<<<blocks_n, 256, 0, cs>>>(m, g.vals_b, n, c, sorted, tree);
+    NSPH_LAUNCH_CHECK("k_ray_leaves");
+    int level = 1;
+    for (; level < tree.levels && tree.count[level - 1] > 4096; ++level) {
+        k_ray_upper<<<(tree.count[level - 1] + 255) / 256, 256, 0, cs>>>(tree, level);
+        NSPH_LAUNCH_CHECK("k_ray_upper");
+    }
+    if (level < tree.levels) {
+        k_ray_top<<<1, 1024, 0, cs>>>(tree, level);
+        NSPH_LAUNCH_CHECK("k_ray_top");
+    }
+    const dim3 blocks((c.width + 15) / 16, (c.height + 7) / 8);
+    k_raycast<<<blocks, 128, 0, cs>>>(g.view(), m, sorted, tree, n, c, search_radius, march_step, max_steps, depth);
     NSPH_LAUNCH_CHECK("k_raycast");
     return NSPH_OK;
 }
