@@ -15,6 +15,7 @@ __global__ void k_integrate(const float* __restrict__ x, const float* __restrict
                             const int* __restrict__ world, const float* __restrict__ gravity, int world_count,
                             int n, float dt, float v_max, float* __restrict__ x_new, float* __restrict__ v_new)
 {
+    launch_entry();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     const size_t i = (size_t)t;
@@ -64,8 +65,8 @@ extern "C" int nsph_integrate_particles(const float* x, const float* v, const fl
     if (!x || !v || !f || !inv_mass || !flags || !gravity || !x_new || !v_new)
         return fail(NSPH_ERR_INVALID_ARG, "null array");
     if (world_count < 1) return fail(NSPH_ERR_INVALID_ARG, "gravity needs world_count >= 1");
-    k_integrate<<<(num + 255) / 256, 256, 0, (cudaStream_t)stream>>>(x, v, f, inv_mass, flags, world, gravity,
-                                                                    world_count, num, dt, v_max, x_new, v_new);
+    NSPH_CUDA_TRY(launch_dependent(k_integrate, (num + 255) / 256, 256, 0, (cudaStream_t)stream,
+                                   x, v, f, inv_mass, flags, world, gravity, world_count, num, dt, v_max, x_new, v_new));
     NSPH_LAUNCH_CHECK("k_integrate");
     return NSPH_OK;
 }

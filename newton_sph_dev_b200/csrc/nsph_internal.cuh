@@ -85,6 +85,44 @@ unsigned long long nsph_bounds_read_raycast();
         if (err__ != cudaSuccess) return ::nsph::cuda_fail(err__, #expr); \
     } while (0)
 
+// Launch as a programmatic dependent of the stream's previous kernel: its
+// blocks are set up while that one drains, instead of after it. Every kernel
+// launched this way opens with launch_entry(), which lets its own dependent be
+// set up and then waits for the previous kernel to have finished and its
+// writes to be visible, so the order of memory accesses is that of plain
+// launches.
+// Not for a kernel that lives off the L1 behind one with much shared memory:
+// its early blocks keep the other's carveout, and so a small L1, until they
+// are done (the force pass after the density pass of the 1M tank).
+template <class... P, class... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = grid;
+    config.blockDim = block;
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    config.attrs = &attr;
+    config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...);
+}
+
+template <class... P, class... A>
+cudaError_t launch_plain(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args)
+{
+    kernel<<<grid, block, smem, stream>>>(static_cast<P>(args)...);
+    return cudaGetLastError();
+}
+
+__device__ __forceinline__ void launch_entry()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 #define NSPH_LAUNCH_CHECK(what)                                       \
     do {                                                              \
         cudaError_t err__ = cudaGetLastError();                       \
@@ -136,6 +174,25 @@ __device__ __forceinline__ void query_bounds(float p, float r, float inv, int di
     b = b < a ? a : b;
     s = a;
     e = b;
+}
+
+// physical coordinate of virtual cell c (not clamped: c + 2^20 >= 0)
+__device__ __forceinline__ int wrap_cell(int c, int dim)
+{
+    const unsigned v = (unsigned)(c + (int)kOrigin);
+    return (int)((dim & (dim - 1)) == 0 ? v & (unsigned)(dim - 1) : v % (unsigned)dim);
+}
+
+constexpr float kRegularCells = 1048560.f;  // |cell coordinate| below which no cell is clamped (2^20 origin)
+
+// one axis of the query box of p +- r (Warp's bounds), and whether any of its
+// cells could be clamped at the 2^20 origin (or p is not finite)
+__device__ __forceinline__ void box_axis_regular(float p, float r, float inv, int dim, int& s, int& e, bool& clamped)
+{
+    const float a = __fmul_rn(__fsub_rn(p, r), inv), b = __fmul_rn(__fadd_rn(p, r), inv);
+    clamped |= !(fabsf(a) < kRegularCells && fabsf(b) < kRegularCells);
+    s = trunc_sat(a);
+    e = max(min(trunc_sat(b), s + dim - 1), s);
 }
 
 __device__ __forceinline__ int point_cell(float x, float y, float z, float inv, int dx, int dy, int dz)
@@ -280,7 +337,7 @@ struct Grid {
 };
 
 // Gather performed by the last radix pass (SPH mode): writes the sorted
-// mirrors xs = (x, y, z, m_eff) and vs = (vx, vy, vz, attr bits).
+// mirrors xs = (x, y, z, mirror_mass) and vs = (vx, vy, vz, attr bits).
 struct GatherArgs {
     const float* x;
     const float* v;
@@ -292,6 +349,12 @@ struct GatherArgs {
     float4* xs;
     float4* vs;
 };
+
+// xs.w of a particle: its mass, or -0 for an inactive one (which then counts
+// as zero in every sum, and is told apart from an active particle without
+// mass by its sign)
+__device__ __forceinline__ float mirror_mass(float m, bool active) { return active ? __fadd_rn(m, 0.f) : -0.f; }
+__device__ __forceinline__ bool mirror_inactive(float4 x) { return __float_as_uint(x.w) == 0x80000000u; }
 
 // attr bits stored in vs.w
 constexpr int kAttrActive = 1;

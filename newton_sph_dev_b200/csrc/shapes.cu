@@ -317,6 +317,7 @@ __global__ void k_soft_count(const nsph_shape* __restrict__ shapes, int shape_co
                              const float* __restrict__ radius, const int* __restrict__ flags,
                              const int* __restrict__ world, float margin, int* __restrict__ block_counts)
 {
+    launch_entry();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     int c = 0;
     if (p < n && particle_active(flags, p))
@@ -330,6 +331,7 @@ __global__ void k_soft_count(const nsph_shape* __restrict__ shapes, int shape_co
 // contact count (soft_contact_count[0], the total before the max clamp)
 __global__ void k_soft_scan(int* __restrict__ block_counts, int blocks, int* __restrict__ count)
 {
+    launch_entry();
     const int per = (blocks + blockDim.x - 1) / blockDim.x;
     const int lo = threadIdx.x * per, hi = min(lo + per, blocks);
     int s = 0;
@@ -351,6 +353,7 @@ __global__ void k_soft_write(const nsph_shape* __restrict__ shapes, int shape_co
                              const int* __restrict__ flags, const int* __restrict__ world, float margin,
                              const int* __restrict__ block_offsets, ContactArrays out)
 {
+    launch_entry();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = p < n && particle_active(flags, p);
     V3 px = v3(0.f, 0.f, 0.f);
@@ -403,6 +406,7 @@ __global__ void k_shape_forces(const nsph_shape* __restrict__ shapes, ContactVie
                                const float* __restrict__ x, const float* __restrict__ v,
                                const float* __restrict__ radius, const int* __restrict__ flags, float* __restrict__ f)
 {
+    launch_entry();
     const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
     const int total = contact_total(c);
     int p = 0;
@@ -439,6 +443,7 @@ __global__ void k_shape_deltas(const nsph_shape* __restrict__ shapes, ContactVie
                                const float* __restrict__ inv_mass, const float* __restrict__ radius,
                                const int* __restrict__ flags, float* __restrict__ delta)
 {
+    launch_entry();
     const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
     const int total = contact_total(c);
     int p = 0;
@@ -478,6 +483,7 @@ __global__ void k_shape_restitution(ContactView c, nsph_soft_contact_params prm,
                                     const float* __restrict__ radius, const int* __restrict__ flags,
                                     float* __restrict__ v_out)
 {
+    launch_entry();
     const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
     const int total = contact_total(c);
     int p = 0;
@@ -507,6 +513,7 @@ __global__ void k_apply_deltas(int n, const float* __restrict__ x_orig, const fl
                                const int* __restrict__ flags, const float* __restrict__ delta, float dt, float v_max,
                                float* __restrict__ x_out, float* __restrict__ v_out)
 {
+    launch_entry();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n || !particle_active(flags, p)) return;
     const V3 x0 = load3(x_orig, p);
@@ -572,14 +579,16 @@ extern "C" int nsph_soft_contacts_create(const nsph_shape* shapes, int shape_cou
         return NSPH_OK;
     }
     const int blocks = (n + kShapeThreads - 1) / kShapeThreads;
-    k_soft_count<<<blocks, kShapeThreads, 0, cs>>>(shapes, shape_count, n, x, radius, flags, world, margin, scratch);
+    NSPH_CUDA_TRY(launch_dependent(k_soft_count, blocks, kShapeThreads, 0, cs,
+                                   shapes, shape_count, n, x, radius, flags, world, margin, scratch));
     NSPH_LAUNCH_CHECK("k_soft_count");
-    k_soft_scan<<<1, kScanMaxThreads, 0, cs>>>(scratch, blocks, contacts->count);
+    NSPH_CUDA_TRY(launch_dependent(k_soft_scan, 1, kScanMaxThreads, 0, cs,
+                                   scratch, blocks, contacts->count));
     NSPH_LAUNCH_CHECK("k_soft_scan");
     ContactArrays out{contacts->count, contacts->particle, contacts->shape, contacts->body_pos, contacts->body_vel,
                       contacts->normal, contacts->max};
-    k_soft_write<<<blocks, kShapeThreads, 0, cs>>>(shapes, shape_count, n, x, radius, flags, world, margin, scratch,
-                                                   out);
+    NSPH_CUDA_TRY(launch_dependent(k_soft_write, blocks, kShapeThreads, 0, cs,
+                                   shapes, shape_count, n, x, radius, flags, world, margin, scratch, out));
     NSPH_LAUNCH_CHECK("k_soft_write");
     return NSPH_OK;
 }
@@ -598,8 +607,8 @@ extern "C" int nsph_particle_shape_contact_forces(const nsph_shape* shapes, int 
     if (!params) return fail(NSPH_ERR_INVALID_ARG, "null params");
     if (contacts->max == 0 || shape_count == 0) return NSPH_OK;
     if (!x || !v || !radius || !flags || !f) return fail(NSPH_ERR_INVALID_ARG, "null particle array");
-    k_shape_forces<<<contact_blocks(contacts), kShapeThreads, 0, (cudaStream_t)stream>>>(
-        shapes, view_of(contacts), *params, x, v, radius, flags, f);
+    NSPH_CUDA_TRY(launch_dependent(k_shape_forces, contact_blocks(contacts), kShapeThreads, 0, (cudaStream_t)stream,
+                                   shapes, view_of(contacts), *params, x, v, radius, flags, f));
     NSPH_LAUNCH_CHECK("k_shape_forces");
     return NSPH_OK;
 }
@@ -618,8 +627,8 @@ extern "C" int nsph_particle_shape_contact_deltas(const nsph_shape* shapes, int 
     if (!params) return fail(NSPH_ERR_INVALID_ARG, "null params");
     if (contacts->max == 0 || shape_count == 0) return NSPH_OK;
     if (!x || !v || !inv_mass || !radius || !flags || !deltas) return fail(NSPH_ERR_INVALID_ARG, "null particle array");
-    k_shape_deltas<<<contact_blocks(contacts), kShapeThreads, 0, (cudaStream_t)stream>>>(
-        shapes, view_of(contacts), *params, x, v, inv_mass, radius, flags, deltas);
+    NSPH_CUDA_TRY(launch_dependent(k_shape_deltas, contact_blocks(contacts), kShapeThreads, 0, (cudaStream_t)stream,
+                                   shapes, view_of(contacts), *params, x, v, inv_mass, radius, flags, deltas));
     NSPH_LAUNCH_CHECK("k_shape_deltas");
     return NSPH_OK;
 }
@@ -636,8 +645,8 @@ extern "C" int nsph_particle_shape_restitution(const nsph_soft_contacts* contact
     if (contacts->max == 0) return NSPH_OK;
     if (!v_new || !x_old || !v_old || !radius || !flags || !v_out)
         return fail(NSPH_ERR_INVALID_ARG, "null particle array");
-    k_shape_restitution<<<contact_blocks(contacts), kShapeThreads, 0, (cudaStream_t)stream>>>(
-        view_of(contacts), *params, v_new, x_old, v_old, radius, flags, v_out);
+    NSPH_CUDA_TRY(launch_dependent(k_shape_restitution, contact_blocks(contacts), kShapeThreads, 0, (cudaStream_t)stream,
+                                   view_of(contacts), *params, v_new, x_old, v_old, radius, flags, v_out));
     NSPH_LAUNCH_CHECK("k_shape_restitution");
     return NSPH_OK;
 }
@@ -652,8 +661,8 @@ extern "C" int nsph_apply_particle_deltas(int n, const float* x_orig, const floa
     if (n == 0) return NSPH_OK;
     if (!x_orig || !x_pred || !flags || !deltas || !x_out || !v_out)
         return fail(NSPH_ERR_INVALID_ARG, "null particle array");
-    k_apply_deltas<<<(n + kShapeThreads - 1) / kShapeThreads, kShapeThreads, 0, (cudaStream_t)stream>>>(
-        n, x_orig, x_pred, flags, deltas, dt, v_max, x_out, v_out);
+    NSPH_CUDA_TRY(launch_dependent(k_apply_deltas, (n + kShapeThreads - 1) / kShapeThreads, kShapeThreads, 0, (cudaStream_t)stream,
+                                   n, x_orig, x_pred, flags, deltas, dt, v_max, x_out, v_out));
     NSPH_LAUNCH_CHECK("k_apply_deltas");
     return NSPH_OK;
 }
