@@ -521,6 +521,23 @@ NSPH_API int nsph_apply_particle_deltas(int num_particles, const float* x_orig, 
                                         const int* flags, const float* deltas, float dt, float v_max, float* x_out,
                                         float* v_out, void* stream);
 
+/* The particle iterations of SolverXPBD.step in one call: per iteration the
+ * shape corrections (when contacts and shapes are given), the particle-particle
+ * corrections on `grid` (built on x_a) and apply_particle_deltas, with the
+ * results of nsph_particle_shape_contact_deltas, nsph_particle_contact_deltas
+ * (on zeroed deltas) and nsph_apply_particle_deltas called in turn. Even
+ * iterations read (x_a, v_a) and write (x_b, v_b), odd ones the reverse;
+ * inactive particles are not written. x_orig: the positions at the step's
+ * start (it may be x_b: it is read before the first write). deltas (3 n
+ * floats; needed with shapes only) and scratch (12 n floats, 16-byte aligned)
+ * are overwritten. */
+NSPH_API int nsph_xpbd_solve(const nsph_grid* grid, int num_particles, int iterations, const float* x_orig,
+                             float* x_a, float* v_a, float* x_b, float* v_b, const float* inv_mass,
+                             const float* radius, const int* flags, const nsph_shape* shapes, int shape_count,
+                             const nsph_soft_contacts* contacts, const nsph_soft_contact_params* soft, float k_mu,
+                             float k_cohesion, float max_radius, float dt, float relaxation, float v_max,
+                             float* deltas, float* scratch, void* stream);
+
 /* ---- learned surrogate step (no counterpart in the reference) -------------
  * A WCSPH step with a larger dt whose acceleration is corrected per particle
  * by a small MLP (16 -> 64 -> 64 -> 3, SiLU; bf16 weights and activations,

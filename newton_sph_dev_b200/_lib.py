@@ -287,6 +287,12 @@ SIGNATURES = [
         ctypes.c_int,
         [ctypes.c_int] + [c_void_p] * 4 + [ctypes.c_float, ctypes.c_float, c_void_p, c_void_p, c_void_p],
     ),
+    (
+        "nsph_xpbd_solve",
+        ctypes.c_int,
+        [c_void_p, ctypes.c_int, ctypes.c_int] + [c_void_p] * 8 + [c_void_p, ctypes.c_int, c_void_p, c_void_p]
+        + [ctypes.c_float] * 6 + [c_void_p] * 3,
+    ),
     ("nsph_sph_enable_surrogate", ctypes.c_int, [c_void_p]),
     (
         "nsph_sph_features",

@@ -162,6 +162,30 @@ def apply_particle_deltas(model, x_orig: torch.Tensor, x_pred: torch.Tensor, del
     _lib.check(st, "apply_particle_deltas")
 
 
+def solve_xpbd_iterations(model, contacts, iterations: int, state_in, state_out, deltas: torch.Tensor,
+                          scratch: torch.Tensor, dt: float, relaxation: float) -> None:
+    """SolverXPBD.step's particle iterations in one call (nsph_xpbd_solve),
+    from the prediction in state_out, on the grid built on it; iterates
+    alternate between state_in's and state_out's arrays. deltas (N, 3) and
+    scratch (N, 12) are work memory."""
+    n = model.particle_count
+    for t, name in ((state_in.particle_q, "particle_q"), (state_in.particle_qd, "particle_qd"),
+                    (state_out.particle_q, "particle_q"), (state_out.particle_qd, "particle_qd")):
+        _check(t, n, name)
+    shapes = model.shape_count and contacts is not None and contacts.soft_contact_max
+    c = contacts.c_struct() if shapes else None
+    p = soft_contact_params(model, dt, relaxation) if shapes else None
+    st = _lib.load().nsph_xpbd_solve(
+        model.particle_grid.id, n, int(iterations), state_in.particle_q.data_ptr(), state_out.particle_q.data_ptr(),
+        state_out.particle_qd.data_ptr(), state_in.particle_q.data_ptr(), state_in.particle_qd.data_ptr(),
+        model.particle_inv_mass.data_ptr(), model.particle_radius.data_ptr(), model.particle_flags.data_ptr(),
+        _shapes_ptr(model) if shapes else None, model.shape_count if shapes else 0,
+        ctypes.byref(c) if shapes else None, ctypes.byref(p) if shapes else None, float(model.particle_mu),
+        float(model.particle_cohesion), float(model.particle_max_radius), float(dt), float(relaxation),
+        float(model.particle_max_velocity), deltas.data_ptr(), scratch.data_ptr(), _lib.stream_handle(model.device))
+    _lib.check(st, "SolverXPBD.step")
+
+
 __all__ = ["apply_particle_deltas", "apply_particle_shape_restitution", "contact_params",
            "eval_particle_body_contact_forces", "eval_particle_contact_forces", "soft_contact_params",
-           "solve_particle_particle_contacts", "solve_particle_shape_contacts"]
+           "solve_particle_particle_contacts", "solve_particle_shape_contacts", "solve_xpbd_iterations"]

@@ -48,6 +48,7 @@ class SolverXPBD(SolverBase):
         self._deltas = None
         self._q_init = None
         self._qd_init = None
+        self._scratch = None
         if model.particle_count:
             _require_cuda(model.particle_q, "model.particle_q")
             self._deltas = torch.empty_like(model.particle_q)
@@ -68,6 +69,35 @@ class SolverXPBD(SolverBase):
         pc.apply_particle_deltas(model, self._q_init, particle_q, self._deltas, dt, new_q, new_qd)
         return new_q, new_qd
 
+    def _one_call(self, state_in: State, state_out: State) -> bool:
+        """Whether the iterations can run as one nsph_xpbd_solve: particle
+        contacts on the model's grid between two states of their own memory."""
+        model = self.model
+        return (self.iterations > 0 and model.particle_count > 1 and model.particle_grid is not None
+                and model.particle_max_radius > 0.0
+                and state_in.particle_q.data_ptr() != state_out.particle_q.data_ptr()
+                and state_in.particle_qd.data_ptr() != state_out.particle_qd.data_ptr())
+
+    def _step_one_call(self, state_in: State, state_out: State, contacts, dt: float) -> None:
+        model, n = self.model, self.model.particle_count
+        if self.enable_restitution:
+            self._q_init.copy_(state_in.particle_q)
+            self._qd_init.copy_(state_in.particle_qd)
+        self.integrate_particles(model, state_in, state_out, dt)
+        model.particle_grid.build(state_out.particle_q, radius=model.particle_max_radius * 2.0 + model.particle_cohesion)
+        if self._scratch is None:
+            self._scratch = torch.empty((n, 12), dtype=torch.float32, device=model.device)
+        pc.solve_xpbd_iterations(model, contacts, self.iterations, state_in, state_out, self._deltas, self._scratch, dt,
+                                 self.soft_contact_relaxation)
+        final_qd = state_out.particle_qd
+        if self.iterations % 2:
+            state_out.particle_q.copy_(state_in.particle_q)
+            state_out.particle_qd.copy_(state_in.particle_qd)
+            final_qd = state_in.particle_qd
+        if self.enable_restitution and contacts is not None:
+            pc.apply_particle_shape_restitution(model, contacts, final_qd, self._q_init, self._qd_init,
+                                                state_out.particle_qd)
+
     def step(self, state_in: State, state_out: State, control: Control | None, contacts, dt: float) -> None:
         model = self.model
         if state_in.requires_grad:
@@ -76,6 +106,9 @@ class SolverXPBD(SolverBase):
         if not model.particle_count:
             return
         particle_q, particle_qd = state_out.particle_q, state_out.particle_qd
+        if self._one_call(state_in, state_out):
+            self._step_one_call(state_in, state_out, contacts, dt)
+            return
         self._q_init.copy_(state_in.particle_q)
         if self.enable_restitution:
             self._qd_init.copy_(state_in.particle_qd)
