@@ -73,6 +73,12 @@ NSPH_API int nsph_build_flags(void);
 /* Bounds-check violations counted on the current device since the last
  * call (the counters are reset); always 0 in the release build. */
 NSPH_API int nsph_debug_bounds_violations(unsigned long long* count);
+/* Self-check of the force terms' square root and reciprocal: sweeps every
+ * fp32 mantissa over two octaves (and those scaled by 2^(2 e), e in
+ * exponents[0 .. num_exponents)) on the current device and counts the values
+ * whose root or reciprocal differs from the correctly rounded operation's.
+ * Synchronises the device. */
+NSPH_API int nsph_debug_root_mismatches(const int* exponents, int num_exponents, unsigned long long* count);
 
 /* ======================================================================== *
  *  HashGrid — replaces wp.HashGrid(dim_x, dim_y, dim_z)                    *

@@ -158,6 +158,7 @@ SIGNATURES = [
     ("nsph_last_error", ctypes.c_char_p, []),
     ("nsph_build_flags", ctypes.c_int, []),
     ("nsph_debug_bounds_violations", ctypes.c_int, [ctypes.POINTER(ctypes.c_ulonglong)]),
+    ("nsph_debug_root_mismatches", ctypes.c_int, [c_void_p, ctypes.c_int, ctypes.POINTER(ctypes.c_ulonglong)]),
     ("nsph_grid_create", ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.POINTER(c_void_p)]),
     ("nsph_grid_destroy", ctypes.c_int, [c_void_p]),
     ("nsph_grid_reserve", ctypes.c_int, [c_void_p, ctypes.c_int]),

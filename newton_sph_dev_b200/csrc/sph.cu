@@ -14,7 +14,7 @@
 // only for inv_mass > 0, |v| clamp, inactive particles keep x and v).
 //
 // Layout in HBM (sorted by cell, written by the last radix pass):
-//   xs[k]  float4 (x, y, z, m_eff)   m_eff = 0 for inactive particles
+//   xs[k]  float4 (x, y, z, m_eff)   m_eff = -0 for inactive particles
 //   vs[k]  float4 (vx, vy, vz, attr) attr = active | dynamic<<1 | gravity<<2
 //   aux[k] float2 (m/rho, p/rho^2)   written by the density pass
 //   rp[k]  float2 (rho, p)           written by the density pass
@@ -23,6 +23,8 @@
 #include <cmath>
 #include <string>
 #include <vector>
+
+#include <cuda_fp16.h>
 
 #include "mlp.cuh"
 #include "nsph_internal.cuh"
@@ -50,22 +52,54 @@ __device__ __forceinline__ float dist2(float4 a, float4 b, float& dx, float& dy,
 // particle's neighbours are summed in the grid's query order, so the device
 // reproduces the fp32 restatement's sums.
 
-// W(q) = sigma * {fma((6q)q, q-1, 1) for q <= 1/2; ((2t)t)t with t = 1-q for q < 1}
-__device__ __forceinline__ float kernel_w(float q, const nsph_sph_params& p)
+// W(q) = sigma * {fma((6q)q, q-1, 1) for q <= 1/2; ((2t)t)t with t = max(1-q, 0) beyond}
+template <class P>
+__device__ __forceinline__ float kernel_w(float q, const P& p)
 {
-    const float t = __fsub_rn(1.f, q);
+    const float t = fmaxf(__fsub_rn(1.f, q), 0.f);
     const float nearv = __fmaf_rn(__fmul_rn(__fmul_rn(6.f, q), q), __fsub_rn(q, 1.f), 1.f);
     const float farv = __fmul_rn(__fmul_rn(__fmul_rn(2.f, t), t), t);
-    return __fmul_rn(p.sigma, q <= 0.5f ? nearv : (q < 1.f ? farv : 0.f));
+    return __fmul_rn(p.sigma, q <= 0.5f ? nearv : farv);
 }
 
-// (dW/dr)/r = {c_near * fma(3, q, -2) for q <= 1/2; ((c_far t) t)(1/r) for q < 1}
-__device__ __forceinline__ float kernel_f(float q, float inv_r, const nsph_sph_params& p)
+// (dW/dr)/r = {c_near * fma(3, q, -2) for q <= 1/2; ((c_far t) t)(1/r), t = max(1-q, 0), beyond}
+template <class P>
+__device__ __forceinline__ float kernel_f(float q, float inv_r, const P& p)
 {
-    const float t = __fsub_rn(1.f, q);
+    const float t = fmaxf(__fsub_rn(1.f, q), 0.f);
     const float nearv = __fmul_rn(p.c_near, __fmaf_rn(3.f, q, -2.f));
     const float farv = __fmul_rn(__fmul_rn(__fmul_rn(p.c_far, t), t), inv_r);
-    return q <= 0.5f ? nearv : (q < 1.f ? farv : 0.f);
+    return q <= 0.5f ? nearv : farv;
+}
+
+// Square root of a squared distance, and its reciprocal, both correctly
+// rounded (the bits of __fsqrt_rn and of __frcp_rn of it), from one hardware
+// reciprocal square root y ~ 1/sqrt(x): Markstein's iterations (IBM J. Res.
+// Dev. 34(1), 1990), whose residuals x - g g and 1 - r y are exact in one FMA.
+// They need no test for special operands, which the general operations spend
+// about half of their instructions on: x outside [2^-100, 2^100] (coincident
+// particles apart, nothing a simulation meets) takes those, and x = 0 gives
+// r = 0. Checked against them over every mantissa and exponent parity.
+__device__ __forceinline__ bool plain_range(float x)  // or zero
+{
+    const unsigned u = __float_as_uint(x);
+    return u - 0x0d800000u < 0x64000000u || u == 0u;
+}
+
+__device__ __forceinline__ float sqrt_plain(float x, float& y)
+{
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    const float g = __fmul_rn(x, y), hy = __fmul_rn(0.5f, y);
+    const float r = __fmaf_rn(__fmaf_rn(-g, g, x), hy, g);
+    return x == 0.f ? 0.f : r;
+}
+
+__device__ __forceinline__ float rcp_plain(float r, float y)  // y ~ 1/r from sqrt_plain
+{
+    // rounded up: the last step then also meets the one mantissa (all ones)
+    // for which an estimate below leads to a tie
+    const float y1 = __fmaf_ru(__fmaf_rn(-r, y, 1.f), y, y);
+    return __fmaf_rn(__fmaf_rn(-r, y1, 1.f), y1, y1);
 }
 
 __device__ __forceinline__ float eos(float rho, const nsph_sph_params& p)
@@ -78,9 +112,26 @@ __device__ __forceinline__ float eos(float rho, const nsph_sph_params& p)
     return pr;
 }
 
-__device__ __forceinline__ float wterm(float r2, const nsph_sph_params& p)
+template <class P>
+__device__ __forceinline__ float wterm(float r2, const P& p)
 {
-    return kernel_w(__fmul_rn(__fsqrt_rn(r2), p.inv_h), p);
+    float y, r;
+    if (plain_range(r2))
+        r = sqrt_plain(r2, y);
+    else
+        r = __fsqrt_rn(r2);
+    return kernel_w(__fmul_rn(r, p.inv_h), p);
+}
+
+// wterm of a squared distance known to be zero or in the plain range: the
+// estimate of max(x, 2^-100) is finite, and gives r = 0 for x = 0
+template <class P>
+__device__ __forceinline__ float wterm_near(float r2, const P& p)
+{
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(fmaxf(r2, 7.8886091e-31f)));
+    const float g = __fmul_rn(r2, y), hy = __fmul_rn(0.5f, y);
+    return kernel_w(__fmul_rn(__fmaf_rn(__fmaf_rn(-g, g, r2), hy, g), p.inv_h), p);
 }
 
 // ---- tolerance ("fast") arithmetic ---------------------------------------------
@@ -90,25 +141,54 @@ __device__ __forceinline__ float wterm(float r2, const nsph_sph_params& p)
 // The neighbour test r2 < h2 is unchanged, so neighbour sets stay bit-exact;
 // sums keep the query order. Results are within the fp64 oracle's tolerance
 // (checked by the tests), not bit-exact with the fp32 oracle.
-__device__ __forceinline__ float kernel_w_fast(float q, const nsph_sph_params& p)
+template <class P>
+__device__ __forceinline__ float kernel_w_fast(float q, const P& p)
 {
     const float t = 1.f - q;
     const float v = q <= 0.5f ? fmaf(6.f * q * q, q - 1.f, 1.f) : (q < 1.f ? 2.f * t * t * t : 0.f);
     return p.sigma * v;
 }
 
-__device__ __forceinline__ float wterm_fast(float r2, const nsph_sph_params& p)
+template <class P>
+__device__ __forceinline__ float wterm_fast(float r2, const P& p)
 {
     const float r = r2 > 0.f ? r2 * rsqrtf(r2) : 0.f;
     return kernel_w_fast(r * p.inv_h, p);
 }
 
 // ---- density + EOS -----------------------------------------------------------
+// What the force pass gathers of a neighbour: one 32-byte record (x, y, z, m |
+// vx, vy, vz, m/rho), read by one 256-bit load, and p/rho^2. The gathers bound
+// that pass (83% of the L1's wavefronts at 49% issue active): a warp's lanes
+// read neighbours from about 10 lines of 16-byte or 25 lines of 32-byte
+// records at a time, one wavefront per line. Two loads instead of three took
+// the 1M tank's pass from 0.158 to 0.152 ms, the batched worlds' (512 worlds,
+// 2.2M particles; with the shorter terms below) from 0.375 to 0.268 ms.
+struct ForceRec {
+    float4* rec;  // 2 per particle
+    float* pr2;
+    unsigned* overflow;  // or null: set when a particle's list overflowed (the segment tape)
+};
+
+struct Neighbour {
+    float4 x, v;  // (x, m), (v, m/rho)
+};
+
+__device__ __forceinline__ Neighbour load_neighbour(const float4* __restrict__ rec, int j)
+{
+    Neighbour r;
+    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=f"(r.x.x), "=f"(r.x.y), "=f"(r.x.z), "=f"(r.x.w), "=f"(r.v.x), "=f"(r.v.y), "=f"(r.v.z), "=f"(r.v.w)
+        : "l"(rec + 2 * (size_t)j));
+    return r;
+}
+
 template <bool Fast = false>
-__device__ __forceinline__ void density_finish(int k, float m, float rho, const nsph_sph_params& p,
-                                               float2* __restrict__ aux, float2* __restrict__ rp,
+__device__ __forceinline__ void density_finish(int k, float4 xi, float4 vi, float rho, const nsph_sph_params& p,
+                                               float2* __restrict__ aux, float2* __restrict__ rp, const ForceRec& fr,
                                                unsigned* __restrict__ status)
 {
+    const float m = xi.w;
     float pr = 0.f, mor = 0.f, pr2 = 0.f;
     if (rho > 0.f) {
         pr = eos(rho, p);
@@ -125,6 +205,9 @@ __device__ __forceinline__ void density_finish(int k, float m, float rho, const 
     }
     aux[k] = make_float2(mor, pr2);
     rp[k] = make_float2(rho, pr);
+    fr.rec[2 * (size_t)k] = xi;
+    fr.rec[2 * (size_t)k + 1] = make_float4(vi.x, vi.y, vi.z, mor);
+    fr.pr2[k] = pr2;
 }
 
 // ---- neighbour lists (the plain step) -----------------------------------------
@@ -164,85 +247,75 @@ __device__ __forceinline__ unsigned push_hit(unsigned acc, float r2, float h2)
     return __funnelshift_l(__float_as_uint(__fsub_rn(r2, h2)), acc, 1);
 }
 
-template <bool kPaddedGroups>
-__device__ __forceinline__ int neighbor_list(const GridDev& g, const float4* __restrict__ xs,
-                                             const nsph_sph_params& p, float4 xi, int4* __restrict__ nbr, int n,
-                                             int k)
-{
+// Appends neighbours to particle k's list in groups of four: the last four
+// are held in registers and a full group is stored at once.
+struct ListWriter {
+    int4* nbr;
+    int n, k;
     int cnt = 0;
     int b0 = 0, b1 = 0, b2 = 0, b3 = 0;
-    auto append = [&](int j) {
+    __device__ __forceinline__ ListWriter(int4* nbr_, int n_, int k_) : nbr(nbr_), n(n_), k(k_) {}
+    __device__ __forceinline__ void append(int j)
+    {
         b0 = b1;
         b1 = b2;
         b2 = b3;
         b3 = j;
         ++cnt;
         if ((cnt & 3) == 0 && cnt <= kNbrSlots) nbr[(size_t)((cnt >> 2) - 1) * n + k] = make_int4(b0, b1, b2, b3);
-    };
-    // Candidates are tested branch-free into a bit mask per chunk of up to 32
-    // of a run; the hits are appended after the chunk, so the append code runs
-    // once per neighbour (a warp iterates over its lanes' largest hit count of
-    // the chunk) instead of at every candidate where any lane has a hit.
-    // Candidates go in groups of four (four loads issued together). With
-    // kPaddedGroups there is no scalar tail loop: a run's last group reads
-    // up to three entries past the run, whose bits are then cleared. Those
-    // reads stay inside the array: every xs array the density passes read
-    // holds at least kXsPad entries past its last particle. (Padded groups
-    // took the 1M tank's density pass from 0.330 to 0.315 ms but the batched
-    // worlds' from 5.18 to 5.39 ms, so the worlds pass keeps the tail loop.)
-    // The padded path takes each hit bit from push_hit (0.318 -> 0.303 ms on
-    // the 1M tank); the worlds pass keeps the comparison, which spilled less.
+    }
+    // the last, partial group: its r hits are b(4-r) .. b3; the rest of it is
+    // filled with the particle itself, which its readers skip
+    __device__ __forceinline__ void finish()
+    {
+        const int r = cnt & 3;
+        if (r && cnt <= kNbrSlots)
+            nbr[(size_t)(cnt >> 2) * n + k] = r == 1 ? make_int4(b3, k, k, k)
+                                                     : (r == 2 ? make_int4(b2, b3, k, k) : make_int4(b1, b2, b3, k));
+    }
+};
+
+// The general scan of one particle by one thread: its candidates are tested
+// branch-free into a bit mask per chunk of up to 32 of a run (four loads
+// issued together; a run's last group reads up to three entries past the run,
+// whose bits are cleared: every xs array the density passes read holds at
+// least kXsPad entries past its last particle), and a chunk's hits are
+// appended to the list after it. Serves the warps that tile_neighbors
+// (below) does not take.
+__device__ __forceinline__ int neighbor_list(const GridDev& g, const float4* __restrict__ xs,
+                                             const nsph_sph_params& p, float4 xi, int4* __restrict__ nbr, int n,
+                                             int k)
+{
+    ListWriter list(nbr, n, k);
     for_each_run(g, xi.x, xi.y, xi.z, p.h, [&](int lo, int hi) {
         for (int c0 = lo; c0 < hi; c0 += 32) {
             const int m = min(32, hi - c0);
-            unsigned bits;
-            if constexpr (kPaddedGroups) {
-                unsigned acc = 0u;  // candidate t of the chunk at bit mp - 1 - t
+            unsigned acc = 0u;  // candidate t of the chunk at bit mp - 1 - t
 #pragma unroll 1
-                for (int j = 0; j < m; j += 4) {
-                    float4 xj[4];
+            for (int j = 0; j < m; j += 4) {
+                float4 xj[4];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) xj[u] = __ldg(xs + c0 + j + u);
+                for (int u = 0; u < 4; ++u) xj[u] = __ldg(xs + c0 + j + u);
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        float dx, dy, dz;
-                        acc = push_hit(acc, dist2(xi, xj[u], dx, dy, dz), p.h2);
-                    }
-                }
-                // reversed, candidate t sits at bit t; the group's reads past
-                // the run (bits m .. mp - 1) are cleared
-                const int mp = (m + 3) & ~3;
-                bits = __brev(acc) >> (32 - mp);
-                if (m < 32) bits &= (1u << m) - 1u;
-            } else {
-                bits = 0u;
-                int j = 0;
-                for (; j + 4 <= m; j += 4) {
-                    float4 xj[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) xj[u] = __ldg(xs + c0 + j + u);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        float dx, dy, dz;
-                        bits |= (unsigned)(dist2(xi, xj[u], dx, dy, dz) < p.h2) << (j + u);
-                    }
-                }
-                for (; j < m; ++j) {
+                for (int u = 0; u < 4; ++u) {
                     float dx, dy, dz;
-                    bits |= (unsigned)(dist2(xi, __ldg(xs + c0 + j), dx, dy, dz) < p.h2) << j;
+                    acc = push_hit(acc, dist2(xi, xj[u], dx, dy, dz), p.h2);
                 }
             }
+            // reversed, candidate t sits at bit t; the group's reads past
+            // the run (bits m .. mp - 1) are cleared
+            const int mp = (m + 3) & ~3;
+            unsigned bits = __brev(acc) >> (32 - mp);
+            if (m < 32) bits &= (1u << m) - 1u;
             while (bits) {
-                append(c0 + __ffs(bits) - 1);
+                const int j = c0 + __ffs(bits) - 1;
+                if (!mirror_inactive(__ldg(xs + j))) list.append(j);
                 bits &= bits - 1u;
             }
         }
     });
-    const int r = cnt & 3;  // the last, partial group: its r hits are b(4-r) .. b3
-    if (r && cnt <= kNbrSlots)
-        nbr[(size_t)(cnt >> 2) * n + k] = r == 1 ? make_int4(b3, 0, 0, 0)
-                                                 : (r == 2 ? make_int4(b2, b3, 0, 0) : make_int4(b1, b2, b3, 0));
-    return cnt;
+    list.finish();
+    return list.cnt;
 }
 
 // Element u (0..3, a constant after unrolling) of a list group.
@@ -315,38 +388,462 @@ __device__ __forceinline__ float density_from_list(const GridDev& g, const float
     return rho;
 }
 
+// The general path of one particle: list, then rho over it (a call, so that
+// its registers do not count against the kernels whose rare path it is).
+template <bool Fast>
+__device__ __noinline__ int scan_general(const GridDev* g, const float4* xs, const nsph_sph_params* p, float4 xi,
+                                         int4* nbr, int n, int k, float* rho)
+{
+    const int cnt = neighbor_list(*g, xs, *p, xi, nbr, n, k);
+    *rho = density_from_list<Fast>(*g, xs, *p, xi, nbr, cnt, n, k);
+    return cnt;
+}
+
+// ---- candidate tests on the tensor cores ----------------------------------------
+// A warp takes 32 consecutive sorted particles, one per lane. Particles of
+// one grid row (the same y and z cells, x cells within kTileSpan) share their
+// candidates: the union of their stencils is one contiguous run of sorted
+// positions per (z, y) row. Each run is tested in chunks of 32 candidates
+// against all 32 particles at once, as the contraction
+//   r2 - T = |a|^2 - T + |b|^2 - 2 a.b
+// of fp16 coordinates relative to the group's origin in units of h
+// (mma.m16n8k8, fp16 accumulators: eight instructions per chunk; the norms
+// are split into fp16 hi + lo parts along K). The sign of r2 - T marks a
+// possible neighbour: T exceeds 1 by a bound on the rounding errors, so no
+// neighbour is missed. A chunk's marks (one 32-bit word per particle) wait in
+// shared memory; then each lane walks its own marks in order, repeats the
+// exact fp32 test of the definition, sums rho and appends to the list. Sets,
+// order and every rounding are therefore those of the general scan.
+//
+// Why: per particle about 216 candidates are tested for 30 neighbours. One
+// thread per particle spent three quarters of its 211 warp instructions per
+// particle on the tests and the traversal; a chunk of 1,024 tests costs about
+// 75 warp instructions, 24 of them the matrix part, and the traversal is done
+// once per group. The 1M tank's pass went from 0.291 to 0.243 ms (166 warp
+// instructions per particle, 75% issue active), the 128^3 block's from 0.563
+// to 0.47. What bounds it now is the walk: some 70 instructions for each of a
+// warp's 38 steps. The tiles are 32 x 32 with K = 8 and live in one warp's
+// registers: tcgen05's 128-row tiles would span 16 cells, of whose joint
+// stencil a particle uses a sixth. 64 registers; 48 (five blocks per SM) were
+// slower (0.288 ms).
+constexpr int kTileWords = 20;   // words of 32 candidates between two walks (a dense stencil has 18)
+constexpr int kTileSpan = 12;     // x cells between the first and the last particle of a group
+
+// resident blocks per SM of the density passes (registers: see the kernels)
+constexpr int kDensityBlocks = 4;
+constexpr int kSmallDensity = 65536;  // particles below which its blocks are small
+
+struct __align__(16) TileSmem {
+    union {
+        // B operand of a chunk's halves: word t (of k = 2t, 2t + 1) of candidate c at [t][c]. Rows of 40 words put
+        // the eight lanes of a 128-bit load's phase (4 rows x 2 columns) on different banks.
+        unsigned frag[2][4][40];
+        int ring[8][32];          // during a walk: the lane's last neighbours, until a group of four is stored
+    };
+    union {
+        unsigned a[4][32];     // A operand: word t of row r at [t][r]
+        unsigned bits[2][32];  // sign bytes of a chunk's halves by lane
+    };
+    unsigned marks[kTileWords][32];  // of 32 waiting candidates, by lane; words from the last one down
+    int first[kTileWords];           // the last of them
+};
+
+__device__ __forceinline__ unsigned pack_h2(float lo, float hi)
+{
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const unsigned*>(&h);
+}
+
+__device__ __forceinline__ float2 unpack_h2(unsigned u)
+{
+    return __half22float2(*reinterpret_cast<const __half2*>(&u));
+}
+
+// D = A (16 x 8) B (8 x 8), fp16: d0 = row lane / 4, d1 = row lane / 4 + 8,
+// columns 2 (lane % 4) and + 1
+__device__ __forceinline__ void mma_16x8x8(unsigned& d0, unsigned& d1, unsigned a0, unsigned a1, unsigned b)
+{
+    asm("mma.sync.aligned.m16n8k8.row.col.f16.f16.f16.f16 {%0,%1}, {%2,%3}, {%4}, {%5,%5};"
+        : "=r"(d0), "=r"(d1)
+        : "r"(a0), "r"(a1), "r"(b), "r"(0u));
+}
+
+// Neighbour list and rho of the warp's particles k (one per lane; lanes with
+// !member have none). g, p: the lane's grid and parameters (the same in every
+// lane unless kWorlds, where `world` tells them apart). Returns the lane's
+// neighbour count, or -1 in every lane when the warp needs the general scan:
+// clamped cells, a stencil as wide as the grid (where it wraps onto itself)
+// or of more than 32 runs, or particles scattered over many rows.
+template <bool Fast, bool kWorlds>
+__device__ __forceinline__ int tile_neighbors(const GridDev& g, const float4* __restrict__ xs,
+                                              const nsph_sph_params& p, int world, float4 xi, bool member,
+                                              int4* __restrict__ nbr, int n, int k, TileSmem& sm, float& rho_out)
+{
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    rho_out = 0.f;
+    // a particle without a finite position has no neighbours
+    member = member && isfinite(xi.x) && isfinite(xi.y) && isfinite(xi.z);
+    int bx = 0, ex = 0, by = 0, ey = 0, bz = 0, ez = 0;
+    bool clamped = false;
+    if (member) {
+        box_axis_regular(xi.x, p.h, g.inv, g.dx, bx, ex, clamped);
+        box_axis_regular(xi.y, p.h, g.inv, g.dy, by, ey, clamped);
+        box_axis_regular(xi.z, p.h, g.inv, g.dz, bz, ez, clamped);
+        // a box as wide as the grid meets its own image
+        clamped |= ex - bx + 3 > g.dx || ey - by + 3 > g.dy || ez - bz + 3 > g.dz;
+        clamped |= (ey - by + 1) * (ez - bz + 1) > 16;
+    }
+    if (__any_sync(kAll, clamped)) return -1;
+    unsigned todo = __ballot_sync(kAll, member);
+    const int k_self = min(k, n - 1);
+    // Below this squared distance a candidate's cell is surely inside the box
+    // (its cell and the box ends are monotone in the coordinate up to three
+    // roundings each); nearer to h the cell is compared, since the definition
+    // visits a cell of the box and nothing else.
+    const float cells = fmaxf(fmaxf(fabsf(xi.x), fabsf(xi.y)), fabsf(xi.z)) * p.inv_h;
+    const float h2_safe = p.h2 * (1.f - (cells + 2.f) * 1.9073486e-6f);  // 2^-19 per cell
+
+    float rho = 0.f;
+    int cnt = 0, stored = 0;         // neighbours, and those in stored groups
+    int p0 = k, p1 = k, p2 = k;      // the cnt - stored < 4 others
+    int nw = kTileWords;             // words free
+    unsigned any = 0u;               // those with marks of this lane
+    int total = 0;                   // this lane's waiting marks
+
+    int groups = 0;
+    while (todo) {
+        // ---- the next group and its runs ----
+        const int lead = __ffs(todo) - 1;
+        const int lbx = __shfl_sync(kAll, bx, lead), lby = __shfl_sync(kAll, by, lead);
+        const int ley = __shfl_sync(kAll, ey, lead), lbz = __shfl_sync(kAll, bz, lead);
+        const int lez = __shfl_sync(kAll, ez, lead);
+        const int lworld = kWorlds ? __shfl_sync(kAll, world, lead) : world;
+        const bool mine = ((todo >> lane) & 1u) && by == lby && ey == ley && bz == lbz && ez == lez &&
+                          world == lworld && (unsigned)(bx - lbx) < (unsigned)kTileSpan;
+        const unsigned in_group = __ballot_sync(kAll, mine);
+        todo &= ~in_group;
+        if (++groups > 12 && todo) return -1;  // scattered particles: one thread each is cheaper
+        const int xe = __reduce_max_sync(kAll, mine ? ex : lbx);
+        const int x0 = __reduce_min_sync(kAll, mine ? bx : lbx);
+        int gdx = g.dx, gdy = g.dy, gdz = g.dz;
+        float inv_h = p.inv_h;
+        const int2* ranges = g.ranges;
+        if (kWorlds) {
+            gdx = __shfl_sync(kAll, g.dx, lead);
+            gdy = __shfl_sync(kAll, g.dy, lead);
+            gdz = __shfl_sync(kAll, g.dz, lead);
+            inv_h = __shfl_sync(kAll, p.inv_h, lead);
+            ranges = reinterpret_cast<const int2*>(
+                __shfl_sync(kAll, reinterpret_cast<unsigned long long>(g.ranges), lead));
+        }
+        const int nx = xe - x0 + 1;
+        if (nx + 2 > gdx) return -1;
+        // runs: row (z, y) of the box, in two parts where x wraps
+        const int ny = ley - lby + 1, rows = ny * (lez - lbz + 1);
+        const int cx0 = wrap_cell(x0, gdx);
+        const int wrap = min(nx, gdx - cx0);  // cells before the wrap
+        const bool two = wrap < nx;
+        int lo = 0x7fffffff, hi = 0;
+        {
+            const int row = two ? lane >> 1 : lane;
+            if (row < rows) {
+                const int iz = ny == 3 ? (row * 0x5556) >> 16 : row / ny, iy = row - iz * ny;
+                const int cz = wrap_cell(lbz + iz, gdz), cy = wrap_cell(lby + iy, gdy);
+                const bool second = two && (lane & 1);
+                const int2* cell = ranges + (cz * gdy + cy) * gdx + (second ? 0 : cx0);
+                const int cells_here = second ? nx - wrap : wrap;
+                // from the first cell with particles to the last (an empty cell reads 0, 0)
+                const int2 front = __ldg(cell), back = __ldg(cell + cells_here - 1);
+                lo = front.x;
+                hi = back.y;
+                if (front.y == front.x || back.y == back.x) {
+                    lo = 0x7fffffff;
+                    hi = 0;
+#pragma unroll 4
+                    for (int c = 0; c < cells_here; ++c) {
+                        const int2 se = __ldg(cell + c);
+                        if (se.y > se.x) {
+                            lo = min(lo, se.x);
+                            hi = max(hi, se.y);
+                        }
+                    }
+                }
+                if (lo < hi && !in_bounds(lo >= 0 && hi <= g.n)) hi = lo;
+            }
+        }
+        unsigned runs = __ballot_sync(kAll, lo < hi);
+
+        // ---- the A operand: rows (-2x, -2y | -2z, 1 | 1, n_hi | n_lo, 0) ----
+        const int last = 31 - __clz(in_group);
+        const float ox = 0.5f * (__shfl_sync(kAll, xi.x, lead) + __shfl_sync(kAll, xi.x, last));
+        const float oy = __shfl_sync(kAll, xi.y, lead), oz = __shfl_sync(kAll, xi.z, lead);
+        unsigned a0, a1, a2, a3;
+        {
+            const float ux = mine ? (xi.x - ox) * inv_h : 0.f, uy = mine ? (xi.y - oy) * inv_h : 0.f,
+                        uz = mine ? (xi.z - oz) * inv_h : 0.f;
+            const unsigned hxy = pack_h2(ux, uy), hz = pack_h2(uz, 0.f);
+            const float2 fxy = unpack_h2(hxy);
+            const float fz = unpack_h2(hz).x;
+            // the largest coordinates bound the fp16 rounding of a pair's
+            // difference: |u| 2^-11 for each of the two (a neighbour lies
+            // within 1 of its particle)
+            const float mx = __uint_as_float(__reduce_max_sync(kAll, __float_as_uint(fabsf(ux)))) + 1.01f;
+            const float myz =
+                __uint_as_float(__reduce_max_sync(kAll, __float_as_uint(fmaxf(fabsf(uy), fabsf(uz))))) + 1.01f;
+            const float d = 9.765625e-4f * sqrtf(mx * mx + 2.f * myz * myz);  // 2 x 2^-11
+            const float big = mx * mx + 2.f * myz * myz;
+            // (1 + d)^2, and 2^-16 of the largest partial sum for the
+            // products' sum and the splits
+            const float thr = (1.f + d) * (1.f + d) + 6.2e-5f * big;
+            const float n2 = fmaf(fz, fz, fmaf(fxy.y, fxy.y, fxy.x * fxy.x)) - thr;
+            const float n2h = unpack_h2(pack_h2(n2, 0.f)).x;
+            const unsigned w0 = pack_h2(-2.f * fxy.x, -2.f * fxy.y), w1 = pack_h2(-2.f * fz, 1.f);
+            const unsigned w2 = pack_h2(1.f, n2h), w3 = pack_h2(n2 - n2h, 0.f);
+            if (!(big < 4096.f)) return -1;  // cells far wider than h: the norms leave fp16's range
+            __syncwarp();  // (the last chunk's sign bytes are read)
+            sm.a[0][lane] = w0;
+            sm.a[1][lane] = w1;
+            sm.a[2][lane] = w2;
+            sm.a[3][lane] = w3;
+            __syncwarp();
+            const unsigned* a = &sm.a[lane & 3][lane >> 2];
+            a0 = a[0];
+            a1 = a[8];
+            a2 = a[16];
+            a3 = a[24];
+            __syncwarp();
+        }
+
+        // ---- chunks of 64 candidates (a dense run has about 50) ----
+        sm.frag[0][3][lane] = sm.frag[1][3][lane] = 0x00003c00u;  // k = 6, 7 of B: (1, 0)
+        int c0 = 0, end = 0;
+        float4 q[2];
+        bool more;
+        auto next_chunk = [&]() {  // and issue the loads of its candidates
+            c0 += 64;
+            if (c0 >= end) {
+                more = runs != 0u;
+                if (!more) return;
+                const int r = __ffs(runs) - 1;
+                runs &= runs - 1u;
+                c0 = __shfl_sync(kAll, lo, r);
+                end = __shfl_sync(kAll, hi, r);
+            }
+            q[0] = __ldg(xs + min(c0 + lane, end - 1));
+            q[1] = __ldg(xs + min(c0 + 32 + lane, end - 1));
+        };
+        q[0] = q[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        more = true;
+        next_chunk();
+        do {
+            if (more) {
+                const int at = c0, m = end - c0;
+                const int halves = m > 32 ? 2 : 1;
+                unsigned counted[2] = {0u, 0u};
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    if (h >= halves) break;
+                    const float ux = (q[h].x - ox) * inv_h, uy = (q[h].y - oy) * inv_h, uz = (q[h].z - oz) * inv_h;
+                    const unsigned hxy = pack_h2(ux, uy);
+                    const float2 fxy = unpack_h2(hxy);
+                    const float fz = unpack_h2(pack_h2(uz, 0.f)).x;
+                    const float n2 = fmaf(fz, fz, fmaf(fxy.y, fxy.y, fxy.x * fxy.x));
+                    const unsigned w1 = pack_h2(fz, n2);
+                    sm.frag[h][0][lane] = hxy;
+                    sm.frag[h][1][lane] = w1;
+                    sm.frag[h][2][lane] = pack_h2(n2 - unpack_h2(w1).y, 1.f);
+                    // past the run's end and inactive (in no list): no mark
+                    counted[h] = __ballot_sync(kAll, 32 * h + lane < m && !mirror_inactive(q[h]));
+                }
+                next_chunk();
+                __syncwarp();
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    if (h >= halves) break;
+                    // column j of tile i is candidate 4 j + i
+                    const uint4 b = *reinterpret_cast<const uint4*>(&sm.frag[h][lane & 3][lane & ~3]);
+                    unsigned acc = 0u;
+                    const unsigned bw[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        unsigned d0, d1, d2, d3;
+                        mma_16x8x8(d0, d1, a0, a1, bw[i]);
+                        mma_16x8x8(d2, d3, a2, a3, bw[i]);
+                        // the four signs as bytes 0 or 0xff (sign-replicating selectors)
+                        unsigned s01, s23;
+                        asm("prmt.b32 %0, %1, %2, 0xfdb9;" : "=r"(s01) : "r"(d0), "r"(d1));
+                        asm("prmt.b32 %0, %1, %2, 0xfdb9;" : "=r"(s23) : "r"(d2), "r"(d3));
+                        acc |= s01 & (0x01010101u << i);
+                        acc |= s23 & (0x10101010u << i);
+                    }
+                    sm.bits[h][lane] = acc;
+                }
+                __syncwarp();
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    if (h >= halves) break;
+                    // this lane's row from the four lanes that hold its columns
+                    const uint4 v = *reinterpret_cast<const uint4*>(&sm.bits[h][4 * (lane & 7)]);
+                    const unsigned sel = (lane & 8) ? 0x7632u : 0x5410u;
+                    const int sh = (lane & 16) ? 4 : 0;
+                    unsigned y0 = (__byte_perm(v.x, v.y, sel) >> sh) & 0x0f0f0f0fu;
+                    unsigned y1 = (__byte_perm(v.z, v.w, sel) >> sh) & 0x0f0f0f0fu;
+                    y0 |= y0 >> 4;
+                    y1 |= y1 >> 4;
+                    const unsigned marks = __byte_perm(y0, y1, 0x6420u) & (mine ? counted[h] : 0u);
+                    // kept so that the order is from the top bit down
+                    --nw;
+                    sm.marks[nw][lane] = __brev(marks);
+                    if (lane == 0) sm.first[nw] = at + 32 * h + 31;
+                    any |= (marks != 0u ? 1u : 0u) << nw;
+                    total += __popc(marks);
+                }
+            }
+            if (nw < 2 || !(more || todo)) {
+                // ---- the walk over the waiting marks ----
+                // without branches on the way; a lane that has run out visits
+                // its own particle in vain
+                const int most = __reduce_max_sync(kAll, total);
+                __syncwarp();  // first[], and the last reads of frag
+                auto push = [&](int j) {
+                    sm.ring[cnt & 7][lane] = j;
+                    ++cnt;
+                };
+                sm.ring[stored & 7][lane] = p0;
+                sm.ring[(stored + 1) & 7][lane] = p1;
+                sm.ring[(stored + 2) & 7][lane] = p2;
+                unsigned cur = 0u;
+                int jb = 0;
+                auto pop = [&](int t) {
+                    const int c = max(31 - __clz(any), 0);
+                    const unsigned word = sm.marks[c][lane];
+                    const int base = sm.first[c];
+                    const bool dry = cur == 0u;
+                    cur = dry ? word : cur;
+                    jb = dry ? base : jb;
+                    any = dry ? any & ~(1u << c) : any;
+                    const int b = 31 - __clz(cur);
+                    cur &= ~(1u << (b & 31));
+                    return t < total ? jb - b : k_self;
+                };
+                int j = pop(0);
+                float4 xj = __ldg(xs + j);
+                for (int t0 = 0; t0 < most; t0 += 4) {
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int t = t0 + u;
+                        const int jn = pop(t + 1);
+                        const float4 xn = __ldg(xs + jn);
+                        float dx, dy, dz;
+                        const float r2 = dist2(xi, xj, dx, dy, dz);
+                        const float rho1 = __fmaf_rn(xj.w, Fast ? wterm_fast(r2, p) : wterm_near(r2, p), rho);
+                        const bool valid = t < total, inside = r2 < h2_safe;
+                        // near the support's edge, or closer than 2^-50: rare
+                        if (valid && (!inside || __float_as_uint(r2) - 1u < 0x0d7fffffu)) {
+                            const int cx = trunc_sat(__fmul_rn(xj.x, g.inv)), cy = trunc_sat(__fmul_rn(xj.y, g.inv)),
+                                      cz = trunc_sat(__fmul_rn(xj.z, g.inv));
+                            if (r2 < p.h2 && cx >= bx && cx <= ex && cy >= by && cy <= ey && cz >= bz && cz <= ez) {
+                                push(j);
+                                rho = __fmaf_rn(xj.w, Fast ? wterm_fast(r2, p) : wterm(r2, p), rho);
+                            }
+                        } else if (valid) {
+                            rho = rho1;
+                            push(j);
+                        }
+                        j = jn;
+                        xj = xn;
+                    }
+                    if (cnt - stored >= 4) {  // (at most seven are in the ring)
+                        const int* r = &sm.ring[stored & 7][lane];
+                        if (stored < kNbrSlots)
+                            nbr[(size_t)(stored >> 2) * n + k] = make_int4(r[0], r[32], r[64], r[96]);
+                        stored += 4;
+                    }
+                }
+                const int* r = &sm.ring[stored & 7][lane];
+                p0 = r[0];
+                p1 = r[32];
+                p2 = r[64];
+                __syncwarp();
+                nw = kTileWords;
+                total = 0;
+                any = 0u;
+                sm.frag[0][3][lane] = sm.frag[1][3][lane] = 0x00003c00u;
+            }
+        } while (more);
+    }
+    // the last, partial group: the rest of it is filled with the particle itself
+    const int rest = cnt - stored;
+    if (rest > 0 && cnt <= kNbrSlots)
+        nbr[(size_t)(stored >> 2) * n + k] = make_int4(p0, rest > 1 ? p1 : k, rest > 2 ? p2 : k, k);
+    rho_out = rho;
+    return cnt;
+}
+
 struct ForceAcc {
     float ax, ay, az, dvx, dvy, dvz;
 };
 
-// pressure and XSPH terms of one neighbour (not self), accumulated in order
-__device__ __forceinline__ void force_term_data(float4 xj, float4 vj, float2 aj, float4 xi, float4 vi, float pr2_i,
-                                                const nsph_sph_params& p, ForceAcc& acc)
+// the constants that a force term reads (of one world, or of all particles)
+struct ForceConst {
+    float inv_h, sigma, c_near, c_far;
+    __device__ __forceinline__ explicit ForceConst(const nsph_sph_params& p)
+        : inv_h(p.inv_h), sigma(p.sigma), c_near(p.c_near), c_far(p.c_far)
+    {
+    }
+};
+
+// Pressure and XSPH terms of one neighbour: a -= s d, dv += c u, accumulated
+// in order (not of the particle itself). A coincident one has no pressure term.
+struct ForceTerm {
+    float s, dx, dy, dz, c, ux, uy, uz;
+};
+
+template <class P>
+__device__ __forceinline__ ForceTerm force_factors(float4 xj, float4 vj, float pr2_j, float4 xi, float4 vi, float pr2_i,
+                                                   const P& p)
 {
-    if (!(__float_as_int(vj.w) & kAttrActive)) return;
-    float dx, dy, dz;
-    const float r2 = dist2(xi, xj, dx, dy, dz);
-    const float r = __fsqrt_rn(r2);
+    ForceTerm t;
+    const float r2 = dist2(xi, xj, t.dx, t.dy, t.dz);
+    float r, inv_r;
+    if (plain_range(r2)) {
+        float y;
+        r = sqrt_plain(r2, y);
+        inv_r = rcp_plain(r, y);  // (not a number for r = 0, where it is not used)
+    } else {
+        r = __fsqrt_rn(r2);
+        inv_r = __frcp_rn(r);
+    }
     const float q = __fmul_rn(r, p.inv_h);
     const float w = kernel_w(q, p);
-    if (r2 > 0.f) {
-        const float f = kernel_f(q, __frcp_rn(r), p);
-        const float s = __fmul_rn(__fmul_rn(xj.w, __fadd_rn(pr2_i, aj.y)), f);
-        acc.ax = __fmaf_rn(-s, dx, acc.ax);
-        acc.ay = __fmaf_rn(-s, dy, acc.ay);
-        acc.az = __fmaf_rn(-s, dz, acc.az);
-    }
-    const float c = __fmul_rn(aj.x, w);
-    acc.dvx = __fmaf_rn(c, __fsub_rn(vj.x, vi.x), acc.dvx);
-    acc.dvy = __fmaf_rn(c, __fsub_rn(vj.y, vi.y), acc.dvy);
-    acc.dvz = __fmaf_rn(c, __fsub_rn(vj.z, vi.z), acc.dvz);
+    const float f = kernel_f(q, inv_r, p);
+    t.s = r2 > 0.f ? __fmul_rn(__fmul_rn(xj.w, __fadd_rn(pr2_i, pr2_j)), f) : 0.f;
+    t.c = __fmul_rn(vj.w, w);
+    t.ux = __fsub_rn(vj.x, vi.x);
+    t.uy = __fsub_rn(vj.y, vi.y);
+    t.uz = __fsub_rn(vj.z, vi.z);
+    return t;
+}
+
+template <class P>
+__device__ __forceinline__ void force_term_data(float4 xj, float4 vj, float pr2_j, float4 xi, float4 vi, float pr2_i,
+                                                const P& p, ForceAcc& acc)
+{
+    const ForceTerm t = force_factors(xj, vj, pr2_j, xi, vi, pr2_i, p);
+    acc.ax = __fmaf_rn(-t.s, t.dx, acc.ax);
+    acc.ay = __fmaf_rn(-t.s, t.dy, acc.ay);
+    acc.az = __fmaf_rn(-t.s, t.dz, acc.az);
+    acc.dvx = __fmaf_rn(t.c, t.ux, acc.dvx);
+    acc.dvy = __fmaf_rn(t.c, t.uy, acc.dvy);
+    acc.dvz = __fmaf_rn(t.c, t.uz, acc.dvz);
 }
 
 // force_term_data in the tolerance arithmetic (see kernel_w_fast)
-__device__ __forceinline__ void force_term_fast(float4 xj, float4 vj, float2 aj, float4 xi, float4 vi, float pr2_i,
-                                                const nsph_sph_params& p, ForceAcc& acc)
+template <class P>
+__device__ __forceinline__ void force_term_fast(float4 xj, float4 vj, float pr2_j, float4 xi, float4 vi, float pr2_i,
+                                                const P& p, ForceAcc& acc)
 {
-    if (!(__float_as_int(vj.w) & kAttrActive)) return;
     const float dx = xi.x - xj.x, dy = xi.y - xj.y, dz = xi.z - xj.z;
     const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
     float w = p.sigma;
@@ -356,12 +853,12 @@ __device__ __forceinline__ void force_term_fast(float4 xj, float4 vj, float2 aj,
         const float t = 1.f - q;
         w = kernel_w_fast(q, p);
         const float f = q <= 0.5f ? p.c_near * fmaf(3.f, q, -2.f) : (q < 1.f ? p.c_far * t * t * ir : 0.f);
-        const float s = xj.w * (pr2_i + aj.y) * f;
+        const float s = xj.w * (pr2_i + pr2_j) * f;
         acc.ax -= s * dx;
         acc.ay -= s * dy;
         acc.az -= s * dz;
     }
-    const float c = aj.x * w;
+    const float c = vj.w * w;
     acc.dvx += c * (vj.x - vi.x);
     acc.dvy += c * (vj.y - vi.y);
     acc.dvz += c * (vj.z - vi.z);
@@ -378,6 +875,7 @@ struct StepOut {
     float* a_out;
     unsigned* status;
     float4* acc_sorted;  // or null: (a, 0), (dv, 0) of sorted particle k at 2k, 2k + 1 (the segment tape)
+    bool carry_v;        // write inactive particles' velocities too (unchanged; a step leaves them alone)
 };
 
 // integrate particle k (original index i) and scatter its outputs
@@ -391,6 +889,11 @@ __device__ __forceinline__ void integrate_out(size_t i, float4 xi, float4 vi, in
         o.x_out[3 * i + 0] = xi.x;
         o.x_out[3 * i + 1] = xi.y;
         o.x_out[3 * i + 2] = xi.z;
+        if (o.carry_v) {
+            o.v_out[3 * i + 0] = vi.x;
+            o.v_out[3 * i + 1] = vi.y;
+            o.v_out[3 * i + 2] = vi.z;
+        }
         if (o.a_out) o.a_out[3 * i + 0] = o.a_out[3 * i + 1] = o.a_out[3 * i + 2] = 0.f;
         return;
     }
@@ -445,75 +948,83 @@ __device__ __forceinline__ void integrate_out(size_t i, float4 xi, float4 vi, in
 }
 
 // ---- the plain step's passes on neighbour lists ----------------------------------
-// Bounded to 48 registers (4 bytes of spills): 40 resident warps per SM.
 template <bool Fast>
-__global__ void __launch_bounds__(kSphThreads, 5) k_density_list(GridDev g, const float4* __restrict__ xs,
-                                                                 const float4* __restrict__ vs, int n,
-                                                                 const __grid_constant__ nsph_sph_params p,
-                                                                 float2* __restrict__ aux, float2* __restrict__ rp,
-                                                                 int4* __restrict__ nbr, int* __restrict__ ncnt,
-                                                                 unsigned* __restrict__ status)
+__global__ void __launch_bounds__(kSphThreads, kDensityBlocks) k_density_list(
+    const __grid_constant__ GridDev g, const float4* __restrict__ xs, const float4* __restrict__ vs, int n,
+    const __grid_constant__ nsph_sph_params p, float2* __restrict__ aux, float2* __restrict__ rp,
+    int4* __restrict__ nbr, int* __restrict__ ncnt, const ForceRec fr, unsigned* __restrict__ status)
 {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const float4 xi = xs[k];
-        if (!(__float_as_int(vs[k].w) & kAttrActive)) {
+    launch_entry();
+    extern __shared__ TileSmem tile_smem[];
+    TileSmem& sm = tile_smem[threadIdx.x >> 5];
+    // whole warps: lanes past n take part as non-members
+    for (int k0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); k0 < n; k0 += gridDim.x * blockDim.x) {
+        const int k = k0 + (threadIdx.x & 31);
+        const bool live = k < n;
+        float4 xi = make_float4(0.f, 0.f, 0.f, 0.f);
+        bool active = false;
+        if (live) {
+            xi = xs[k];
+            active = (__float_as_int(vs[k].w) & kAttrActive) != 0;
+        }
+        float rho;
+        int cnt = tile_neighbors<Fast, false>(g, xs, p, 0, xi, active, nbr, n, k, sm, rho);
+        if (active) {
+            if (cnt < 0) cnt = scan_general<Fast>(&g, xs, &p, xi, nbr, n, k, &rho);
+            ncnt[k] = cnt;
+            if (cnt > kNbrSlots && fr.overflow) atomicOr(fr.overflow, 1u);
+            density_finish<Fast>(k, xi, vs[k], rho, p, aux, rp, fr, status);
+        } else if (live) {
             aux[k] = make_float2(0.f, 0.f);
             rp[k] = make_float2(0.f, 0.f);
+            fr.rec[2 * (size_t)k] = xi;  // (marked inactive)
             ncnt[k] = 0;
-            continue;
         }
-        const int cnt = neighbor_list<true>(g, xs, p, xi, nbr, n, k);
-        ncnt[k] = cnt;
-        const float rho = density_from_list<Fast>(g, xs, p, xi, nbr, cnt, n, k);
-        density_finish<Fast>(k, xi.w, rho, p, aux, rp, status);
     }
 }
 
-// pressure and XSPH sums of particle k over its list, in order (loads of
-// neighbour t+1 issued before the terms of neighbour t), or by re-testing
-// its candidates when the list overflowed
-template <bool Fast, bool kUnrolledWalk = true>
-__device__ __forceinline__ void force_from_list(const GridDev& g, const float4* __restrict__ xs,
-                                                const float4* __restrict__ vs, const float2* __restrict__ aux,
-                                                const int4* __restrict__ nbr, int cnt, int n, int k, float4 xi,
-                                                float4 vi, float pr2_i, const nsph_sph_params& p, ForceAcc& acc)
+// pressure and XSPH sums of particle k over its list, in order, by whole
+// groups (the last one is filled with the particle itself): the loads of two
+// neighbours are issued together, those of the next group's indices ahead. A
+// particle whose list overflowed re-tests its candidates.
+template <bool Fast, class P>
+__device__ __forceinline__ void force_from_list(const GridDev& g, const ForceRec& fr, const int4* __restrict__ nbr,
+                                                int cnt, int n, int k, float4 xi, float4 vi, float h, float h2,
+                                                const P& p, ForceAcc& acc)
 {
+    const float pr2_i = fr.pr2[k];
+    auto term = [&](const Neighbour& o, float pr2_j) {
+        if (Fast)
+            force_term_fast(o.x, o.v, pr2_j, xi, vi, pr2_i, p, acc);
+        else
+            force_term_data(o.x, o.v, pr2_j, xi, vi, pr2_i, p, acc);
+    };
+    auto checked = [&](int j) { return in_bounds(j >= 0 && j < n) ? j : 0; };
     if (cnt <= kNbrSlots) {
-        bool have = false;
-        float4 pxj = make_float4(0.f, 0.f, 0.f, 0.f), pvj = pxj;
-        float2 paj = make_float2(0.f, 0.f);
-        for_each_listed<true, kUnrolledWalk>(nbr, n, k, cnt, [&](int j) {
-            if (j == k) return;
-            const float4 nxj = __ldg(xs + j);
-            const float4 nvj = __ldg(vs + j);
-            const float2 naj = __ldg(aux + j);
-            if (have) {
-                if (Fast)
-                    force_term_fast(pxj, pvj, paj, xi, vi, pr2_i, p, acc);
-                else
-                    force_term_data(pxj, pvj, paj, xi, vi, pr2_i, p, acc);
+        const int4* a = nbr + k;
+        int4 next = cnt > 0 ? __ldg(a) : make_int4(k, k, k, k);
+#pragma unroll 1
+        for (int t = 0; t < cnt; t += 4) {
+            const int4 gr = next;
+            a += n;
+            if (t + 4 < cnt) next = __ldg(a);
+#pragma unroll
+            for (int u = 0; u < 4; u += 2) {
+                const int j0 = checked(group_item(gr, u)), j1 = checked(group_item(gr, u + 1));
+                const Neighbour o0 = load_neighbour(fr.rec, j0);
+                const float p0 = __ldg(fr.pr2 + j0);
+                const Neighbour o1 = load_neighbour(fr.rec, j1);
+                const float p1 = __ldg(fr.pr2 + j1);
+                if (j0 != k) term(o0, p0);
+                if (j1 != k) term(o1, p1);
             }
-            pxj = nxj;
-            pvj = nvj;
-            paj = naj;
-            have = true;
-        });
-        if (have) {
-            if (Fast)
-                force_term_fast(pxj, pvj, paj, xi, vi, pr2_i, p, acc);
-            else
-                force_term_data(pxj, pvj, paj, xi, vi, pr2_i, p, acc);
         }
     } else {
-        for_each_run(g, xi.x, xi.y, xi.z, p.h, [&](int lo, int hi) {
+        for_each_run(g, xi.x, xi.y, xi.z, h, [&](int lo, int hi) {
             for (int j = lo; j < hi; ++j) {
+                const Neighbour o = load_neighbour(fr.rec, j);
                 float dx, dy, dz;
-                if (dist2(xi, __ldg(xs + j), dx, dy, dz) < p.h2 && j != k) {
-                    if (Fast)
-                        force_term_fast(__ldg(xs + j), __ldg(vs + j), __ldg(aux + j), xi, vi, pr2_i, p, acc);
-                    else
-                        force_term_data(__ldg(xs + j), __ldg(vs + j), __ldg(aux + j), xi, vi, pr2_i, p, acc);
-                }
+                if (dist2(xi, o.x, dx, dy, dz) < h2 && j != k && !mirror_inactive(o.x)) term(o, __ldg(fr.pr2 + j));
             }
         });
     }
@@ -521,24 +1032,122 @@ __device__ __forceinline__ void force_from_list(const GridDev& g, const float4* 
 
 template <bool Fast>
 __global__ void __launch_bounds__(kSphThreads, 4) k_force_list(GridDev g, const float4* __restrict__ xs,
-                                                               const float4* __restrict__ vs,
-                                                               const float2* __restrict__ aux,
+                                                               const float4* __restrict__ vs, const ForceRec fr,
                                                                const float2* __restrict__ rp, int n,
                                                                const __grid_constant__ nsph_sph_params p,
                                                                const int4* __restrict__ nbr,
                                                                const int* __restrict__ ncnt, const StepOut o)
 {
+    launch_entry();
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const float4 xi = xs[k], vi = vs[k];
         const int attr = __float_as_int(vi.w);
         ForceAcc acc{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        if (attr & kAttrActive) force_from_list<Fast>(g, xs, vs, aux, nbr, ncnt[k], n, k, xi, vi, aux[k].y, p, acc);
+        if (attr & kAttrActive) force_from_list<Fast>(g, fr, nbr, ncnt[k], n, k, xi, vi, p.h, p.h2, p, acc);
         if (o.acc_sorted) {  // the force sums, for the adjoint's segment tape
             o.acc_sorted[2 * (size_t)k] = make_float4(acc.ax, acc.ay, acc.az, 0.f);
             o.acc_sorted[2 * (size_t)k + 1] = make_float4(acc.dvx, acc.dvy, acc.dvz, 0.f);
         }
         integrate_out((size_t)g.ids[k], xi, vi, attr, rp[k], acc, p, p.dt, o);
     }
+}
+
+// The force pass of a small scene: four lanes per particle. Lane u of a
+// particle evaluates the factors of item u of each list group; the factors
+// cross through shared memory, and lanes 0 .. 2 accumulate the x, y and z sums
+// of the group's four terms in order, so every rounding is k_force_list's.
+// It spends about 1.4 times the instructions, but a particle's chain of
+// dependent work is a third as long and there are four times the warps, which
+// is what bounds scenes that do not fill the SMs.
+constexpr int kQuadThreads = 256;
+constexpr int kQuadMax = 131072;
+
+__global__ void __launch_bounds__(kQuadThreads, 4) k_force_quad(const __grid_constant__ GridDev g,
+                                                                const float4* __restrict__ xs,
+                                                                const float4* __restrict__ vs,
+                                                                const ForceRec fr, const float2* __restrict__ rp,
+                                                                int n, const __grid_constant__ nsph_sph_params p,
+                                                                const int4* __restrict__ nbr,
+                                                                const int* __restrict__ ncnt, const StepOut o)
+{
+    launch_entry();
+    constexpr unsigned kAll = 0xffffffffu;
+    __shared__ __align__(16) float cross[kQuadThreads / 32][2][8][32];  // [parity][factor][lane]
+    const int lane = threadIdx.x & 31, u = lane & 3;
+    const int kt = (blockIdx.x * kQuadThreads + threadIdx.x) >> 2;
+    const int k = min(kt, n - 1);
+    const float4 xi = xs[k], vi = vs[k];
+    const int attr = __float_as_int(vi.w);
+    const bool active = kt < n && (attr & kAttrActive);
+    const int cnt = active ? ncnt[k] : 0;
+    const float pr2_i = fr.pr2[k];
+    const int groups = cnt <= kNbrSlots ? (cnt + 3) >> 2 : 0;  // an overflowed list: see below
+    const int most = __reduce_max_sync(kAll, groups);
+    const int* item = reinterpret_cast<const int*>(nbr + k) + u;
+    auto load = [&](int gi) {
+        const int j = gi < groups ? __ldg(item + 4 * (size_t)gi * n) : k;
+        return in_bounds(j >= 0 && j < n) ? j : 0;
+    };
+    const int axis = min(u, 2);
+    float a = 0.f, dv = 0.f;
+    int j = load(0), jn = load(1);
+    Neighbour oj = load_neighbour(fr.rec, j);
+    float pj = __ldg(fr.pr2 + j);
+    for (int gi = 0; gi < most; ++gi) {
+        // the next group's data and the index after it go out first
+        const int j1 = jn;
+        const Neighbour on = load_neighbour(fr.rec, j1);
+        const float pn = __ldg(fr.pr2 + j1);
+        jn = load(gi + 2);
+        const unsigned live = __ballot_sync(kAll, j != k);  // (fillers are the particle itself)
+        const ForceTerm t = force_factors(oj.x, oj.v, pj, xi, vi, pr2_i, p);
+        float(*c)[32] = cross[threadIdx.x >> 5][gi & 1];
+        c[0][lane] = t.dx;
+        c[1][lane] = t.dy;
+        c[2][lane] = t.dz;
+        c[3][lane] = -t.s;
+        c[4][lane] = t.ux;
+        c[5][lane] = t.uy;
+        c[6][lane] = t.uz;
+        c[7][lane] = t.c;
+        __syncwarp();
+        const int row = lane & ~3;
+        const float4 d = *reinterpret_cast<const float4*>(&c[axis][row]);
+        const float4 s = *reinterpret_cast<const float4*>(&c[3][row]);
+        const float4 w = *reinterpret_cast<const float4*>(&c[4 + axis][row]);
+        const float4 m = *reinterpret_cast<const float4*>(&c[7][row]);
+        const unsigned in = (live >> row) & 15u;  // the group's items that are neighbours
+        auto add = [&](unsigned bit, float sv, float dvv, float mv, float wv) {
+            if (in & bit) {
+                a = __fmaf_rn(sv, dvv, a);
+                dv = __fmaf_rn(mv, wv, dv);
+            }
+        };
+        add(1u, s.x, d.x, m.x, w.x);
+        add(2u, s.y, d.y, m.y, w.y);
+        add(4u, s.z, d.z, m.z, w.z);
+        add(8u, s.w, d.w, m.w, w.w);
+        j = j1;
+        oj = on;
+        pj = pn;
+    }
+    ForceAcc acc;
+    acc.ax = a;
+    acc.dvx = dv;
+    acc.ay = __shfl_down_sync(kAll, a, 1, 4);
+    acc.dvy = __shfl_down_sync(kAll, dv, 1, 4);
+    acc.az = __shfl_down_sync(kAll, a, 2, 4);
+    acc.dvz = __shfl_down_sync(kAll, dv, 2, 4);
+    if (u != 0 || kt >= n) return;
+    if (cnt > kNbrSlots) {
+        acc = ForceAcc{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        force_from_list<false>(g, fr, nbr, cnt, n, k, xi, vi, p.h, p.h2, p, acc);
+    }
+    if (o.acc_sorted) {  // the force sums, for the adjoint's segment tape
+        o.acc_sorted[2 * (size_t)k] = make_float4(acc.ax, acc.ay, acc.az, 0.f);
+        o.acc_sorted[2 * (size_t)k + 1] = make_float4(acc.dvx, acc.dvy, acc.dvz, 0.f);
+    }
+    integrate_out((size_t)g.ids[k], xi, vi, attr, rp[k], acc, p, p.dt, o);
 }
 
 // ---- batched worlds ------------------------------------------------------------
@@ -555,36 +1164,51 @@ __device__ __forceinline__ GridDev world_grid(const WorldCells& c, const int2* _
     return GridDev{c.dx, c.dy, c.dz, c.inv, ranges + c.off, ids, n};
 }
 
-// Bounded to 64 registers (36 bytes of spills outside the candidate loop):
-// 5.81 -> 5.18 ms per pass on worlds_4096 against its unbounded 80 (same
-// box, back to back); a reference into the parameter table instead of the
-// copy was slower at 64 (5.41) and at 48 registers (5.53).
-__global__ void __launch_bounds__(kSphThreads, 4) k_density_worlds(const WorldCells* __restrict__ wc,
-                                                                   const nsph_sph_params* __restrict__ wp,
-                                                                   const int2* __restrict__ ranges,
-                                                                   const int* __restrict__ ids,
-                                                                   const float4* __restrict__ xs,
-                                                                   const float4* __restrict__ vs, int n,
-                                                                   float2* __restrict__ aux, float2* __restrict__ rp,
-                                                                   int4* __restrict__ nbr, int* __restrict__ ncnt,
-                                                                   unsigned* __restrict__ status)
+// scan_general of a particle of world w
+__device__ __noinline__ int scan_general_world(const WorldCells* wc, const nsph_sph_params* wp, const int2* ranges,
+                                               const int* ids, int w, const float4* xs, float4 xi, int4* nbr, int n,
+                                               int k, float* rho)
 {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const float4 xi = xs[k];
-        const int attr = __float_as_int(vs[k].w);
-        if (!(attr & kAttrActive)) {
-            aux[k] = make_float2(0.f, 0.f);
-            rp[k] = make_float2(0.f, 0.f);
-            ncnt[k] = 0;
-            continue;
+    const GridDev g = world_grid(wc[w], ranges, ids, n);
+    const int cnt = neighbor_list(g, xs, wp[w], xi, nbr, n, k);
+    *rho = density_from_list<false>(g, xs, wp[w], xi, nbr, cnt, n, k);
+    return cnt;
+}
+
+__global__ void __launch_bounds__(kSphThreads, kDensityBlocks) k_density_worlds(
+    const WorldCells* __restrict__ wc, const nsph_sph_params* __restrict__ wp, const int2* __restrict__ ranges,
+    const int* __restrict__ ids, const float4* __restrict__ xs, const float4* __restrict__ vs, int n,
+    float2* __restrict__ aux, float2* __restrict__ rp, int4* __restrict__ nbr, int* __restrict__ ncnt,
+    const ForceRec fr, unsigned* __restrict__ status)
+{
+    launch_entry();
+    extern __shared__ TileSmem tile_smem[];
+    TileSmem& sm = tile_smem[threadIdx.x >> 5];
+    for (int k0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); k0 < n; k0 += gridDim.x * blockDim.x) {
+        const int k = k0 + (threadIdx.x & 31);
+        const bool live = k < n;
+        float4 xi = make_float4(0.f, 0.f, 0.f, 0.f);
+        int attr = 0;
+        if (live) {
+            xi = xs[k];
+            attr = __float_as_int(vs[k].w);
         }
+        const bool active = (attr & kAttrActive) != 0;
         const int w = attr >> kAttrGravShift;
         const nsph_sph_params p = wp[w];  // a copy: its fields stay in registers across the candidate loop
         const GridDev g = world_grid(wc[w], ranges, ids, n);
-        const int cnt = neighbor_list<false>(g, xs, p, xi, nbr, n, k);
-        ncnt[k] = cnt;
-        const float rho = density_from_list<false>(g, xs, p, xi, nbr, cnt, n, k);
-        density_finish(k, xi.w, rho, p, aux, rp, status);
+        float rho;
+        int cnt = tile_neighbors<false, true>(g, xs, p, w, xi, active, nbr, n, k, sm, rho);
+        if (active) {
+            if (cnt < 0) cnt = scan_general_world(wc, wp, ranges, ids, w, xs, xi, nbr, n, k, &rho);
+            ncnt[k] = cnt;
+            density_finish(k, xi, vs[k], rho, p, aux, rp, fr, status);
+        } else if (live) {
+            aux[k] = make_float2(0.f, 0.f);
+            rp[k] = make_float2(0.f, 0.f);
+            fr.rec[2 * (size_t)k] = xi;  // (marked inactive)
+            ncnt[k] = 0;
+        }
     }
 }
 
@@ -595,12 +1219,12 @@ __global__ void __launch_bounds__(kSphThreads, 4) k_force_worlds(const WorldCell
                                                                  const int2* __restrict__ ranges,
                                                                  const int* __restrict__ ids,
                                                                  const float4* __restrict__ xs,
-                                                                 const float4* __restrict__ vs,
-                                                                 const float2* __restrict__ aux,
+                                                                 const float4* __restrict__ vs, const ForceRec fr,
                                                                  const float2* __restrict__ rp, int n, float dt,
                                                                  const int4* __restrict__ nbr,
                                                                  const int* __restrict__ ncnt, const StepOut o)
 {
+    launch_entry();
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const float4 xi = xs[k], vi = vs[k];
         const int attr = __float_as_int(vi.w);
@@ -608,7 +1232,7 @@ __global__ void __launch_bounds__(kSphThreads, 4) k_force_worlds(const WorldCell
         const nsph_sph_params& p = wp[w];
         const GridDev g = world_grid(wc[w], ranges, ids, n);
         ForceAcc acc{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        if (attr & kAttrActive) force_from_list<false, false>(g, xs, vs, aux, nbr, ncnt[k], n, k, xi, vi, aux[k].y, p, acc);
+        if (attr & kAttrActive) force_from_list<false>(g, fr, nbr, ncnt[k], n, k, xi, vi, p.h, p.h2, ForceConst(p), acc);
         integrate_out((size_t)ids[k], xi, vi, attr, rp[k], acc, p, dt, o);
     }
 }
@@ -619,6 +1243,7 @@ __global__ void k_neighbors_worlds(const WorldCells* __restrict__ wc, const nsph
                                    int* __restrict__ counts, const long long* __restrict__ offsets,
                                    int* __restrict__ out)
 {
+    launch_entry();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const int i = ids[k];
@@ -646,6 +1271,7 @@ __global__ void k_neighbors(GridDev g, const float4* __restrict__ xs, const floa
                             nsph_sph_params p, int* __restrict__ counts, const long long* __restrict__ offsets,
                             int* __restrict__ out)
 {
+    launch_entry();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const int i = g.ids[k];
@@ -664,6 +1290,19 @@ __global__ void k_neighbors(GridDev g, const float4* __restrict__ xs, const floa
         });
     }
     if (!out) counts[i] = c;
+}
+
+// The part of a step's grid that its reverse reads, into the segment tape: the
+// sorted ids and, only when a list of the step overflowed (its particle's
+// neighbours are then found through the grid again), the cell table.
+__global__ void k_tape_copy(const GridDev g, long long ncells, int n, const unsigned* __restrict__ overflow,
+                            int* __restrict__ ids, int2* __restrict__ ranges)
+{
+    launch_entry();
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+    for (long long k = t; k < n; k += step) ids[k] = g.ids[k];
+    if (*overflow)
+        for (long long c = t; c < ncells; c += step) ranges[c] = g.ranges[c];
 }
 
 // ==========================================================================
@@ -702,24 +1341,47 @@ __device__ __forceinline__ float kernel_df_over_r(float q, float inv_r, const ns
 
 // visit(j) for every neighbour j != k of sorted particle k, in query order,
 // from the density pass's neighbour list (re-testing its candidates when the
-// list overflowed)
-template <class V>
+// list overflowed). With kLanes = 4, lane `sub` of the particle's four visits
+// item `sub` of each list group (or every fourth candidate).
+template <int kLanes, class V>
 __device__ __forceinline__ void for_each_neighbor(const GridDev& g, const float4* __restrict__ xs,
-                                                  const int4* __restrict__ nbr, int cnt, int n, int k, float4 xi,
-                                                  const nsph_sph_params& p, V&& visit)
+                                                  const int4* __restrict__ nbr, int cnt, int n, int k, int sub,
+                                                  float4 xi, const nsph_sph_params& p, V&& visit)
 {
     if (cnt <= kNbrSlots) {
-        for_each_listed<true>(nbr, n, k, cnt, [&](int j) {
-            if (j != k) visit(j);
-        });
+        if constexpr (kLanes == 1) {
+            for_each_listed<true>(nbr, n, k, cnt, [&](int j) {
+                if (j != k) visit(j);
+            });
+        } else {
+            const int* item = reinterpret_cast<const int*>(nbr + k) + sub;
+            const size_t stride = 4 * (size_t)n;
+            int next = sub < cnt ? __ldg(item) : k;
+            for (int t = sub; t < cnt; t += 4) {
+                const int j = in_bounds(next >= 0 && next < n) ? next : k;
+                item += stride;
+                if (t + 4 < cnt) next = __ldg(item);
+                if (j != k) visit(j);
+            }
+        }
     } else {
         for_each_run(g, xi.x, xi.y, xi.z, p.h, [&](int lo, int hi) {
-            for (int j = lo; j < hi; ++j) {
+            for (int j = lo + sub; j < hi; j += kLanes) {
                 float dx, dy, dz;
-                if (j != k && dist2(xi, __ldg(xs + j), dx, dy, dz) < p.h2) visit(j);
+                const float4 xj = __ldg(xs + j);
+                if (j != k && dist2(xi, xj, dx, dy, dz) < p.h2 && !mirror_inactive(xj)) visit(j);
             }
         });
     }
+}
+
+// the sum over a particle's lanes, in each of them (all of a warp's lanes call it)
+template <int kLanes>
+__device__ __forceinline__ float lanes_sum(float v)
+{
+#pragma unroll
+    for (int o = 1; o < kLanes; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
 }
 
 struct AdjIO {
@@ -732,8 +1394,7 @@ struct AdjIO {
     const float* f_ext;
     const float* inv_mass;
     const float* gravity;
-    float4* g;     // sorted: adj(a)
-    float4* d;     // sorted: adj(dv)
+    float4* gd;    // sorted: adj(a), adj(dv) of particle k at 2k, 2k + 1
     float* rho;    // sorted: adj(rho)
     float* bpart;  // per block: partial adj(B)
     const float4* acc;  // or null: the forward's sorted (a, 0), (dv, 0) (the segment tape), else recomputed
@@ -744,11 +1405,12 @@ struct AdjIO {
 // sums a, dv are the forward's, stored (io.acc) or recomputed here.
 __global__ void __launch_bounds__(kSphThreads, 2) k_adj_local(GridDev g, const float4* __restrict__ xs,
                                                               const float4* __restrict__ vs,
-                                                              const float2* __restrict__ aux, int n,
+                                                              const ForceRec fr, int n,
                                                               const __grid_constant__ nsph_sph_params p,
                                                               const int4* __restrict__ nbr,
                                                               const int* __restrict__ ncnt, const AdjIO io)
 {
+    launch_entry();
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const float4 xi = xs[k], vi = vs[k];
         const int attr = __float_as_int(vi.w);
@@ -768,7 +1430,7 @@ __global__ void __launch_bounds__(kSphThreads, 2) k_adj_local(GridDev g, const f
                 const float4 a = io.acc[2 * (size_t)k], d = io.acc[2 * (size_t)k + 1];
                 acc = ForceAcc{a.x, a.y, a.z, d.x, d.y, d.z};
             } else {
-                force_from_list<false>(g, xs, vs, aux, nbr, ncnt[k], n, k, xi, vi, aux[k].y, p, acc);
+                force_from_list<false>(g, fr, nbr, ncnt[k], n, k, xi, vi, p.h, p.h2, p, acc);
             }
             const bool dynamic = (attr & kAttrDynamic) != 0;
             float w = 0.f;
@@ -826,8 +1488,8 @@ __global__ void __launch_bounds__(kSphThreads, 2) k_adj_local(GridDev g, const f
         }
         if (io.f_ext_adj)
             for (int c = 0; c < 3; ++c) io.f_ext_adj[3 * i + c] += fb[c];
-        io.g[k] = gk;
-        io.d[k] = dk;
+        io.gd[2 * (size_t)k] = gk;
+        io.gd[2 * (size_t)k + 1] = dk;
     }
 }
 
@@ -849,34 +1511,36 @@ __device__ __forceinline__ float block_sum(float v)
 }
 
 // gather of the transposed pressure and XSPH terms, then adj(rho) through
-// the EOS; per-block partial sums of adj(B)
+// the EOS; per-block partial sums of adj(B). kLanes = 4 gives each particle
+// four lanes, for scenes that do not fill the SMs with one thread each.
+template <int kLanes>
 __global__ void __launch_bounds__(kSphThreads, 2) k_adj_pair(GridDev g, const float4* __restrict__ xs,
                                                              const float4* __restrict__ vs,
-                                                             const float2* __restrict__ aux,
+                                                             const float2* __restrict__ aux, const ForceRec fr,
                                                              const float2* __restrict__ rp, int n,
                                                              const __grid_constant__ nsph_sph_params p,
                                                              const int4* __restrict__ nbr,
                                                              const int* __restrict__ ncnt, const AdjIO io)
 {
+    launch_entry();
     float bsum = 0.f;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+    const int sub = threadIdx.x & (kLanes - 1);
+    const int step = gridDim.x * blockDim.x / kLanes;
+    // whole warps: the lanes of a particle sum together
+    for (int k0 = (blockIdx.x * blockDim.x + (threadIdx.x & ~31)) / kLanes; k0 < n; k0 += step) {
+        const int kt = k0 + (threadIdx.x & 31) / kLanes, k = min(kt, n - 1);
         const float4 xi = xs[k], vi = vs[k];
         const size_t i = (size_t)g.ids[k];
-        if (!(__float_as_int(vi.w) & kAttrActive)) {
-            io.rho[k] = 0.f;
-            continue;
-        }
+        const bool active = kt < n && (__float_as_int(vi.w) & kAttrActive);
         const float2 ak = aux[k];
-        const float4 gk = io.g[k], dk = io.d[k];
+        const float4 gk = io.gd[2 * (size_t)k], dk = io.gd[2 * (size_t)k + 1];
         const float mk = xi.w;
         float pr2b = 0.f, morb = 0.f;
         float xb[3] = {0.f, 0.f, 0.f}, vb[3] = {0.f, 0.f, 0.f};
-        for_each_neighbor(g, xs, nbr, ncnt[k], n, k, xi, p, [&](int j) {
-            const float4 vj = __ldg(vs + j);
-            if (!(__float_as_int(vj.w) & kAttrActive)) return;
-            const float4 xj = __ldg(xs + j);
-            const float2 aj = __ldg(aux + j);
-            const float4 gj = __ldg(io.g + j), dj = __ldg(io.d + j);
+        for_each_neighbor<kLanes>(g, xs, nbr, active ? ncnt[k] : 0, n, k, sub, xi, p, [&](int j) {
+            const Neighbour o = load_neighbour(fr.rec, j), od = load_neighbour(io.gd, j);
+            const float4 xj = o.x, vj = o.v, gj = od.x, dj = od.v;
+            const float2 aj = make_float2(vj.w, __ldg(fr.pr2 + j));
             float dx, dy, dz;
             const float r2 = dist2(xi, xj, dx, dy, dz);
             const float r = __fsqrt_rn(r2);
@@ -902,6 +1566,19 @@ __global__ void __launch_bounds__(kSphThreads, 2) k_adj_pair(GridDev g, const fl
             vb[2] -= w * yz;
             morb -= w * (dj.x * rvx + dj.y * rvy + dj.z * rvz);
         });
+        if constexpr (kLanes > 1) {
+            pr2b = lanes_sum<kLanes>(pr2b);
+            morb = lanes_sum<kLanes>(morb);
+            for (int c = 0; c < 3; ++c) {
+                xb[c] = lanes_sum<kLanes>(xb[c]);
+                vb[c] = lanes_sum<kLanes>(vb[c]);
+            }
+        }
+        if (sub != 0 || kt >= n) continue;
+        if (!active) {
+            io.rho[k] = 0.f;
+            continue;
+        }
         // adj(rho) from p/rho^2 (through the EOS) and m/rho
         const float2 rpk = rp[k];
         float rb = io.rho_out_adj ? io.rho_out_adj[i] : 0.f;
@@ -928,6 +1605,7 @@ __global__ void __launch_bounds__(kSphThreads, 2) k_adj_pair(GridDev g, const fl
 }
 
 // gather of the transposed density sum
+template <int kLanes>
 __global__ void __launch_bounds__(kSphThreads, 3) k_adj_density(GridDev g, const float4* __restrict__ xs,
                                                                 const float4* __restrict__ vs, int n,
                                                                 const __grid_constant__ nsph_sph_params p,
@@ -936,12 +1614,16 @@ __global__ void __launch_bounds__(kSphThreads, 3) k_adj_density(GridDev g, const
                                                                 const float* __restrict__ rho_adj,
                                                                 float* __restrict__ x_in_adj)
 {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        if (!(__float_as_int(vs[k].w) & kAttrActive)) continue;
+    launch_entry();
+    const int sub = threadIdx.x & (kLanes - 1);
+    const int step = gridDim.x * blockDim.x / kLanes;
+    for (int k0 = (blockIdx.x * blockDim.x + (threadIdx.x & ~31)) / kLanes; k0 < n; k0 += step) {
+        const int kt = k0 + (threadIdx.x & 31) / kLanes, k = min(kt, n - 1);
+        const bool active = kt < n && (__float_as_int(vs[k].w) & kAttrActive);
         const float4 xi = xs[k];
         const float rbk = rho_adj[k], mk = xi.w;
         float xb[3] = {0.f, 0.f, 0.f};
-        for_each_neighbor(g, xs, nbr, ncnt[k], n, k, xi, p, [&](int j) {
+        for_each_neighbor<kLanes>(g, xs, nbr, active ? ncnt[k] : 0, n, k, sub, xi, p, [&](int j) {
             const float4 xj = __ldg(xs + j);
             float dx, dy, dz;
             const float r2 = dist2(xi, xj, dx, dy, dz);
@@ -952,6 +1634,8 @@ __global__ void __launch_bounds__(kSphThreads, 3) k_adj_density(GridDev g, const
             xb[1] += c * dy;
             xb[2] += c * dz;
         });
+        for (int c = 0; c < 3; ++c) xb[c] = lanes_sum<kLanes>(xb[c]);
+        if (sub != 0 || !active) continue;
         const size_t i = (size_t)g.ids[k];
         for (int c = 0; c < 3; ++c) x_in_adj[3 * i + c] += xb[c];
     }
@@ -960,6 +1644,7 @@ __global__ void __launch_bounds__(kSphThreads, 3) k_adj_density(GridDev g, const
 // adj(B) += sum of the per-block partials, in a fixed order
 __global__ void k_adj_b_reduce(const float* __restrict__ bpart, int blocks, float* __restrict__ b_adj)
 {
+    launch_entry();
     float v = 0.f;
     for (int b = threadIdx.x; b < blocks; b += blockDim.x) v += bpart[b];
     v = block_sum(v);
@@ -989,10 +1674,9 @@ struct FeatAcc {
 
 // the pressure and XSPH terms of force_term_data (same statements, so the
 // same rounding) plus the feature sums
-__device__ __forceinline__ void force_feature_term(float4 xj, float4 vj, float2 aj, float4 xi, float4 vi, float pr2_i,
+__device__ __forceinline__ void force_feature_term(float4 xj, float4 vj, float pr2_j, float4 xi, float4 vi, float pr2_i,
                                                    const nsph_sph_params& p, ForceAcc& acc, FeatAcc& fa)
 {
-    if (!(__float_as_int(vj.w) & kAttrActive)) return;
     float dx, dy, dz;
     const float r2 = dist2(xi, xj, dx, dy, dz);
     const float r = __fsqrt_rn(r2);
@@ -1001,12 +1685,12 @@ __device__ __forceinline__ void force_feature_term(float4 xj, float4 vj, float2 
     float f = 0.f;
     if (r2 > 0.f) {
         f = kernel_f(q, __frcp_rn(r), p);
-        const float s = __fmul_rn(__fmul_rn(xj.w, __fadd_rn(pr2_i, aj.y)), f);
+        const float s = __fmul_rn(__fmul_rn(xj.w, __fadd_rn(pr2_i, pr2_j)), f);
         acc.ax = __fmaf_rn(-s, dx, acc.ax);
         acc.ay = __fmaf_rn(-s, dy, acc.ay);
         acc.az = __fmaf_rn(-s, dz, acc.az);
     }
-    const float c = __fmul_rn(aj.x, w);
+    const float c = __fmul_rn(vj.w, w);
     const float rvx = __fsub_rn(vj.x, vi.x), rvy = __fsub_rn(vj.y, vi.y), rvz = __fsub_rn(vj.z, vi.z);
     acc.dvx = __fmaf_rn(c, rvx, acc.dvx);
     acc.dvy = __fmaf_rn(c, rvy, acc.dvy);
@@ -1016,40 +1700,38 @@ __device__ __forceinline__ void force_feature_term(float4 xj, float4 vj, float2 
     fa.my -= c * dy;
     fa.mz -= c * dz;
     fa.m2 += c * r2;
-    fa.dvg += aj.x * f * (rvx * dx + rvy * dy + rvz * dz);
+    fa.dvg += vj.w * f * (rvx * dx + rvy * dy + rvz * dz);
 }
 
 // pressure and XSPH sums (the statements of force_term_data, so the same
 // rounding) and the feature sums of particle k over its neighbour list, in
 // order
-__device__ __forceinline__ void force_features_from_list(const GridDev& g, const float4* __restrict__ xs,
-                                                         const float4* __restrict__ vs,
-                                                         const float2* __restrict__ aux, const int4* __restrict__ nbr,
-                                                         int cnt, int n, int k, float4 xi, float4 vi, float pr2_i,
-                                                         const nsph_sph_params& p, ForceAcc& acc, FeatAcc& fa)
+__device__ __forceinline__ void force_features_from_list(const GridDev& g, const ForceRec& fr,
+                                                         const int4* __restrict__ nbr, int cnt, int n, int k, float4 xi,
+                                                         float4 vi, float pr2_i, const nsph_sph_params& p,
+                                                         ForceAcc& acc, FeatAcc& fa)
 {
     if (cnt <= kNbrSlots) {
         bool have = false;
-        float4 pxj = make_float4(0.f, 0.f, 0.f, 0.f), pvj = pxj;
-        float2 paj = make_float2(0.f, 0.f);
+        Neighbour po{make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+        float pp = 0.f;
         for_each_listed<true>(nbr, n, k, cnt, [&](int j) {
             if (j == k) return;
-            const float4 nxj = __ldg(xs + j);
-            const float4 nvj = __ldg(vs + j);
-            const float2 naj = __ldg(aux + j);
-            if (have) force_feature_term(pxj, pvj, paj, xi, vi, pr2_i, p, acc, fa);
-            pxj = nxj;
-            pvj = nvj;
-            paj = naj;
+            const Neighbour o = load_neighbour(fr.rec, j);
+            const float pj = __ldg(fr.pr2 + j);
+            if (have) force_feature_term(po.x, po.v, pp, xi, vi, pr2_i, p, acc, fa);
+            po = o;
+            pp = pj;
             have = true;
         });
-        if (have) force_feature_term(pxj, pvj, paj, xi, vi, pr2_i, p, acc, fa);
+        if (have) force_feature_term(po.x, po.v, pp, xi, vi, pr2_i, p, acc, fa);
     } else {
         for_each_run(g, xi.x, xi.y, xi.z, p.h, [&](int lo, int hi) {
             for (int j = lo; j < hi; ++j) {
+                const Neighbour o = load_neighbour(fr.rec, j);
                 float dx, dy, dz;
-                if (dist2(xi, __ldg(xs + j), dx, dy, dz) < p.h2 && j != k)
-                    force_feature_term(__ldg(xs + j), __ldg(vs + j), __ldg(aux + j), xi, vi, pr2_i, p, acc, fa);
+                if (dist2(xi, o.x, dx, dy, dz) < p.h2 && j != k && !mirror_inactive(o.x))
+                    force_feature_term(o.x, o.v, __ldg(fr.pr2 + j), xi, vi, pr2_i, p, acc, fa);
             }
         });
     }
@@ -1058,8 +1740,7 @@ __device__ __forceinline__ void force_features_from_list(const GridDev& g, const
 // The 16 features of sorted particle k (all zero for an inactive one) and
 // its force sums; adds the particle's compression max(0, rho/rho0 - 1) and
 // 1 to (csum, ccount) when it is active.
-__device__ __forceinline__ void particle_features(const GridDev& g, const float4* __restrict__ xs,
-                                                  const float4* __restrict__ vs, const float2* __restrict__ aux,
+__device__ __forceinline__ void particle_features(const GridDev& g, const ForceRec& fr, const float2* __restrict__ aux,
                                                   const float2* __restrict__ rp, const int4* __restrict__ nbr,
                                                   const int* __restrict__ ncnt, int n, int k, float4 xi, float4 vi,
                                                   const nsph_sph_params& p, float (&f)[kFeat], ForceAcc& acc,
@@ -1076,7 +1757,7 @@ __device__ __forceinline__ void particle_features(const GridDev& g, const float4
     const float ascale = p.h / c0sq;
     const float2 ak = aux[k];
     FeatAcc fa{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    force_features_from_list(g, xs, vs, aux, nbr, ncnt[k], n, k, xi, vi, ak.y, p, acc, fa);
+    force_features_from_list(g, fr, nbr, ncnt[k], n, k, xi, vi, ak.y, p, acc, fa);
     const float2 rpk = rp[k];
     const float ratio = rpk.x * p.inv_rho0;
     f[0] = ratio;
@@ -1104,7 +1785,7 @@ __device__ __forceinline__ void particle_features(const GridDev& g, const float4
 // active count)
 __global__ void __launch_bounds__(kSphThreads, 4) k_force_features_list(GridDev g, const float4* __restrict__ xs,
                                                                         const float4* __restrict__ vs,
-                                                                        const float2* __restrict__ aux,
+                                                                        const ForceRec fr, const float2* __restrict__ aux,
                                                                         const float2* __restrict__ rp, int n,
                                                                         const __grid_constant__ nsph_sph_params p,
                                                                         const int4* __restrict__ nbr,
@@ -1113,12 +1794,13 @@ __global__ void __launch_bounds__(kSphThreads, 4) k_force_features_list(GridDev 
                                                                         float4* __restrict__ sacc,
                                                                         float* __restrict__ cpart)
 {
+    launch_entry();
     float csum = 0.f, ccount = 0.f;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const float4 xi = xs[k], vi = vs[k];
         float f[kFeat];
         ForceAcc acc;
-        particle_features(g, xs, vs, aux, rp, nbr, ncnt, n, k, xi, vi, p, f, acc, csum, ccount);
+        particle_features(g, fr, aux, rp, nbr, ncnt, n, k, xi, vi, p, f, acc, csum, ccount);
         float4* fo = reinterpret_cast<float4*>(feat + (size_t)k * kFeat);
 #pragma unroll
         for (int j = 0; j < kFeat; j += 4) fo[j / 4] = make_float4(f[j], f[j + 1], f[j + 2], f[j + 3]);
@@ -1138,6 +1820,7 @@ __global__ void __launch_bounds__(kSphThreads, 4) k_force_features_list(GridDev 
 // stats[2] += 1; stats[3] += stats[0]
 __global__ void k_compression_reduce(const float* __restrict__ cpart, int blocks, float* __restrict__ stats)
 {
+    launch_entry();
     float s = 0.f, c = 0.f;
     for (int b = threadIdx.x; b < blocks; b += blockDim.x) {
         s += cpart[2 * b];
@@ -1170,13 +1853,14 @@ __global__ void __launch_bounds__(kMlpTile, 6) k_surrogate_fused(const float* __
                                                                  int wait_limit, GridDev g,
                                                                  const float4* __restrict__ xs,
                                                                  const float4* __restrict__ vs,
-                                                                 const float2* __restrict__ aux,
+                                                                 const ForceRec fr, const float2* __restrict__ aux,
                                                                  const float2* __restrict__ rp, int n,
                                                                  const __grid_constant__ nsph_sph_params p,
                                                                  const int4* __restrict__ nbr,
                                                                  const int* __restrict__ ncnt, const StepOut o,
                                                                  float* __restrict__ cpart)
 {
+    launch_entry();
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     MlpFwdSmem& s = *reinterpret_cast<MlpFwdSmem*>(smem_raw);
     const uint32_t tmem = mlp_cta_begin(model, s, kMlpFwdCols);
@@ -1191,7 +1875,7 @@ __global__ void __launch_bounds__(kMlpTile, 6) k_surrogate_fused(const float* __
         float f[kFeat];
         ForceAcc acc;
         if (k < n) {
-            particle_features(g, xs, vs, aux, rp, nbr, ncnt, n, k, xi, vi, p, f, acc, csum, ccount);
+            particle_features(g, fr, aux, rp, nbr, ncnt, n, k, xi, vi, p, f, acc, csum, ccount);
         } else {
             acc = ForceAcc{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -1236,10 +1920,11 @@ template <int kGroups>
 __global__ void __launch_bounds__(kGroups * kMlpTile, 6 / kGroups)
     k_surrogate_fused_groups(const float* __restrict__ model, float acc_scale, int wait_limit, GridDev g,
                              const float4* __restrict__ xs, const float4* __restrict__ vs,
-                             const float2* __restrict__ aux, const float2* __restrict__ rp, int n,
+                             const ForceRec fr, const float2* __restrict__ aux, const float2* __restrict__ rp, int n,
                              const __grid_constant__ nsph_sph_params p, const int4* __restrict__ nbr,
                              const int* __restrict__ ncnt, const StepOut o, float* __restrict__ cpart)
 {
+    launch_entry();
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     auto& s = *reinterpret_cast<MlpFwdGroupSmem<kGroups>*>(smem_raw);
     const int grp = threadIdx.x / kMlpTile, row = threadIdx.x % kMlpTile;
@@ -1259,7 +1944,7 @@ __global__ void __launch_bounds__(kGroups * kMlpTile, 6 / kGroups)
         float f[kFeat];
         ForceAcc acc;
         if (k < n) {
-            particle_features(g, xs, vs, aux, rp, nbr, ncnt, n, k, xi, vi, p, f, acc, csum, ccount);
+            particle_features(g, fr, aux, rp, nbr, ncnt, n, k, xi, vi, p, f, acc, csum, ccount);
         } else {
             acc = ForceAcc{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -1303,6 +1988,7 @@ __global__ void k_scatter_features(const int* __restrict__ ids, int n, const flo
                                    const float4* __restrict__ sacc, float* __restrict__ feat_out,
                                    float* __restrict__ acc_out)
 {
+    launch_entry();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const size_t i = (size_t)ids[k];
@@ -1322,12 +2008,43 @@ __global__ void k_scatter_features(const int* __restrict__ ids, int n, const flo
 __global__ void k_scatter_rho(const int* __restrict__ ids, int n, const float2* __restrict__ rp,
                               float* __restrict__ rho_out)
 {
+    launch_entry();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < n) rho_out[ids[k]] = rp[k].x;
 }
 
+// mismatches of sqrt_plain / rcp_plain over the mantissas of [1, 4) x 2^(2 e)
+__global__ void k_root_mismatches(int e, unsigned long long* __restrict__ count)
+{
+    unsigned bad = 0;
+    for (unsigned u = 0x3f800000u + blockIdx.x * blockDim.x + threadIdx.x; u < 0x40800000u; u += gridDim.x * blockDim.x) {
+        const float x = ldexpf(__uint_as_float(u), 2 * e);
+        float y;
+        const float r = sqrt_plain(x, y);
+        bad += !plain_range(x) || __float_as_uint(r) != __float_as_uint(__fsqrt_rn(x)) ||
+               __float_as_uint(rcp_plain(r, y)) != __float_as_uint(__frcp_rn(r));
+    }
+    if (bad) atomicAdd(count, (unsigned long long)bad);
+}
+
 }  // namespace
 }  // namespace nsph
+
+extern "C" int nsph_debug_root_mismatches(const int* exponents, int num_exponents, unsigned long long* count)
+{
+    using namespace nsph;
+    clear_error();
+    if (!count || num_exponents < 0 || (num_exponents > 0 && !exponents))
+        return fail(NSPH_ERR_INVALID_ARG, "null argument");
+    unsigned long long* d = nullptr;
+    NSPH_CUDA_TRY(cudaMalloc(&d, sizeof(*d)));
+    cudaError_t e = cudaMemset(d, 0, sizeof(*d));
+    for (int i = 0; i < num_exponents; ++i) k_root_mismatches<<<1024, 256>>>(exponents[i], d);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpy(count, d, sizeof(*d), cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return e == cudaSuccess ? NSPH_OK : cuda_fail(e, "nsph_debug_root_mismatches");
+}
 
 // ==========================================================================
 // C ABI: solver context
@@ -1341,6 +2058,7 @@ struct nsph_sph {
     float4* vs = nullptr;
     float2* aux = nullptr;
     float2* rp = nullptr;
+    ForceRec fr{nullptr, nullptr, nullptr};  // the force pass's records
     int4* nbr = nullptr;       // kNbrGroups x capacity neighbour lists (group-major), every step form
     int* ncnt = nullptr;       //   neighbours per particle
     int fast = 0;              // plain step: tolerance arithmetic (nsph_sph_set_arithmetic)
@@ -1354,8 +2072,7 @@ struct nsph_sph {
     int launch_threads = 0;              // neighbour passes: threads per block (0 = default)
     int launch_blocks_per_sm = -1;       // neighbour passes: persistent blocks per SM (-1 = default, 0 = one thread per particle)
     int sms = 0;
-    float4* adj_g = nullptr;             // adjoint scratch (nsph_sph_enable_adjoint), sorted order: adj(a)
-    float4* adj_d = nullptr;             //   adj(dv)
+    float4* adj_gd = nullptr;            // adjoint scratch (nsph_sph_enable_adjoint), sorted: adj(a), adj(dv) at 2k, 2k + 1
     float* adj_rho = nullptr;            //   adj(rho)
     float* adj_bpart = nullptr;          //   per-block partial sums of adj(B)
     int adj_bcap = 0;                    //   entries of adj_bpart
@@ -1379,6 +2096,7 @@ struct TapeStep {
     float4* vs;
     float2* aux;
     float2* rp;
+    ForceRec fr;
     int4* nbr;
     int* ncnt;
     int* ids;
@@ -1391,6 +2109,7 @@ static size_t tape_align(size_t b) { return (b + 255) & ~(size_t)255; }
 static size_t tape_slot_bytes(size_t c, long long ncells)
 {
     return 2 * tape_align(sizeof(float4) * c) + 2 * tape_align(sizeof(float2) * c) +
+           tape_align(sizeof(float4) * 2 * c) + tape_align(sizeof(float) * c) +
            tape_align(sizeof(int4) * kNbrGroups * c) + 2 * tape_align(sizeof(int) * c) +
            tape_align(sizeof(int2) * (size_t)ncells) + tape_align(sizeof(float4) * 2 * c);
 }
@@ -1408,6 +2127,11 @@ static TapeStep tape_slot(const nsph_sph* s, int t)
     b += tape_align(sizeof(float2) * c);
     ts.rp = reinterpret_cast<float2*>(b);
     b += tape_align(sizeof(float2) * c);
+    ts.fr.rec = reinterpret_cast<float4*>(b);
+    b += tape_align(sizeof(float4) * 2 * c);
+    ts.fr.pr2 = reinterpret_cast<float*>(b);
+    ts.fr.overflow = nullptr;
+    b += tape_align(sizeof(float) * c);
     ts.nbr = reinterpret_cast<int4*>(b);
     b += tape_align(sizeof(int4) * kNbrGroups * c);
     ts.ncnt = reinterpret_cast<int*>(b);
@@ -1420,7 +2144,15 @@ static TapeStep tape_slot(const nsph_sph* s, int t)
     return ts;
 }
 
-// the two recompute states (x then v, 3 x capacity floats each) after the slots
+// after the slots: the two recompute states (x then v, 3 x capacity floats
+// each), then a word per step that tells whether a list overflowed
+static unsigned* tape_overflow(const nsph_sph* s)
+{
+    const size_t c = (size_t)s->capacity;
+    return reinterpret_cast<unsigned*>(s->tape + (size_t)s->tape_steps * s->tape_step_bytes +
+                                       tape_align(sizeof(float) * 12 * c));
+}
+
 static float* tape_state(const nsph_sph* s, int which)
 {
     return reinterpret_cast<float*>(s->tape + (size_t)s->tape_steps * s->tape_step_bytes) +
@@ -1443,6 +2175,28 @@ static void pass_launch(const nsph_sph* s, int n, bool persistent_default, int& 
         blocks = std::min(full, std::max(1, s->sms * bps));
     blocks = std::max(blocks, 1);
 }
+
+// whether the force and adjoint passes take four lanes per particle: scenes of
+// fewer than kQuadMax particles, unless the caller set a launch shape
+static bool quad_pass(const nsph_sph* s, int n)
+{
+    static const int lim = getenv("NSPH_QUAD") ? atoi(getenv("NSPH_QUAD")) : kQuadMax;
+    return n <= lim && s->launch_threads == 0 && s->launch_blocks_per_sm < 0;
+}
+
+// grid of a density pass: as pass_launch, but small scenes in blocks of two
+// warps, so that their warps spread over the SMs
+static void density_launch(const nsph_sph* s, int n, bool persistent_default, int& blocks, int& threads)
+{
+    pass_launch(s, n, persistent_default, blocks, threads);
+    if (s->launch_threads == 0 && s->launch_blocks_per_sm < 0 && n < kSmallDensity) {
+        threads = 64;
+        blocks = std::max(1, (n + threads - 1) / threads);
+    }
+}
+
+// shared memory of a density pass: one TileSmem per warp
+static size_t tile_smem_bytes(int threads) { return sizeof(TileSmem) * (size_t)(threads / 32); }
 
 // Record a timing event: as an external event node while the stream is being
 // captured (so a replayed graph records it), as a plain record otherwise.
@@ -1472,12 +2226,13 @@ static void sph_free(nsph_sph* s)
     cudaFree(s->vs);
     cudaFree(s->aux);
     cudaFree(s->rp);
+    cudaFree(s->fr.rec);
+    cudaFree(s->fr.pr2);
     cudaFree(s->nbr);
     cudaFree(s->ncnt);
     cudaFree(s->wparams);
     cudaFree(s->status);
-    cudaFree(s->adj_g);
-    cudaFree(s->adj_d);
+    cudaFree(s->adj_gd);
     cudaFree(s->adj_rho);
     cudaFree(s->adj_bpart);
     cudaFree(s->sfeat);
@@ -1505,6 +2260,7 @@ extern "C" int nsph_sph_create(int device, int capacity, const int grid_dims[3],
         cudaFuncAttributes fa;
         if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_density_list<false>);
         if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_force_list<false>);
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_force_quad);
         if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_density_list<true>);
         if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_force_list<true>);
         if (e != cudaSuccess) {
@@ -1572,6 +2328,8 @@ static int sph_create_common(nsph_sph* s, int device, int capacity)
         if (e == cudaSuccess) e = cudaMalloc(&s->vs, sizeof(float4) * c);
         if (e == cudaSuccess) e = cudaMalloc(&s->aux, sizeof(float2) * c);
         if (e == cudaSuccess) e = cudaMalloc(&s->rp, sizeof(float2) * c);
+        if (e == cudaSuccess) e = cudaMalloc(&s->fr.rec, sizeof(float4) * 2 * c);
+        if (e == cudaSuccess) e = cudaMalloc(&s->fr.pr2, sizeof(float) * c);
         if (e == cudaSuccess) e = cudaMalloc(&s->nbr, sizeof(int4) * kNbrGroups * c);
         if (e == cudaSuccess) e = cudaMalloc(&s->ncnt, sizeof(int) * c);
         if (e == cudaSuccess) e = cudaMalloc(&s->status, sizeof(unsigned));
@@ -1627,7 +2385,8 @@ static int check_step_inputs(const nsph_sph* s, int n, const float* x_in, const 
 static int step_enqueue(nsph_sph* s, const nsph_sph_params* p, int n, const float* x_in, const float* v_in,
                         const float* f_ext, const float* mass, const float* inv_mass, const int* flags,
                         const int* world, const float* gravity, int world_count, float* x_out, float* v_out,
-                        float* rho_out, float* p_out, float* a_out, cudaStream_t cs, int& launches)
+                        float* rho_out, float* p_out, float* a_out, cudaStream_t cs, int& launches,
+                        bool carry_v = false)
 {
     GatherArgs ga{x_in, v_in, mass, inv_mass, flags, world, world_count, s->xs, s->vs};
     if (s->ev[0]) NSPH_CUDA_TRY(record_mark(s->ev[0], cs));
@@ -1638,22 +2397,27 @@ static int step_enqueue(nsph_sph* s, const nsph_sph_params* p, int n, const floa
     if (n > 0) {
         const GridDev g = s->grid.view();
         int blocks, threads;
-        pass_launch(s, n, false, blocks, threads);
+        density_launch(s, n, false, blocks, threads);
         if (s->fast)
-            k_density_list<true><<<blocks, threads, 0, cs>>>(g, s->xs, s->vs, n, *p, s->aux, s->rp, s->nbr, s->ncnt,
-                                                             s->status);
+            NSPH_CUDA_TRY(launch_dependent(k_density_list<true>, blocks, threads, tile_smem_bytes(threads), cs,
+                                           g, s->xs, s->vs, n, *p, s->aux, s->rp, s->nbr, s->ncnt, s->fr, s->status));
         else
-            k_density_list<false><<<blocks, threads, 0, cs>>>(g, s->xs, s->vs, n, *p, s->aux, s->rp, s->nbr,
-                                                              s->ncnt, s->status);
+            NSPH_CUDA_TRY(launch_dependent(k_density_list<false>, blocks, threads, tile_smem_bytes(threads), cs,
+                                           g, s->xs, s->vs, n, *p, s->aux, s->rp, s->nbr, s->ncnt, s->fr, s->status));
         NSPH_LAUNCH_CHECK("k_density_list");
         ++launches;
         if (s->ev[2]) NSPH_CUDA_TRY(record_mark(s->ev[2], cs));
-        const StepOut o{f_ext, inv_mass, gravity, x_out, v_out, rho_out, p_out, a_out, s->status};
+        pass_launch(s, n, false, blocks, threads);
+        const StepOut o{f_ext, inv_mass, gravity, x_out, v_out, rho_out, p_out, a_out, s->status, nullptr, carry_v};
         if (s->fast)
-            k_force_list<true><<<blocks, threads, 0, cs>>>(g, s->xs, s->vs, s->aux, s->rp, n, *p, s->nbr, s->ncnt, o);
+            NSPH_CUDA_TRY(launch_plain(k_force_list<true>, blocks, threads, 0, cs,
+                                           g, s->xs, s->vs, s->fr, s->rp, n, *p, s->nbr, s->ncnt, o));
+        else if (quad_pass(s, n))
+            NSPH_CUDA_TRY(launch_dependent(k_force_quad, (4 * n + kQuadThreads - 1) / kQuadThreads, kQuadThreads, 0, cs,
+                                           g, s->xs, s->vs, s->fr, s->rp, n, *p, s->nbr, s->ncnt, o));
         else
-            k_force_list<false><<<blocks, threads, 0, cs>>>(g, s->xs, s->vs, s->aux, s->rp, n, *p, s->nbr, s->ncnt,
-                                                            o);
+            NSPH_CUDA_TRY(launch_plain(k_force_list<false>, blocks, threads, 0, cs,
+                                           g, s->xs, s->vs, s->fr, s->rp, n, *p, s->nbr, s->ncnt, o));
         NSPH_LAUNCH_CHECK("k_force_list");
         ++launches;
     } else if (s->ev[2]) {
@@ -1721,10 +2485,9 @@ extern "C" int nsph_sph_rollout(nsph_sph* s, const nsph_sph_params* p, int n, in
         const float* vi = t == 0 ? v0 : v_traj + (size_t)(t - 1) * len;
         float* xo = x_traj + (size_t)t * len;
         float* vo = v_traj + (size_t)t * len;
-        // inactive particles keep their velocity (the step leaves it untouched)
-        NSPH_CUDA_TRY(cudaMemcpyAsync(vo, vi, sizeof(float) * len, cudaMemcpyDeviceToDevice, cs));
+        // inactive particles keep their velocity
         st = step_enqueue(s, p, n, xi, vi, f_ext, mass, inv_mass, flags, world, gravity, world_count, xo, vo, nullptr,
-                          nullptr, nullptr, cs, launches);
+                          nullptr, nullptr, cs, launches, true);
         if (st != NSPH_OK) return st;
     }
     s->last_launches = launches;
@@ -1783,17 +2546,16 @@ extern "C" int nsph_sph_step_worlds(nsph_sph* s, float dt, int n, const float* x
     if (s->ev[1]) NSPH_CUDA_TRY(record_mark(s->ev[1], cs));
     if (n > 0) {
         int blocks, threads;
-        pass_launch(s, n, true, blocks, threads);
-        k_density_worlds<<<blocks, threads, 0, cs>>>(s->grid.worlds, s->wparams, s->grid.cell_ranges,
-                                                         s->grid.point_ids, s->xs, s->vs, n, s->aux, s->rp, s->nbr,
-                                                         s->ncnt, s->status);
+        density_launch(s, n, true, blocks, threads);
+        NSPH_CUDA_TRY(launch_dependent(k_density_worlds, blocks, threads, tile_smem_bytes(threads), cs,
+                                       s->grid.worlds, s->wparams, s->grid.cell_ranges, s->grid.point_ids, s->xs, s->vs, n, s->aux, s->rp, s->nbr, s->ncnt, s->fr, s->status));
         NSPH_LAUNCH_CHECK("k_density_worlds");
         ++launches;
         if (s->ev[2]) NSPH_CUDA_TRY(record_mark(s->ev[2], cs));
+        pass_launch(s, n, true, blocks, threads);
         const StepOut o{f_ext, inv_mass, gravity, x_out, v_out, rho_out, p_out, a_out, s->status};
-        k_force_worlds<<<blocks, threads, 0, cs>>>(s->grid.worlds, s->wparams, s->grid.cell_ranges,
-                                                       s->grid.point_ids, s->xs, s->vs, s->aux, s->rp, n, dt, s->nbr,
-                                                       s->ncnt, o);
+        NSPH_CUDA_TRY(launch_plain(k_force_worlds, blocks, threads, 0, cs,
+                                       s->grid.worlds, s->wparams, s->grid.cell_ranges, s->grid.point_ids, s->xs, s->vs, s->fr, s->rp, n, dt, s->nbr, s->ncnt, o));
         NSPH_LAUNCH_CHECK("k_force_worlds");
         ++launches;
     } else if (s->ev[2]) {
@@ -1817,9 +2579,8 @@ extern "C" int nsph_sph_neighbors(const nsph_sph* s, const nsph_sph_params* p, i
         if (n == 0) return NSPH_OK;
         DeviceGuard guard(s->grid.device);
         if (!guard.ok) return fail(NSPH_ERR_CUDA, "cannot select CUDA device");
-        k_neighbors_worlds<<<(n + 127) / 128, 128, 0, (cudaStream_t)stream>>>(
-            s->grid.worlds, s->wparams, s->grid.cell_ranges, s->grid.point_ids, s->xs, s->vs, n, counts, offsets,
-            out_ids);
+        NSPH_CUDA_TRY(launch_dependent(k_neighbors_worlds, (n + 127) / 128, 128, 0, (cudaStream_t)stream,
+                                       s->grid.worlds, s->wparams, s->grid.cell_ranges, s->grid.point_ids, s->xs, s->vs, n, counts, offsets, out_ids));
         NSPH_LAUNCH_CHECK("k_neighbors_worlds");
         return NSPH_OK;
     }
@@ -1831,8 +2592,8 @@ extern "C" int nsph_sph_neighbors(const nsph_sph* s, const nsph_sph_params* p, i
     if (n == 0) return NSPH_OK;
     DeviceGuard guard(s->grid.device);
     if (!guard.ok) return fail(NSPH_ERR_CUDA, "cannot select CUDA device");
-    k_neighbors<<<(n + 127) / 128, 128, 0, (cudaStream_t)stream>>>(s->grid.view(), s->xs, s->vs, n, *p, counts,
-                                                                   offsets, out_ids);
+    NSPH_CUDA_TRY(launch_dependent(k_neighbors, (n + 127) / 128, 128, 0, (cudaStream_t)stream,
+                                   s->grid.view(), s->xs, s->vs, n, *p, counts, offsets, out_ids));
     NSPH_LAUNCH_CHECK("k_neighbors");
     return NSPH_OK;
 }
@@ -1932,26 +2693,26 @@ extern "C" int nsph_sph_enable_adjoint(nsph_sph* s)
     clear_error();
     if (!s) return fail(NSPH_ERR_INVALID_ARG, "null solver");
     if (s->grid.world_count > 0) return fail(NSPH_ERR_INVALID_ARG, "the adjoint supports single-world solvers only");
-    if (s->adj_g) return NSPH_OK;
+    if (s->adj_gd) return NSPH_OK;
     DeviceGuard guard(s->grid.device);
     if (!guard.ok) return fail(NSPH_ERR_CUDA, "cannot select CUDA device");
     const size_t c = (size_t)(s->capacity > 0 ? s->capacity : 1);
-    const int bcap = (int)((c + 31) / 32) + 1;  // blocks of a pass of >= 32 threads per block
-    cudaError_t e = cudaMalloc(&s->adj_g, sizeof(float4) * c);
-    if (e == cudaSuccess) e = cudaMalloc(&s->adj_d, sizeof(float4) * c);
+    const int bcap = (int)((c + 31) / 32) + 1;  // blocks of a pass of >= 32 threads per block, or of 64 particles
+    cudaError_t e = cudaMalloc(&s->adj_gd, sizeof(float4) * 2 * c);
     if (e == cudaSuccess) e = cudaMalloc(&s->adj_rho, sizeof(float) * c);
     if (e == cudaSuccess) e = cudaMalloc(&s->adj_bpart, sizeof(float) * (size_t)bcap);
     cudaFuncAttributes fa;
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_adj_local);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_adj_pair);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_adj_density);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_adj_pair<1>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_adj_density<1>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_adj_pair<4>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_adj_density<4>);
     if (e != cudaSuccess) {
         cudaGetLastError();
-        cudaFree(s->adj_g);
-        cudaFree(s->adj_d);
+        cudaFree(s->adj_gd);
         cudaFree(s->adj_rho);
         cudaFree(s->adj_bpart);
-        s->adj_g = s->adj_d = nullptr;
+        s->adj_gd = nullptr;
         s->adj_rho = s->adj_bpart = nullptr;
         return fail(NSPH_ERR_OUT_OF_MEMORY, std::string("adjoint allocation: ") + cudaGetErrorString(e));
     }
@@ -1966,17 +2727,32 @@ static int adjoint_kernels(nsph_sph* s, const nsph_sph_params* p, int n, const G
 {
     int blocks, threads;
     pass_launch(s, n, false, blocks, threads);
-    k_adj_local<<<blocks, threads, 0, cs>>>(g, ts.xs, ts.vs, ts.aux, n, *p, ts.nbr, ts.ncnt, io);
+    NSPH_CUDA_TRY(launch_dependent(k_adj_local, blocks, threads, 0, cs,
+                                   g, ts.xs, ts.vs, ts.fr, n, *p, ts.nbr, ts.ncnt, io));
     NSPH_LAUNCH_CHECK("k_adj_local");
     if (mark && s->eva[3]) NSPH_CUDA_TRY(record_mark(s->eva[3], cs));
-    k_adj_pair<<<blocks, threads, 0, cs>>>(g, ts.xs, ts.vs, ts.aux, ts.rp, n, *p, ts.nbr, ts.ncnt, io);
+    const bool quad = quad_pass(s, n);
+    const int pair_blocks = quad ? (4 * n + kSphThreads - 1) / kSphThreads : blocks;
+    const int pair_threads = quad ? kSphThreads : threads;
+    if (quad)
+        NSPH_CUDA_TRY(launch_dependent(k_adj_pair<4>, pair_blocks, pair_threads, 0, cs,
+                                       g, ts.xs, ts.vs, ts.aux, ts.fr, ts.rp, n, *p, ts.nbr, ts.ncnt, io));
+    else
+        NSPH_CUDA_TRY(launch_dependent(k_adj_pair<1>, pair_blocks, pair_threads, 0, cs,
+                                       g, ts.xs, ts.vs, ts.aux, ts.fr, ts.rp, n, *p, ts.nbr, ts.ncnt, io));
     NSPH_LAUNCH_CHECK("k_adj_pair");
     if (mark && s->eva[4]) NSPH_CUDA_TRY(record_mark(s->eva[4], cs));
-    k_adj_density<<<blocks, threads, 0, cs>>>(g, ts.xs, ts.vs, n, *p, ts.nbr, ts.ncnt, io.rho, io.x_in_adj);
+    if (quad)
+        NSPH_CUDA_TRY(launch_dependent(k_adj_density<4>, pair_blocks, pair_threads, 0, cs,
+                                       g, ts.xs, ts.vs, n, *p, ts.nbr, ts.ncnt, io.rho, io.x_in_adj));
+    else
+        NSPH_CUDA_TRY(launch_dependent(k_adj_density<1>, pair_blocks, pair_threads, 0, cs,
+                                       g, ts.xs, ts.vs, n, *p, ts.nbr, ts.ncnt, io.rho, io.x_in_adj));
     NSPH_LAUNCH_CHECK("k_adj_density");
     launches += 3;
     if (eos_b_adj) {
-        k_adj_b_reduce<<<1, 256, 0, cs>>>(io.bpart, blocks, eos_b_adj);
+        NSPH_CUDA_TRY(launch_dependent(k_adj_b_reduce, 1, 256, 0, cs,
+                                       io.bpart, pair_blocks, eos_b_adj));
         NSPH_LAUNCH_CHECK("k_adj_b_reduce");
         ++launches;
     }
@@ -1999,15 +2775,15 @@ static int adjoint_enqueue(nsph_sph* s, const nsph_sph_params* p, int n, const f
     if (n > 0) {
         const GridDev g = s->grid.view();
         int blocks, threads;
-        pass_launch(s, n, false, blocks, threads);
-        k_density_list<false><<<blocks, threads, 0, cs>>>(g, s->xs, s->vs, n, *p, s->aux, s->rp, s->nbr, s->ncnt,
-                                                          s->status);
+        density_launch(s, n, false, blocks, threads);
+        NSPH_CUDA_TRY(launch_dependent(k_density_list<false>, blocks, threads, tile_smem_bytes(threads), cs,
+                                       g, s->xs, s->vs, n, *p, s->aux, s->rp, s->nbr, s->ncnt, s->fr, s->status));
         NSPH_LAUNCH_CHECK("k_density_list");
         if (s->eva[2]) NSPH_CUDA_TRY(record_mark(s->eva[2], cs));
         ++launches;
         const AdjIO io{x_out_adj, v_out_adj, rho_out_adj, x_in_adj, v_in_adj, f_ext_adj, f_ext, inv_mass, gravity,
-                       s->adj_g, s->adj_d, s->adj_rho, s->adj_bpart};
-        const TapeStep ts{s->xs, s->vs, s->aux, s->rp, s->nbr, s->ncnt, nullptr, nullptr, nullptr};
+                       s->adj_gd, s->adj_rho, s->adj_bpart};
+        const TapeStep ts{s->xs, s->vs, s->aux, s->rp, s->fr, s->nbr, s->ncnt, nullptr, nullptr, nullptr};
         st = adjoint_kernels(s, p, n, g, ts, io, eos_b_adj, cs, launches, true);
         if (st != NSPH_OK) return st;
     } else {
@@ -2021,7 +2797,7 @@ static int adjoint_enqueue(nsph_sph* s, const nsph_sph_params* p, int n, const f
 static int check_adjoint_ready(const nsph_sph* s)
 {
     if (s->grid.world_count > 0) return fail(NSPH_ERR_INVALID_ARG, "the adjoint supports single-world solvers only");
-    if (!s->adj_g) return fail(NSPH_ERR_INVALID_ARG, "adjoint scratch not allocated (nsph_sph_enable_adjoint)");
+    if (!s->adj_gd) return fail(NSPH_ERR_INVALID_ARG, "adjoint scratch not allocated (nsph_sph_enable_adjoint)");
     return NSPH_OK;
 }
 
@@ -2101,7 +2877,7 @@ extern "C" int nsph_sph_reserve_segment(nsph_sph* s, int steps)
     if (!guard.ok) return fail(NSPH_ERR_CUDA, "cannot select CUDA device");
     const size_t c = (size_t)(s->capacity > 0 ? s->capacity : 1);
     const size_t slot = tape_slot_bytes(c, s->grid.ncells);
-    const size_t bytes = slot * (size_t)steps + tape_align(sizeof(float) * 12 * c);
+    const size_t bytes = slot * (size_t)steps + tape_align(sizeof(float) * 12 * c) + sizeof(unsigned) * (size_t)steps;
     char* t = nullptr;
     const cudaError_t e = cudaMalloc(&t, bytes);
     if (e != cudaSuccess) {
@@ -2147,34 +2923,40 @@ extern "C" int nsph_sph_segment_adjoint(nsph_sph* s, const nsph_sph_params* p, i
     if (!guard.ok) return fail(NSPH_ERR_CUDA, "cannot select CUDA device");
     cudaStream_t cs = (cudaStream_t)stream;
     int launches = 0;
-    int blocks, threads;
+    int blocks, threads, dblocks, dthreads;
     pass_launch(s, n, false, blocks, threads);
+    density_launch(s, n, false, dblocks, dthreads);
     // forward: the build, density and force passes of every step, their
     // outputs into the step's slot (the last step's new state is not used)
+    NSPH_CUDA_TRY(cudaMemsetAsync(tape_overflow(s), 0, sizeof(unsigned) * (size_t)steps, cs));
     for (int t = 0; t < steps; ++t) {
         const float* xi = t == 0 ? x0 : tape_state(s, t & 1);
         const float* vi = t == 0 ? v0 : tape_state(s, t & 1) + len;
-        const TapeStep ts = tape_slot(s, t);
+        TapeStep ts = tape_slot(s, t);
+        ts.fr.overflow = tape_overflow(s) + t;
         GatherArgs ga{xi, vi, mass, inv_mass, flags, world, world_count, ts.xs, ts.vs};
         st = grid_build(s->grid, xi, n, p->cell_width, p->cell_inv, &ga, s->status, cs, &launches);
         if (st != NSPH_OK) return st;
-        NSPH_CUDA_TRY(cudaMemcpyAsync(ts.ranges, s->grid.cell_ranges, sizeof(int2) * (size_t)s->grid.ncells,
-                                      cudaMemcpyDeviceToDevice, cs));
-        NSPH_CUDA_TRY(cudaMemcpyAsync(ts.ids, s->grid.point_ids, sizeof(int) * (size_t)n, cudaMemcpyDeviceToDevice,
-                                      cs));
-        GridDev g = s->grid.view();
-        g.ranges = ts.ranges;
-        g.ids = ts.ids;
-        k_density_list<false><<<blocks, threads, 0, cs>>>(g, ts.xs, ts.vs, n, *p, ts.aux, ts.rp, ts.nbr, ts.ncnt,
-                                                          s->status);
+        const GridDev g = s->grid.view();
+        NSPH_CUDA_TRY(launch_dependent(k_density_list<false>, dblocks, dthreads, tile_smem_bytes(dthreads), cs,
+                                       g, ts.xs, ts.vs, n, *p, ts.aux, ts.rp, ts.nbr, ts.ncnt, ts.fr, s->status));
         NSPH_LAUNCH_CHECK("k_density_list");
         ++launches;
         float* xo = tape_state(s, (t + 1) & 1);
         float* vo = xo + len;
-        // inactive particles keep their velocity (the step leaves it untouched)
-        if (t + 1 < steps) NSPH_CUDA_TRY(cudaMemcpyAsync(vo, vi, sizeof(float) * len, cudaMemcpyDeviceToDevice, cs));
-        const StepOut o{f_ext, inv_mass, gravity, xo, vo, nullptr, nullptr, nullptr, s->status, ts.acc};
-        k_force_list<false><<<blocks, threads, 0, cs>>>(g, ts.xs, ts.vs, ts.aux, ts.rp, n, *p, ts.nbr, ts.ncnt, o);
+        // the sorted ids and, where a list overflowed, the cell table into the slot
+        NSPH_CUDA_TRY(launch_dependent(k_tape_copy, s->sms * 2, 512, 0, cs, g, s->grid.ncells, n, ts.fr.overflow, ts.ids,
+                                       ts.ranges));
+        NSPH_LAUNCH_CHECK("k_tape_copy");
+        ++launches;
+        // inactive particles keep their velocity
+        const StepOut o{f_ext, inv_mass, gravity, xo, vo, nullptr, nullptr, nullptr, s->status, ts.acc, true};
+        if (quad_pass(s, n))
+            NSPH_CUDA_TRY(launch_dependent(k_force_quad, (4 * n + kQuadThreads - 1) / kQuadThreads, kQuadThreads, 0, cs,
+                                           g, ts.xs, ts.vs, ts.fr, ts.rp, n, *p, ts.nbr, ts.ncnt, o));
+        else
+            NSPH_CUDA_TRY(launch_plain(k_force_list<false>, blocks, threads, 0, cs,
+                                           g, ts.xs, ts.vs, ts.fr, ts.rp, n, *p, ts.nbr, ts.ncnt, o));
         NSPH_LAUNCH_CHECK("k_force_list");
         ++launches;
     }
@@ -2185,7 +2967,7 @@ extern "C" int nsph_sph_segment_adjoint(nsph_sph* s, const nsph_sph_params* p, i
     s->last_n = n;
     // reverse, from the slots
     AdjIO io{x_adj, v_adj, nullptr, x_adj, v_adj, f_ext_adj, f_ext, inv_mass, gravity,
-             s->adj_g, s->adj_d, s->adj_rho, s->adj_bpart, nullptr};
+             s->adj_gd, s->adj_rho, s->adj_bpart, nullptr};
     for (int t = steps - 1; t >= 0; --t) {
         const TapeStep ts = tape_slot(s, t);
         io.acc = ts.acc;
@@ -2335,15 +3117,16 @@ static int features_enqueue(nsph_sph* s, const nsph_sph_params* p, int n, const 
     if (n > 0) {
         const GridDev g = s->grid.view();
         int threads;
-        pass_launch(s, n, false, blocks, threads);
-        k_density_list<false><<<blocks, threads, 0, cs>>>(g, s->xs, s->vs, n, *p, s->aux, s->rp, s->nbr, s->ncnt,
-                                                          s->status);
+        density_launch(s, n, false, blocks, threads);
+        NSPH_CUDA_TRY(launch_dependent(k_density_list<false>, blocks, threads, tile_smem_bytes(threads), cs,
+                                       g, s->xs, s->vs, n, *p, s->aux, s->rp, s->nbr, s->ncnt, s->fr, s->status));
         NSPH_LAUNCH_CHECK("k_density_list");
         ++launches;
         if (mark && s->eva[2]) NSPH_CUDA_TRY(record_mark(s->eva[2], cs));
+        pass_launch(s, n, false, blocks, threads);
         if (features) {
-            k_force_features_list<<<blocks, threads, 0, cs>>>(g, s->xs, s->vs, s->aux, s->rp, n, *p, s->nbr,
-                                                              s->ncnt, s->sfeat, s->sacc, s->cpart);
+            NSPH_CUDA_TRY(launch_plain(k_force_features_list, blocks, threads, 0, cs,
+                                           g, s->xs, s->vs, s->fr, s->aux, s->rp, n, *p, s->nbr, s->ncnt, s->sfeat, s->sacc, s->cpart));
             NSPH_LAUNCH_CHECK("k_force_features_list");
             ++launches;
         }
@@ -2379,13 +3162,14 @@ extern "C" int nsph_sph_features(nsph_sph* s, const nsph_sph_params* p, int n, c
     st = features_enqueue(s, p, n, x_in, v_in, mass, inv_mass, flags, world, world_count, cs, launches, blocks);
     if (st != NSPH_OK) return st;
     if (n > 0 && (feat_out || acc_out)) {
-        k_scatter_features<<<(n + 255) / 256, 256, 0, cs>>>(s->grid.point_ids, n, s->sfeat, s->sacc, feat_out,
-                                                              acc_out);
+        NSPH_CUDA_TRY(launch_dependent(k_scatter_features, (n + 255) / 256, 256, 0, cs,
+                                       s->grid.point_ids, n, s->sfeat, s->sacc, feat_out, acc_out));
         NSPH_LAUNCH_CHECK("k_scatter_features");
         ++launches;
     }
     if (n > 0 && rho_out) {
-        k_scatter_rho<<<(n + 255) / 256, 256, 0, cs>>>(s->grid.point_ids, n, s->rp, rho_out);
+        NSPH_CUDA_TRY(launch_dependent(k_scatter_rho, (n + 255) / 256, 256, 0, cs,
+                                       s->grid.point_ids, n, s->rp, rho_out));
         NSPH_LAUNCH_CHECK("k_scatter_rho");
         ++launches;
     }
@@ -2424,19 +3208,18 @@ extern "C" int nsph_sph_step_surrogate(nsph_sph* s, const nsph_sph_params* p, co
         int grid;
         if (s->surr_groups == 2) {
             grid = std::min((tiles + 1) / 2, std::max(1, s->surr_ctas));
-            k_surrogate_fused_groups<2><<<grid, 2 * kMlpTile, sizeof(MlpFwdGroupSmem<2>), cs>>>(
-                model, acc_scale, wait_limit, s->grid.view(), s->xs, s->vs, s->aux, s->rp, n, *p, s->nbr, s->ncnt, o,
-                s->cpart);
+            NSPH_CUDA_TRY(launch_plain(k_surrogate_fused_groups<2>, grid, 2 * kMlpTile, sizeof(MlpFwdGroupSmem<2>), cs,
+                                           model, acc_scale, wait_limit, s->grid.view(), s->xs, s->vs, s->fr, s->aux, s->rp, n, *p, s->nbr, s->ncnt, o, s->cpart));
             NSPH_LAUNCH_CHECK("k_surrogate_fused_groups");
         } else {
             grid = std::min(tiles, std::max(1, s->surr_ctas));
-            k_surrogate_fused<<<grid, kMlpTile, sizeof(MlpFwdSmem), cs>>>(model, acc_scale, wait_limit,
-                                                                          s->grid.view(), s->xs, s->vs, s->aux, s->rp,
-                                                                          n, *p, s->nbr, s->ncnt, o, s->cpart);
+            NSPH_CUDA_TRY(launch_plain(k_surrogate_fused, grid, kMlpTile, sizeof(MlpFwdSmem), cs,
+                                           model, acc_scale, wait_limit, s->grid.view(), s->xs, s->vs, s->fr, s->aux, s->rp, n, *p, s->nbr, s->ncnt, o, s->cpart));
             NSPH_LAUNCH_CHECK("k_surrogate_fused");
         }
         if (s->eva[3]) NSPH_CUDA_TRY(record_mark(s->eva[3], cs));
-        k_compression_reduce<<<1, 256, 0, cs>>>(s->cpart, grid, stats);
+        NSPH_CUDA_TRY(launch_dependent(k_compression_reduce, 1, 256, 0, cs,
+                                       s->cpart, grid, stats));
         NSPH_LAUNCH_CHECK("k_compression_reduce");
         launches += 2;
     } else if (s->eva[3]) {
