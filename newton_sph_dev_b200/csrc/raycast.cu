@@ -33,6 +33,12 @@
 // of the query box are monotone in t, so a cell that an earlier sample tested
 // and that this box still holds was in the previous box.
 //
+// 3. A ray whose first window is empty has all its computed hits collected
+//    from the tree. Up to kRayList of them, only these spheres' cells matter:
+//    march_few passes over the samples far from all of them in strides. (Without
+//    it such rays marched through ever wider windows; the image of the block
+//    at 640 x 480 took 1.11 ms, now 0.99.)
+//
 // The march alone was bound by instruction issue: most rays miss, and each
 // missing ray took every sample up to max_distance through cells that the
 // grid's 128 cells per axis alias onto the scene.
@@ -339,24 +345,46 @@ __device__ __forceinline__ void box_axis(float p, float r, float inv, int dim, i
 // cells [lo, lo + span] per axis, as physical coordinates. `all`: every cell.
 // A sample farther than `half` cells from `centre` along an axis, modulo the
 // grid's dims, has a box that does not meet them (two cells of slack for the
-// roundings): the test of nearly every sample of a march, at a tenth of the
-// cost of the box itself.
+// roundings).
 struct RayRegion {
     int first[3], span[3];
     float centre[3], half[3];
     bool all;
 };
 
-__device__ __forceinline__ bool far_from(const RayRegion& g, int a, float p, float inv, float dim, float inv_dim)
+// Samples from the one at p on, `move` cells apart along the axis, that are
+// sure to be that far: the distance modulo the dims shrinks by at most `move`
+// per sample. So a march passes over the samples that cannot matter in strides,
+// at one addition each (the sample's t is the repeated sum).
+__device__ __forceinline__ int far_samples(float p, float inv, float centre, float half, float dim, float move)
 {
-    const float c = p * inv, w = c - g.centre[a];
+    const float c = p * inv, w = c - centre;
+    const float e = fabsf(fmaf(-dim, rintf(w / dim), w)) - half;
     // (a sample whose cells the 2^20 origin may clamp is left to the box)
-    return fabsf(c) < 1e6f && fabsf(fmaf(-dim, rintf(w * inv_dim), w)) > g.half[a];
+    return fabsf(c) < 1e6f && e > 0.f ? (int)fminf(e / move, 1e6f) + 1 : 0;
 }
+
+// per-sample movement along the axes, in cells, and the grid's dims
+struct RayMoves {
+    float move[3], dim[3];
+    __device__ __forceinline__ RayMoves(const GridDev& g, const Ray& r, float march_step, float max_distance);
+};
 
 __device__ __forceinline__ int wrap_dim(unsigned v, int dim)
 {
     return (int)((dim & (dim - 1)) == 0 ? v & (unsigned)(dim - 1) : v % (unsigned)dim);
+}
+
+__device__ __forceinline__ RayMoves::RayMoves(const GridDev& g, const Ray& r, float march_step, float max_distance)
+{
+    const float step = march_step + 1.2e-7f * fminf(max_distance, 1e30f);  // with the rounding of t
+    const float d[3] = {r.dx, r.dy, r.dz};
+    const int dims[3] = {g.dx, g.dy, g.dz};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        move[a] = fabsf(d[a]) * step * g.inv * 1.01f + 1e-3f;
+        dim[a] = (float)dims[a];
+    }
 }
 
 // whether the physical cells of the virtual run [lo, hi] meet those of the region's axis a
@@ -377,17 +405,24 @@ __device__ __noinline__ bool march(const GridDev& g, const float4* __restrict__ 
     bool hit = false;
     // previous query box, empty at first (every cell then counts as new)
     int pxl = 0, pxh = -1, pyl = 0, pyh = -1, pzl = 0, pzh = -1;
-    const float fx = (float)g.dx, fy = (float)g.dy, fz = (float)g.dz;
-    const float ifx = 1.f / fx, ify = 1.f / fy, ifz = 1.f / fz;
+    const RayMoves mv(g, r, march_step, max_distance);
     int s = 0;
     float t = 0.f;
     while (s < max_steps && t <= max_distance && t <= best && t <= stop) {
-        if (!region.all && (far_from(region, 0, fmaf(r.dx, t, r.ox), g.inv, fx, ifx) ||
-                            far_from(region, 1, fmaf(r.dy, t, r.oy), g.inv, fy, ify) ||
-                            far_from(region, 2, fmaf(r.dz, t, r.oz), g.inv, fz, ifz))) {
-            ++s;
-            t = __fadd_rn(t, march_step);
-            continue;
+        if (!region.all) {
+            int far = 0;
+            const float p[3] = {fmaf(r.dx, t, r.ox), fmaf(r.dy, t, r.oy), fmaf(r.dz, t, r.oz)};
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+                far = max(far, far_samples(p[a], g.inv, region.centre[a], region.half[a], mv.dim[a], mv.move[a]));
+            if (far > 0) {
+                const float lim = fminf(fminf(max_distance, best), stop);
+                do {
+                    ++s;
+                    t = __fadd_rn(t, march_step);
+                } while (--far > 0 && s < max_steps && t <= lim);
+                continue;
+            }
         }
         int xl, xh, yl, yh, zl, zh;
         box_axis(__fadd_rn(r.ox, __fmul_rn(r.dx, t)), search_radius, g.inv, g.dx, xl, xh);
@@ -440,12 +475,18 @@ __device__ __noinline__ bool march(const GridDev& g, const float4* __restrict__ 
 // nearest computed hit of the warp's rays over all spheres: a depth-first walk
 // of the tree shared by the warp, nearest child first. `best` is the bound on
 // entry; returns the sphere's Morton position or -1.
+// kList: instead, the Morton positions of all hits below `best` into list (at
+// most kRayList; a ray with more drops out), returning their number.
+constexpr int kRayList = 8;
+
+template <bool kList>
 __device__ __forceinline__ int nearest_hit(const RayTree& tree, const float4* __restrict__ sorted, int n,
-                                           const Ray& r, bool live, float max_distance, float& best, int2* stack)
+                                           const Ray& r, bool live, float max_distance, float& best, int2* stack,
+                                           int* list = nullptr)
 {
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    int who = -1;
+    int who = kList ? 0 : -1;
     if (!live) best = -1.f;
     // a zero component would give 0 x inf on a box face
     auto inverse = [](float d) { return 1.f / (fabsf(d) < 1e-12f ? copysignf(1e-12f, d) : d); };
@@ -468,8 +509,16 @@ __device__ __forceinline__ int nearest_hit(const RayTree& tree, const float4* __
                 if (!(q.w > 0.f)) continue;
                 const float th = ray_sphere(r, q);
                 if (th >= 0.f && th <= max_distance && th < best) {
-                    best = th;
-                    who = first + c;
+                    if (kList) {
+                        if (who < kRayList)
+                            list[who] = first + c;
+                        else
+                            best = -1.f;
+                        ++who;
+                    } else {
+                        best = th;
+                        who = first + c;
+                    }
                 }
             }
             continue;
@@ -514,6 +563,100 @@ __device__ __forceinline__ int nearest_hit(const RayTree& tree, const float4* __
     return who;
 }
 
+// The march of a ray whose computed hits are the spheres list[0 .. count), all
+// of them: which of them a taken sample's box holds decides the depth, and no
+// other candidate matters. False when a sphere's cell may be clamped.
+__device__ __noinline__ bool march_few(const GridDev& g, const float4* __restrict__ sorted, const int* list, int count,
+                                       const Ray& r, float max_distance, float search_radius, float march_step,
+                                       int max_steps, float& best)
+{
+    // (the box's two cells of slack hold the roundings of coordinates this small)
+    if (!(fmaxf(fmaxf(fabsf(r.ox), fabsf(r.oy)), fabsf(r.oz)) * g.inv < 1e6f)) return false;
+    float hit[kRayList], cell[kRayList][3];
+    for (int i = 0; i < count; ++i) {
+        const float4 q = sorted[list[i]];
+        hit[i] = ray_sphere(r, q);
+        const float x[3] = {q.x, q.y, q.z};
+        for (int a = 0; a < 3; ++a) {
+            const float c = __fmul_rn(x[a], g.inv);
+            if (!(fabsf(c) < 1e6f)) return false;
+            cell[i][a] = (float)trunc_sat(c);
+        }
+    }
+    const RayMoves mv(g, r, march_step, max_distance);
+    const float half = 0.5f + search_radius * g.inv + 2.f;
+    unsigned left = (1u << count) - 1u;  // spheres no sample has tested
+    int s = 0;
+    float t = 0.f;
+    while (left && s < max_steps && t <= max_distance && t <= best) {
+        int far = 1 << 30;
+        const float p[3] = {fmaf(r.dx, t, r.ox), fmaf(r.dy, t, r.oy), fmaf(r.dz, t, r.oz)};
+        for (int i = 0; i < count; ++i) {
+            if (!((left >> i) & 1u)) continue;
+            int f = 0;
+            for (int a = 0; a < 3; ++a)
+                f = max(f, far_samples(p[a], g.inv, cell[i][a] + 0.5f, half, mv.dim[a], mv.move[a]));
+            far = min(far, f);
+        }
+        if (far == 0) {
+            int xl, xh, yl, yh, zl, zh;
+            box_axis(__fadd_rn(r.ox, __fmul_rn(r.dx, t)), search_radius, g.inv, g.dx, xl, xh);
+            box_axis(__fadd_rn(r.oy, __fmul_rn(r.dy, t)), search_radius, g.inv, g.dy, yl, yh);
+            box_axis(__fadd_rn(r.oz, __fmul_rn(r.dz, t)), search_radius, g.inv, g.dz, zl, zh);
+            for (int i = 0; i < count; ++i) {
+                auto holds = [&](int lo, int hi, float c, int dim) {
+                    const int pc = wrap_dim((unsigned)((int)c + (int)kOrigin), dim);
+                    for (int v = lo; v <= hi; ++v)
+                        if (phys_axis(v, dim) == pc) return true;
+                    return false;
+                };
+                if (((left >> i) & 1u) && holds(xl, xh, cell[i][0], g.dx) && holds(yl, yh, cell[i][1], g.dy) &&
+                    holds(zl, zh, cell[i][2], g.dz)) {
+                    left &= ~(1u << i);
+                    best = fminf(best, hit[i]);
+                }
+            }
+            far = 1;
+        }
+        const float lim = fminf(max_distance, best);
+        do {
+            ++s;
+            t = __fadd_rn(t, march_step);
+        } while (--far > 0 && s < max_steps && t <= lim);
+    }
+    return true;
+}
+
+// The samples with t <= th are all taken: does the box of one of the last of
+// them hold the cell of sphere q, hit at th?
+__device__ __forceinline__ bool held_before(const GridDev& g, const Ray& r, float4 q, float th, float max_distance,
+                                            float search_radius, float march_step, int max_steps)
+{
+    const int cx = phys_axis(trunc_sat(__fmul_rn(q.x, g.inv)), g.dx),
+              cy = phys_axis(trunc_sat(__fmul_rn(q.y, g.inv)), g.dy),
+              cz = phys_axis(trunc_sat(__fmul_rn(q.z, g.inv)), g.dz);
+    auto holds = [](int lo, int hi, int c, int dim) {
+        if ((long long)lo + kOrigin < 0) return false;  // clamped cells: left to the march
+        int d = c - wrap_dim((unsigned)(lo + (int)kOrigin), dim);
+        if (d < 0) d += dim;
+        return d <= hi - lo;
+    };
+    int s = 0;
+    float t = 0.f;
+    while (s < max_steps && t <= max_distance && t <= th) {
+        if (t + 4.f * march_step > th) {
+            int xl, xh, yl, yh, zl, zh;
+            box_axis(__fadd_rn(r.ox, __fmul_rn(r.dx, t)), search_radius, g.inv, g.dx, xl, xh);
+            box_axis(__fadd_rn(r.oy, __fmul_rn(r.dy, t)), search_radius, g.inv, g.dy, yl, yh);
+            box_axis(__fadd_rn(r.oz, __fmul_rn(r.dz, t)), search_radius, g.inv, g.dz, zl, zh);
+            if (holds(xl, xh, cx, g.dx) && holds(yl, yh, cy, g.dy) && holds(zl, zh, cz, g.dz)) return true;
+        }
+        ++s;
+        t = __fadd_rn(t, march_step);
+    }
+    return false;
+}
+
 constexpr int kRayStack = kRayLevels * kRayArity;
 
 // a warp takes a tile of 8 x 4 pixels, a block one of 16 x 8
@@ -533,46 +676,36 @@ __global__ void __launch_bounds__(128) k_raycast(const __grid_constant__ GridDev
     float* out = depth + (live ? (size_t)py * cam.width + px : 0);
     const float had = live ? (*out < 0.f ? cam.max_distance : *out) : 0.f;
     float best = had;
-    const int who = nearest_hit(tree, sorted, n, r, live, cam.max_distance, best, stacks[warp]);
-    if (!live || who < 0) return;
-
-    // the samples with t <= best are all taken: does one of the last of them
-    // hold the sphere's cell?
-    const float4 q = sorted[who];
-    const int cx = phys_axis(trunc_sat(__fmul_rn(q.x, g.inv)), g.dx), cy = phys_axis(trunc_sat(__fmul_rn(q.y, g.inv)), g.dy),
-              cz = phys_axis(trunc_sat(__fmul_rn(q.z, g.inv)), g.dz);
-    auto holds = [](int lo, int hi, int c, int dim) {
-        if ((long long)lo + kOrigin < 0) return false;  // clamped cells: left to the march
-        int d = c - wrap_dim((unsigned)(lo + (int)kOrigin), dim);
-        if (d < 0) d += dim;
-        return d <= hi - lo;
-    };
-    int s = 0;
-    float t = 0.f;
-    while (s < max_steps && t <= cam.max_distance && t <= best) {
-        if (t + 4.f * march_step > best) {
-            int xl, xh, yl, yh, zl, zh;
-            box_axis(__fadd_rn(r.ox, __fmul_rn(r.dx, t)), search_radius, g.inv, g.dx, xl, xh);
-            box_axis(__fadd_rn(r.oy, __fmul_rn(r.dy, t)), search_radius, g.inv, g.dy, yl, yh);
-            box_axis(__fadd_rn(r.oz, __fmul_rn(r.dz, t)), search_radius, g.inv, g.dz, zl, zh);
-            if (holds(xl, xh, cx, g.dx) && holds(yl, yh, cy, g.dy) && holds(zl, zh, cz, g.dz)) {
-                *out = best;
-                return;
-            }
-        }
-        ++s;
-        t = __fadd_rn(t, march_step);
-    }
-
+    const int who = nearest_hit<false>(tree, sorted, n, r, live, cam.max_distance, best, stacks[warp]);
     const float nearest = best, rmax = tree.node(tree.levels - 1, 0)->w;
-    const float cell = 1.f / g.inv;
-    for (float window = 4.f * (search_radius + march_step);; window *= 4.f) {
+    float window = 4.f * (search_radius + march_step);
+    bool open = live && who >= 0;  // the depth is not known yet
+    if (open && held_before(g, r, sorted[who], nearest, cam.max_distance, search_radius, march_step, max_steps)) {
+        *out = nearest;
+        open = false;
+    }
+    // one window, then the ray's hits if they are few, then wider windows
+    for (int round = 0; __any_sync(0xffffffffu, open); ++round) {
+        if (round == 1) {
+            int list[kRayList];
+            best = had;
+            const int count = nearest_hit<true>(tree, sorted, n, r, open, cam.max_distance, best, stacks[warp], list);
+            if (open && count <= kRayList) {
+                best = had;
+                if (march_few(g, sorted, list, count, r, cam.max_distance, search_radius, march_step, max_steps, best)) {
+                    if (best < had) *out = best;
+                    open = false;
+                }
+            }
+            continue;
+        }
+        if (!open) continue;
         // centres of spheres hit in [nearest, until]: within `w` of the ray's
         // points at [nearest - w, until + w]
         const float until = nearest + window;
         const float w = 1.001f * reach(rmax, until + 2.f * rmax) + 1e-5f * until;
         RayRegion region;
-        region.all = !(until < cam.max_distance && max_steps < (1 << 24) && window < 1e6f * cell);
+        region.all = !(until < cam.max_distance && max_steps < (1 << 24) && window * g.inv < 1e6f);
         const float o[3] = {r.ox, r.oy, r.oz}, d[3] = {r.dx, r.dy, r.dz};
         const int dims[3] = {g.dx, g.dy, g.dz};
 #pragma unroll
@@ -593,8 +726,9 @@ __global__ void __launch_bounds__(128) k_raycast(const __grid_constant__ GridDev
         // a march that ended on a hit inside the window is the reference's
         if (region.all || (hit && best <= until)) {
             if (hit) *out = best;
-            return;
+            open = false;
         }
+        window *= 4.f;
     }
 }
 

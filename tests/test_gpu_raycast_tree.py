@@ -86,3 +86,28 @@ def test_tree_sizes(oracle_mod, n):
     raw, _ = _device_depth(x, r, (128, 128, 128), cam, sr, step, steps, init)
     ref = oracle_mod.raycast_particles(x, r, (128, 128, 128), ocam, sr, step, steps, depth_init=init, clamp=False)
     np.testing.assert_array_equal(raw, ref)
+
+
+@pytest.mark.parametrize("offset", [0.0, 700.0, 2.0e5])
+@pytest.mark.parametrize("k", [1, 7, 8, 9, 24])
+def test_few_hits(oracle_mod, k, offset):
+    """Rays whose nearest hits no sample's box holds, and that cross as many
+    spheres as the list of all hits has places, fewer and more; near the
+    origin, and where coordinates are coarse."""
+    rng = np.random.default_rng(k)
+    column = np.zeros((k, 3), np.float32)
+    column[:, 0] = np.linspace(0.0, 1.5, k)
+    column[:, 1:] = rng.uniform(-0.03, 0.03, (k, 2))
+    x = np.concatenate([column, rng.uniform(-0.5, 1.5, (200, 3))]).astype(np.float32) + np.float32(offset)
+    r = np.full(len(x), 0.01, np.float32)
+    r[:k] = rng.uniform(0.03, 0.2, k)  # much wider than the search radius
+    far = 3.5
+    pos = tuple(float(np.float32(offset) + np.float32(c)) for c in (-1.0, 0.003, -0.002))
+    cam, ocam = _camera(oracle_mod, pos, (1, 0.001, 0.002), (0, 0, 1), 0.25, 36, 28, far)
+    init = np.full((28, 36), np.float32(far), np.float32)
+    for sr, step, dims in ((0.012, 0.006, (128,) * 3), (0.02, 0.013, (23, 16, 9)), (0.004, 0.0001, (64,) * 3)):
+        sr, step = float(np.float32(sr)), float(np.float32(step))
+        steps = int(far / step) + 2
+        raw, _ = _device_depth(x, r, dims, cam, sr, step, steps, init)
+        ref = oracle_mod.raycast_particles(x, r, dims, ocam, sr, step, steps, depth_init=init, clamp=False)
+        np.testing.assert_array_equal(raw, ref)
