@@ -1395,6 +1395,10 @@ struct AdjIO {
     const float* inv_mass;
     const float* gravity;
     float4* gd;    // sorted: adj(a), adj(dv) of particle k at 2k, 2k + 1
+    float4* xv;    // sorted: the adjoints of x and v so far, at 2k, 2k + 1 (the particle arrays, in original
+                   // order, are only read by the first pass and only written by the last one: adding to
+                   // their scattered rows in place, where a line's rows belong to blocks on both dies,
+                   // made each addition wait for the other die's L2)
     float* rho;    // sorted: adj(rho)
     float* bpart;  // per block: partial adj(B)
     const float4* acc;  // or null: the forward's sorted (a, 0), (dv, 0) (the segment tape), else recomputed
@@ -1420,10 +1424,8 @@ __global__ void __launch_bounds__(kSphThreads, 2) k_adj_local(GridDev g, const f
         float fb[3] = {0.f, 0.f, 0.f};
         float4 gk = make_float4(0.f, 0.f, 0.f, 0.f), dk = gk;
         if (!(attr & kAttrActive)) {
-            for (int c = 0; c < 3; ++c) {
-                io.x_in_adj[3 * i + c] = xb1[c];
-                io.v_in_adj[3 * i + c] = vb1[c];
-            }
+            io.xv[2 * (size_t)k] = make_float4(xb1[0], xb1[1], xb1[2], 0.f);
+            io.xv[2 * (size_t)k + 1] = make_float4(vb1[0], vb1[1], vb1[2], 0.f);
         } else {
             ForceAcc acc{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             if (io.acc) {
@@ -1475,10 +1477,8 @@ __global__ void __launch_bounds__(kSphThreads, 2) k_adj_local(GridDev g, const f
                 const float dot = uh[0] * vcb[0] + uh[1] * vcb[1] + uh[2] * vcb[2];
                 for (int c = 0; c < 3; ++c) ub[c] = s * (vcb[c] - uh[c] * dot);
             }
-            for (int c = 0; c < 3; ++c) {
-                io.x_in_adj[3 * i + c] = xpb[c];
-                io.v_in_adj[3 * i + c] = ub[c];
-            }
+            io.xv[2 * (size_t)k] = make_float4(xpb[0], xpb[1], xpb[2], 0.f);
+            io.xv[2 * (size_t)k + 1] = make_float4(ub[0], ub[1], ub[2], 0.f);
             if (dynamic) {
                 gk = make_float4(ub[0] * p.dt, ub[1] * p.dt, ub[2] * p.dt, 0.f);
                 dk = make_float4(ub[0] * p.xsph_eps, ub[1] * p.xsph_eps, ub[2] * p.xsph_eps, 0.f);
@@ -1575,10 +1575,15 @@ __global__ void __launch_bounds__(kSphThreads, 2) k_adj_pair(GridDev g, const fl
             }
         }
         if (sub != 0 || kt >= n) continue;
+        const float4 x0 = io.xv[2 * (size_t)k], v0 = io.xv[2 * (size_t)k + 1];
+        io.v_in_adj[3 * i + 0] = active ? v0.x + vb[0] : v0.x;
+        io.v_in_adj[3 * i + 1] = active ? v0.y + vb[1] : v0.y;
+        io.v_in_adj[3 * i + 2] = active ? v0.z + vb[2] : v0.z;
         if (!active) {
             io.rho[k] = 0.f;
             continue;
         }
+        io.xv[2 * (size_t)k] = make_float4(x0.x + xb[0], x0.y + xb[1], x0.z + xb[2], 0.f);
         // adj(rho) from p/rho^2 (through the EOS) and m/rho
         const float2 rpk = rp[k];
         float rb = io.rho_out_adj ? io.rho_out_adj[i] : 0.f;
@@ -1595,10 +1600,6 @@ __global__ void __launch_bounds__(kSphThreads, 2) k_adj_pair(GridDev g, const fl
             if (live) bsum += pr2b * (pw - 1.f) * inv_rho2;
         }
         io.rho[k] = rb;
-        for (int c = 0; c < 3; ++c) {
-            io.x_in_adj[3 * i + c] += xb[c];
-            io.v_in_adj[3 * i + c] += vb[c];
-        }
     }
     bsum = block_sum(bsum);
     if (threadIdx.x == 0) io.bpart[blockIdx.x] = bsum;
@@ -1612,6 +1613,7 @@ __global__ void __launch_bounds__(kSphThreads, 3) k_adj_density(GridDev g, const
                                                                 const int4* __restrict__ nbr,
                                                                 const int* __restrict__ ncnt,
                                                                 const float* __restrict__ rho_adj,
+                                                                const float4* __restrict__ xv,
                                                                 float* __restrict__ x_in_adj)
 {
     launch_entry();
@@ -1635,9 +1637,12 @@ __global__ void __launch_bounds__(kSphThreads, 3) k_adj_density(GridDev g, const
             xb[2] += c * dz;
         });
         for (int c = 0; c < 3; ++c) xb[c] = lanes_sum<kLanes>(xb[c]);
-        if (sub != 0 || !active) continue;
+        if (sub != 0 || kt >= n) continue;
         const size_t i = (size_t)g.ids[k];
-        for (int c = 0; c < 3; ++c) x_in_adj[3 * i + c] += xb[c];
+        const float4 x0 = xv[2 * (size_t)k];
+        x_in_adj[3 * i + 0] = active ? x0.x + xb[0] : x0.x;
+        x_in_adj[3 * i + 1] = active ? x0.y + xb[1] : x0.y;
+        x_in_adj[3 * i + 2] = active ? x0.z + xb[2] : x0.z;
     }
 }
 
@@ -2073,6 +2078,7 @@ struct nsph_sph {
     int launch_blocks_per_sm = -1;       // neighbour passes: persistent blocks per SM (-1 = default, 0 = one thread per particle)
     int sms = 0;
     float4* adj_gd = nullptr;            // adjoint scratch (nsph_sph_enable_adjoint), sorted: adj(a), adj(dv) at 2k, 2k + 1
+    float4* adj_xv = nullptr;            //   the adjoints of x and v so far
     float* adj_rho = nullptr;            //   adj(rho)
     float* adj_bpart = nullptr;          //   per-block partial sums of adj(B)
     int adj_bcap = 0;                    //   entries of adj_bpart
@@ -2233,6 +2239,7 @@ static void sph_free(nsph_sph* s)
     cudaFree(s->wparams);
     cudaFree(s->status);
     cudaFree(s->adj_gd);
+    cudaFree(s->adj_xv);
     cudaFree(s->adj_rho);
     cudaFree(s->adj_bpart);
     cudaFree(s->sfeat);
@@ -2699,6 +2706,7 @@ extern "C" int nsph_sph_enable_adjoint(nsph_sph* s)
     const size_t c = (size_t)(s->capacity > 0 ? s->capacity : 1);
     const int bcap = (int)((c + 31) / 32) + 1;  // blocks of a pass of >= 32 threads per block, or of 64 particles
     cudaError_t e = cudaMalloc(&s->adj_gd, sizeof(float4) * 2 * c);
+    if (e == cudaSuccess) e = cudaMalloc(&s->adj_xv, sizeof(float4) * 2 * c);
     if (e == cudaSuccess) e = cudaMalloc(&s->adj_rho, sizeof(float) * c);
     if (e == cudaSuccess) e = cudaMalloc(&s->adj_bpart, sizeof(float) * (size_t)bcap);
     cudaFuncAttributes fa;
@@ -2710,9 +2718,10 @@ extern "C" int nsph_sph_enable_adjoint(nsph_sph* s)
     if (e != cudaSuccess) {
         cudaGetLastError();
         cudaFree(s->adj_gd);
+        cudaFree(s->adj_xv);
         cudaFree(s->adj_rho);
         cudaFree(s->adj_bpart);
-        s->adj_gd = nullptr;
+        s->adj_gd = s->adj_xv = nullptr;
         s->adj_rho = s->adj_bpart = nullptr;
         return fail(NSPH_ERR_OUT_OF_MEMORY, std::string("adjoint allocation: ") + cudaGetErrorString(e));
     }
@@ -2744,10 +2753,10 @@ static int adjoint_kernels(nsph_sph* s, const nsph_sph_params* p, int n, const G
     if (mark && s->eva[4]) NSPH_CUDA_TRY(record_mark(s->eva[4], cs));
     if (quad)
         NSPH_CUDA_TRY(launch_dependent(k_adj_density<4>, pair_blocks, pair_threads, 0, cs,
-                                       g, ts.xs, ts.vs, n, *p, ts.nbr, ts.ncnt, io.rho, io.x_in_adj));
+                                       g, ts.xs, ts.vs, n, *p, ts.nbr, ts.ncnt, io.rho, io.xv, io.x_in_adj));
     else
         NSPH_CUDA_TRY(launch_dependent(k_adj_density<1>, pair_blocks, pair_threads, 0, cs,
-                                       g, ts.xs, ts.vs, n, *p, ts.nbr, ts.ncnt, io.rho, io.x_in_adj));
+                                       g, ts.xs, ts.vs, n, *p, ts.nbr, ts.ncnt, io.rho, io.xv, io.x_in_adj));
     NSPH_LAUNCH_CHECK("k_adj_density");
     launches += 3;
     if (eos_b_adj) {
@@ -2782,7 +2791,7 @@ static int adjoint_enqueue(nsph_sph* s, const nsph_sph_params* p, int n, const f
         if (s->eva[2]) NSPH_CUDA_TRY(record_mark(s->eva[2], cs));
         ++launches;
         const AdjIO io{x_out_adj, v_out_adj, rho_out_adj, x_in_adj, v_in_adj, f_ext_adj, f_ext, inv_mass, gravity,
-                       s->adj_gd, s->adj_rho, s->adj_bpart};
+                       s->adj_gd, s->adj_xv, s->adj_rho, s->adj_bpart};
         const TapeStep ts{s->xs, s->vs, s->aux, s->rp, s->fr, s->nbr, s->ncnt, nullptr, nullptr, nullptr};
         st = adjoint_kernels(s, p, n, g, ts, io, eos_b_adj, cs, launches, true);
         if (st != NSPH_OK) return st;
@@ -2967,7 +2976,7 @@ extern "C" int nsph_sph_segment_adjoint(nsph_sph* s, const nsph_sph_params* p, i
     s->last_n = n;
     // reverse, from the slots
     AdjIO io{x_adj, v_adj, nullptr, x_adj, v_adj, f_ext_adj, f_ext, inv_mass, gravity,
-             s->adj_gd, s->adj_rho, s->adj_bpart, nullptr};
+             s->adj_gd, s->adj_xv, s->adj_rho, s->adj_bpart, nullptr};
     for (int t = steps - 1; t >= 0; --t) {
         const TapeStep ts = tape_slot(s, t);
         io.acc = ts.acc;
