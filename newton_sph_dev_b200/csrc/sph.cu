@@ -431,7 +431,6 @@ constexpr int kTileSpan = 12;     // x cells between the first and the last part
 
 // resident blocks per SM of the density passes (registers: see the kernels)
 constexpr int kDensityBlocks = 4;
-constexpr int kSmallDensity = 65536;  // particles below which its blocks are small
 
 struct __align__(16) TileSmem {
     union {
@@ -947,6 +946,174 @@ __device__ __forceinline__ void integrate_out(size_t i, float4 xi, float4 vi, in
     o.v_out[3 * i + 2] = v1z;
 }
 
+// ---- the density pass of a small scene: eight lanes per particle -----------------
+// A tile's warp is one long chain of dependent work (50,000 cycles and more),
+// which nothing hides while there are only a few warps per SM. Here the
+// candidates of a particle's query box, its rows' runs one after another, are
+// dealt to eight lanes in equal stretches: each tests its own into bit marks, a
+// prefix sum over the lanes gives each one's place in the list, the lanes
+// evaluate their neighbours' kernel values into shared memory at those places,
+// and the sum over them runs in order. Same sets, order and roundings as the
+// general scan, which takes a particle whose box has clamped cells, wraps in
+// x, has more than 16 rows or 512 candidates, or whose list overflows.
+constexpr int kOctetThreads = 128;
+constexpr int kOctetParticles = kOctetThreads / 8;
+// Density pass on a B200: 14 us instead of 28 at 1,000 to 4,096 particles, 21
+// and 30 at 15,625, 29 and 29 at 24,389, 36 and 34 at 32,768, 157 and 70 at
+// 219k (it issues three times the instructions); hence kOctetMax.
+constexpr int kOctetMax = 16384;
+
+struct OctetSmem {
+    float2 terms[kNbrSlots + 1];  // (m, W) by place in the list
+    int off[17];                  // candidate t of row r is at sorted position t + off[r]
+    int upto[17];                 //   for t < upto[r] (the last entry ends every row)
+};
+
+template <bool Fast>
+__device__ __forceinline__ int octet_neighbors(const GridDev& g, const float4* __restrict__ xs,
+                                               const nsph_sph_params& p, float4 xi, bool active,
+                                               int4* __restrict__ nbr, int n, int k, OctetSmem& sm, float& rho_out)
+{
+    constexpr unsigned kAll = 0xffffffffu;
+    const int sub = threadIdx.x & 7;
+    int xl, xh, yl, yh, zl, zh;
+    bool general = !active;
+    box_axis_regular(xi.x, p.h, g.inv, g.dx, xl, xh, general);
+    box_axis_regular(xi.y, p.h, g.inv, g.dy, yl, yh, general);
+    box_axis_regular(xi.z, p.h, g.inv, g.dz, zl, zh, general);
+    const int nx = xh - xl + 1, ny = yh - yl + 1;
+    const int cx = general ? 0 : wrap_cell(xl, g.dx);
+    general = general || cx + nx > g.dx || (long long)ny * (zh - zl + 1) > 16;
+    const int rows = general ? 0 : ny * (zh - zl + 1);
+    // rows sub and sub + 8: their runs, and the candidates up to each
+    int lo[2] = {0, 0}, num[2] = {0, 0};
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int row = sub + 8 * h;
+        if (row < rows) {
+            const int iz = ny == 3 ? (row * 0x5556) >> 16 : row / ny, iy = row - iz * ny;
+            const int2* cell = g.ranges + (wrap_cell(zl + iz, g.dz) * g.dy + wrap_cell(yl + iy, g.dy)) * g.dx + cx;
+            int first = 0x7fffffff, end = 0;
+#pragma unroll 3
+            for (int c = 0; c < nx; ++c) {
+                const int2 se = __ldg(cell + c);
+                if (se.y > se.x && in_bounds(se.x >= 0 && se.y <= g.n)) {
+                    first = min(first, se.x);
+                    end = max(end, se.y);
+                }
+            }
+            lo[h] = first;
+            num[h] = max(end - first, 0);
+        }
+    }
+    int cands = 0;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        int inc = num[h];
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            const int y = __shfl_up_sync(kAll, inc, o, 8);
+            if (sub >= o) inc += y;
+        }
+        const int row = sub + 8 * h;
+        if (row < rows) {
+            sm.off[row] = lo[h] - (cands + inc - num[h]);
+            sm.upto[row] = cands + inc;
+        }
+        cands += __shfl_sync(kAll, inc, 7, 8);
+    }
+    if (sub == 0) sm.upto[rows] = 0x7fffffff;
+    __syncwarp();
+    const int each = (cands + 7) >> 3;  // candidates per lane
+    general = general || each > 64;
+    const int t0 = sub * each, t1 = general ? t0 : min(t0 + each, cands);
+    // the row of candidate t0 (rows without candidates are passed over)
+    int r0 = 0;
+    if (t0 < t1)
+        while (sm.upto[r0] <= t0) ++r0;
+    unsigned marks[2] = {0u, 0u};
+    {
+        int r = r0, next = sm.upto[r], off = sm.off[r];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            unsigned bits = 0u;
+            const int end = min(t1, t0 + 32 * (c + 1));
+            for (int t = t0 + 32 * c; t < end; t += 4) {
+                float4 xj[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int tu = min(t + u, end - 1);
+                    if (tu >= next) {
+                        do {
+                            ++r;
+                            next = sm.upto[r];
+                        } while (tu >= next);
+                        off = sm.off[r];
+                    }
+                    xj[u] = __ldg(xs + tu + off);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    float dx, dy, dz;
+                    const bool hit = dist2(xi, xj[u], dx, dy, dz) < p.h2 && !mirror_inactive(xj[u]) && t + u < end;
+                    bits |= (hit ? 1u : 0u) << (t - t0 - 32 * c + u);
+                }
+            }
+            marks[c] = bits;
+        }
+    }
+    const int mine = __popc(marks[0]) + __popc(marks[1]);
+    int inc = mine;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+        const int y = __shfl_up_sync(kAll, inc, o, 8);
+        if (sub >= o) inc += y;
+    }
+    const int total = __shfl_sync(kAll, inc, 7, 8);
+    general = general || total > kNbrSlots;
+    if (!general) {
+        int at = inc - mine;
+        int r = r0, next = sm.upto[r], off = sm.off[r];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            unsigned bits = marks[c];
+            while (bits) {
+                const int t = t0 + 32 * c + __ffs(bits) - 1;
+                bits &= bits - 1u;
+                if (t >= next) {
+                    do {
+                        ++r;
+                        next = sm.upto[r];
+                    } while (t >= next);
+                    off = sm.off[r];
+                }
+                const int j = t + off;
+                const float4 xj = __ldg(xs + j);
+                float dx, dy, dz;
+                const float r2 = dist2(xi, xj, dx, dy, dz);
+                sm.terms[at] = make_float2(xj.w, Fast ? wterm_fast(r2, p) : wterm(r2, p));
+                reinterpret_cast<int*>(nbr + (size_t)(at >> 2) * n + k)[at & 3] = j;
+                ++at;
+            }
+        }
+        // the rest of the last group is the particle itself
+        const int pad = total + sub;
+        if (sub < 3 && (total & 3) && (pad >> 2) == (total >> 2))
+            reinterpret_cast<int*>(nbr + (size_t)(pad >> 2) * n + k)[pad & 3] = k;
+    }
+    __syncwarp();
+    float rho = 0.f;
+    if (!general) {
+#pragma unroll 4
+        for (int t = 0; t < total; ++t) {
+            const float2 mw = sm.terms[t];
+            rho = __fmaf_rn(mw.x, mw.y, rho);
+        }
+    }
+    rho_out = rho;
+    return general ? -1 : total;
+}
+
 // ---- the plain step's passes on neighbour lists ----------------------------------
 template <bool Fast>
 __global__ void __launch_bounds__(kSphThreads, kDensityBlocks) k_density_list(
@@ -980,6 +1147,33 @@ __global__ void __launch_bounds__(kSphThreads, kDensityBlocks) k_density_list(
             fr.rec[2 * (size_t)k] = xi;  // (marked inactive)
             ncnt[k] = 0;
         }
+    }
+}
+
+template <bool Fast>
+__global__ void __launch_bounds__(kOctetThreads) k_density_octet(
+    const __grid_constant__ GridDev g, const float4* __restrict__ xs, const float4* __restrict__ vs, int n,
+    const __grid_constant__ nsph_sph_params p, float2* __restrict__ aux, float2* __restrict__ rp,
+    int4* __restrict__ nbr, int* __restrict__ ncnt, const ForceRec fr, unsigned* __restrict__ status)
+{
+    launch_entry();
+    __shared__ OctetSmem octets[kOctetParticles];
+    const int kt = blockIdx.x * kOctetParticles + threadIdx.x / 8, k = min(kt, n - 1);
+    const float4 xi = xs[k], vi = vs[k];
+    const bool active = kt < n && (__float_as_int(vi.w) & kAttrActive) != 0;
+    float rho;
+    int cnt = octet_neighbors<Fast>(g, xs, p, xi, active, nbr, n, k, octets[threadIdx.x / 8], rho);
+    if ((threadIdx.x & 7) != 0 || kt >= n) return;
+    if (active) {
+        if (cnt < 0) cnt = scan_general<Fast>(&g, xs, &p, xi, nbr, n, k, &rho);
+        ncnt[k] = cnt;
+        if (cnt > kNbrSlots && fr.overflow) atomicOr(fr.overflow, 1u);
+        density_finish<Fast>(k, xi, vi, rho, p, aux, rp, fr, status);
+    } else {
+        aux[k] = make_float2(0.f, 0.f);
+        rp[k] = make_float2(0.f, 0.f);
+        fr.rec[2 * (size_t)k] = xi;  // (marked inactive)
+        ncnt[k] = 0;
     }
 }
 
@@ -1058,9 +1252,12 @@ __global__ void __launch_bounds__(kSphThreads, 4) k_force_list(GridDev g, const 
 // of the group's four terms in order, so every rounding is k_force_list's.
 // It spends about 1.4 times the instructions, but a particle's chain of
 // dependent work is a third as long and there are four times the warps, which
-// is what bounds scenes that do not fill the SMs.
+// is what bounds scenes that do not fill the SMs. Whole step with it and
+// without on a B200: 25 and 31 us at 2,197 particles, 54 and 59 at 24,389, 66
+// and 64 at 32,768, 76 and 70 at 64,000 (a 64k rollout with its gradient, whose
+// pair passes follow the same rule: 4.25 and 3.87 ms); hence kQuadMax.
 constexpr int kQuadThreads = 256;
-constexpr int kQuadMax = 131072;
+constexpr int kQuadMax = 24576;
 
 __global__ void __launch_bounds__(kQuadThreads, 4) k_force_quad(const __grid_constant__ GridDev g,
                                                                 const float4* __restrict__ xs,
@@ -1209,6 +1406,35 @@ __global__ void __launch_bounds__(kSphThreads, kDensityBlocks) k_density_worlds(
             fr.rec[2 * (size_t)k] = xi;  // (marked inactive)
             ncnt[k] = 0;
         }
+    }
+}
+
+__global__ void __launch_bounds__(kOctetThreads) k_density_octet_worlds(
+    const WorldCells* __restrict__ wc, const nsph_sph_params* __restrict__ wp, const int2* __restrict__ ranges,
+    const int* __restrict__ ids, const float4* __restrict__ xs, const float4* __restrict__ vs, int n,
+    float2* __restrict__ aux, float2* __restrict__ rp, int4* __restrict__ nbr, int* __restrict__ ncnt,
+    const ForceRec fr, unsigned* __restrict__ status)
+{
+    launch_entry();
+    __shared__ OctetSmem octets[kOctetParticles];
+    const int kt = blockIdx.x * kOctetParticles + threadIdx.x / 8, k = min(kt, n - 1);
+    const float4 xi = xs[k], vi = vs[k];
+    const int attr = __float_as_int(vi.w), w = attr >> kAttrGravShift;
+    const bool active = kt < n && (attr & kAttrActive) != 0;
+    const nsph_sph_params& p = wp[w];
+    const GridDev g = world_grid(wc[w], ranges, ids, n);
+    float rho;
+    int cnt = octet_neighbors<false>(g, xs, p, xi, active, nbr, n, k, octets[threadIdx.x / 8], rho);
+    if ((threadIdx.x & 7) != 0 || kt >= n) return;
+    if (active) {
+        if (cnt < 0) cnt = scan_general_world(wc, wp, ranges, ids, w, xs, xi, nbr, n, k, &rho);
+        ncnt[k] = cnt;
+        density_finish(k, xi, vi, rho, p, aux, rp, fr, status);
+    } else {
+        aux[k] = make_float2(0.f, 0.f);
+        rp[k] = make_float2(0.f, 0.f);
+        fr.rec[2 * (size_t)k] = xi;  // (marked inactive)
+        ncnt[k] = 0;
     }
 }
 
@@ -2183,26 +2409,56 @@ static void pass_launch(const nsph_sph* s, int n, bool persistent_default, int& 
 }
 
 // whether the force and adjoint passes take four lanes per particle: scenes of
-// fewer than kQuadMax particles, unless the caller set a launch shape
+// at most kQuadMax particles, unless the caller set a launch shape
 static bool quad_pass(const nsph_sph* s, int n)
 {
-    static const int lim = getenv("NSPH_QUAD") ? atoi(getenv("NSPH_QUAD")) : kQuadMax;
-    return n <= lim && s->launch_threads == 0 && s->launch_blocks_per_sm < 0;
-}
-
-// grid of a density pass: as pass_launch, but small scenes in blocks of two
-// warps, so that their warps spread over the SMs
-static void density_launch(const nsph_sph* s, int n, bool persistent_default, int& blocks, int& threads)
-{
-    pass_launch(s, n, persistent_default, blocks, threads);
-    if (s->launch_threads == 0 && s->launch_blocks_per_sm < 0 && n < kSmallDensity) {
-        threads = 64;
-        blocks = std::max(1, (n + threads - 1) / threads);
-    }
+    return n <= kQuadMax && s->launch_threads == 0 && s->launch_blocks_per_sm < 0;
 }
 
 // shared memory of a density pass: one TileSmem per warp
 static size_t tile_smem_bytes(int threads) { return sizeof(TileSmem) * (size_t)(threads / 32); }
+
+// whether the density pass takes eight lanes per particle, by the same rule
+static bool octet_pass(const nsph_sph* s, int n)
+{
+    return n <= kOctetMax && s->launch_threads == 0 && s->launch_blocks_per_sm < 0;
+}
+
+// How a density pass of tiles is launched. One whose blocks are all resident
+// at once (kDensityBlocks per SM) must not start early: its blocks would be
+// placed while the build's last blocks still hold some of the SMs, two and
+// three on one SM beside an idle one, and the pass lasts as long as its fullest
+// SM. A step took 80 us with the early start and 54 without at 24k particles,
+// 82 and 70 at 64k, 96 and 95 at 125k; larger passes level out over their
+// blocks and gain the launch (116 and 118 us at 166k). A pass of eight lanes
+// per particle is always that small (31 and 25 us at 2,197 particles).
+template <class... P, class... A>
+static cudaError_t launch_tiles(const nsph_sph* s, void (*kernel)(P...), int blocks, int threads, cudaStream_t cs,
+                                A&&... args)
+{
+    return blocks <= s->sms * kDensityBlocks
+               ? launch_plain(kernel, blocks, threads, tile_smem_bytes(threads), cs, std::forward<A>(args)...)
+               : launch_dependent(kernel, blocks, threads, tile_smem_bytes(threads), cs, std::forward<A>(args)...);
+}
+
+// the density pass of a single-world step into the given arrays
+static int density_enqueue(const nsph_sph* s, const GridDev& g, const nsph_sph_params* p, int n, bool fast,
+                           const float4* xs, const float4* vs, float2* aux, float2* rp, int4* nbr, int* ncnt,
+                           const ForceRec& fr, cudaStream_t cs, int& launches)
+{
+    if (octet_pass(s, n)) {
+        const int blocks = (n + kOctetParticles - 1) / kOctetParticles;
+        NSPH_CUDA_TRY(launch_plain(fast ? k_density_octet<true> : k_density_octet<false>, blocks, kOctetThreads,
+                                   0, cs, g, xs, vs, n, *p, aux, rp, nbr, ncnt, fr, s->status));
+    } else {
+        int blocks, threads;
+        pass_launch(s, n, false, blocks, threads);
+        NSPH_CUDA_TRY(launch_tiles(s, fast ? k_density_list<true> : k_density_list<false>, blocks, threads, cs, g, xs,
+                                   vs, n, *p, aux, rp, nbr, ncnt, fr, s->status));
+    }
+    ++launches;
+    return NSPH_OK;
+}
 
 // Record a timing event: as an external event node while the stream is being
 // captured (so a replayed graph records it), as a plain record otherwise.
@@ -2268,6 +2524,9 @@ extern "C" int nsph_sph_create(int device, int capacity, const int grid_dims[3],
         if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_density_list<false>);
         if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_force_list<false>);
         if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_force_quad);
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_density_octet<false>);
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_density_octet<true>);
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_tape_copy);
         if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_density_list<true>);
         if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_force_list<true>);
         if (e != cudaSuccess) {
@@ -2304,6 +2563,7 @@ extern "C" int nsph_sph_create_worlds(int device, int capacity, int world_count,
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_force_worlds, kSphThreads, 0);
         cudaFuncAttributes fa;
         if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_density_worlds);
+        if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_density_octet_worlds);
         if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k_neighbors_worlds);
         if (e != cudaSuccess) {
             cudaGetLastError();
@@ -2404,15 +2664,8 @@ static int step_enqueue(nsph_sph* s, const nsph_sph_params* p, int n, const floa
     if (n > 0) {
         const GridDev g = s->grid.view();
         int blocks, threads;
-        density_launch(s, n, false, blocks, threads);
-        if (s->fast)
-            NSPH_CUDA_TRY(launch_dependent(k_density_list<true>, blocks, threads, tile_smem_bytes(threads), cs,
-                                           g, s->xs, s->vs, n, *p, s->aux, s->rp, s->nbr, s->ncnt, s->fr, s->status));
-        else
-            NSPH_CUDA_TRY(launch_dependent(k_density_list<false>, blocks, threads, tile_smem_bytes(threads), cs,
-                                           g, s->xs, s->vs, n, *p, s->aux, s->rp, s->nbr, s->ncnt, s->fr, s->status));
-        NSPH_LAUNCH_CHECK("k_density_list");
-        ++launches;
+        st = density_enqueue(s, g, p, n, s->fast != 0, s->xs, s->vs, s->aux, s->rp, s->nbr, s->ncnt, s->fr, cs, launches);
+        if (st != NSPH_OK) return st;
         if (s->ev[2]) NSPH_CUDA_TRY(record_mark(s->ev[2], cs));
         pass_launch(s, n, false, blocks, threads);
         const StepOut o{f_ext, inv_mass, gravity, x_out, v_out, rho_out, p_out, a_out, s->status, nullptr, carry_v};
@@ -2553,10 +2806,17 @@ extern "C" int nsph_sph_step_worlds(nsph_sph* s, float dt, int n, const float* x
     if (s->ev[1]) NSPH_CUDA_TRY(record_mark(s->ev[1], cs));
     if (n > 0) {
         int blocks, threads;
-        density_launch(s, n, true, blocks, threads);
-        NSPH_CUDA_TRY(launch_dependent(k_density_worlds, blocks, threads, tile_smem_bytes(threads), cs,
-                                       s->grid.worlds, s->wparams, s->grid.cell_ranges, s->grid.point_ids, s->xs, s->vs, n, s->aux, s->rp, s->nbr, s->ncnt, s->fr, s->status));
-        NSPH_LAUNCH_CHECK("k_density_worlds");
+        if (octet_pass(s, n)) {
+            NSPH_CUDA_TRY(launch_plain(k_density_octet_worlds, (n + kOctetParticles - 1) / kOctetParticles,
+                                       kOctetThreads, 0, cs, s->grid.worlds, s->wparams, s->grid.cell_ranges,
+                                       s->grid.point_ids, s->xs, s->vs, n, s->aux, s->rp, s->nbr, s->ncnt, s->fr,
+                                       s->status));
+        } else {
+            pass_launch(s, n, true, blocks, threads);
+            NSPH_CUDA_TRY(launch_tiles(s, k_density_worlds, blocks, threads, cs, s->grid.worlds, s->wparams,
+                                       s->grid.cell_ranges, s->grid.point_ids, s->xs, s->vs, n, s->aux, s->rp, s->nbr,
+                                       s->ncnt, s->fr, s->status));
+        }
         ++launches;
         if (s->ev[2]) NSPH_CUDA_TRY(record_mark(s->ev[2], cs));
         pass_launch(s, n, true, blocks, threads);
@@ -2783,13 +3043,9 @@ static int adjoint_enqueue(nsph_sph* s, const nsph_sph_params* p, int n, const f
     if (s->eva[1]) NSPH_CUDA_TRY(record_mark(s->eva[1], cs));
     if (n > 0) {
         const GridDev g = s->grid.view();
-        int blocks, threads;
-        density_launch(s, n, false, blocks, threads);
-        NSPH_CUDA_TRY(launch_dependent(k_density_list<false>, blocks, threads, tile_smem_bytes(threads), cs,
-                                       g, s->xs, s->vs, n, *p, s->aux, s->rp, s->nbr, s->ncnt, s->fr, s->status));
-        NSPH_LAUNCH_CHECK("k_density_list");
+        st = density_enqueue(s, g, p, n, false, s->xs, s->vs, s->aux, s->rp, s->nbr, s->ncnt, s->fr, cs, launches);
+        if (st != NSPH_OK) return st;
         if (s->eva[2]) NSPH_CUDA_TRY(record_mark(s->eva[2], cs));
-        ++launches;
         const AdjIO io{x_out_adj, v_out_adj, rho_out_adj, x_in_adj, v_in_adj, f_ext_adj, f_ext, inv_mass, gravity,
                        s->adj_gd, s->adj_xv, s->adj_rho, s->adj_bpart};
         const TapeStep ts{s->xs, s->vs, s->aux, s->rp, s->fr, s->nbr, s->ncnt, nullptr, nullptr, nullptr};
@@ -2932,9 +3188,8 @@ extern "C" int nsph_sph_segment_adjoint(nsph_sph* s, const nsph_sph_params* p, i
     if (!guard.ok) return fail(NSPH_ERR_CUDA, "cannot select CUDA device");
     cudaStream_t cs = (cudaStream_t)stream;
     int launches = 0;
-    int blocks, threads, dblocks, dthreads;
+    int blocks, threads;
     pass_launch(s, n, false, blocks, threads);
-    density_launch(s, n, false, dblocks, dthreads);
     // forward: the build, density and force passes of every step, their
     // outputs into the step's slot (the last step's new state is not used)
     NSPH_CUDA_TRY(cudaMemsetAsync(tape_overflow(s), 0, sizeof(unsigned) * (size_t)steps, cs));
@@ -2947,10 +3202,8 @@ extern "C" int nsph_sph_segment_adjoint(nsph_sph* s, const nsph_sph_params* p, i
         st = grid_build(s->grid, xi, n, p->cell_width, p->cell_inv, &ga, s->status, cs, &launches);
         if (st != NSPH_OK) return st;
         const GridDev g = s->grid.view();
-        NSPH_CUDA_TRY(launch_dependent(k_density_list<false>, dblocks, dthreads, tile_smem_bytes(dthreads), cs,
-                                       g, ts.xs, ts.vs, n, *p, ts.aux, ts.rp, ts.nbr, ts.ncnt, ts.fr, s->status));
-        NSPH_LAUNCH_CHECK("k_density_list");
-        ++launches;
+        st = density_enqueue(s, g, p, n, false, ts.xs, ts.vs, ts.aux, ts.rp, ts.nbr, ts.ncnt, ts.fr, cs, launches);
+        if (st != NSPH_OK) return st;
         float* xo = tape_state(s, (t + 1) & 1);
         float* vo = xo + len;
         // the sorted ids and, where a list overflowed, the cell table into the slot
@@ -3126,11 +3379,8 @@ static int features_enqueue(nsph_sph* s, const nsph_sph_params* p, int n, const 
     if (n > 0) {
         const GridDev g = s->grid.view();
         int threads;
-        density_launch(s, n, false, blocks, threads);
-        NSPH_CUDA_TRY(launch_dependent(k_density_list<false>, blocks, threads, tile_smem_bytes(threads), cs,
-                                       g, s->xs, s->vs, n, *p, s->aux, s->rp, s->nbr, s->ncnt, s->fr, s->status));
-        NSPH_LAUNCH_CHECK("k_density_list");
-        ++launches;
+        st = density_enqueue(s, g, p, n, false, s->xs, s->vs, s->aux, s->rp, s->nbr, s->ncnt, s->fr, cs, launches);
+        if (st != NSPH_OK) return st;
         if (mark && s->eva[2]) NSPH_CUDA_TRY(record_mark(s->eva[2], cs));
         pass_launch(s, n, false, blocks, threads);
         if (features) {
