@@ -15,7 +15,7 @@
 // minimum over the candidates of the samples taken, which does not depend on
 // the order they are tested in.
 //
-// Two facts make most of the march unnecessary:
+// Three facts make most of the march unnecessary:
 // 1. Every hit is at least M, the nearest computed hit over ALL spheres. A
 //    ray without any computed hit leaves its pixel as it is, whatever cells
 //    its march would visit. M comes from a bounding-box tree over the spheres
@@ -23,21 +23,21 @@
 //    rounding of the sphere test, so it misses no computed hit.
 // 2. Every sample with t <= M is taken (nothing stops the march before). So
 //    when the box of such a sample holds the nearest sphere's cell, the depth
-//    is M. Otherwise the march is run, but only over the samples whose box
-//    overlaps (modulo the grid's dims) the cells that can hold a sphere hit
+//    is M. Otherwise, and if 3 does not apply, the march is run, but only over
+//    the samples whose box overlaps (modulo the grid's dims) the cells that can hold a sphere hit
 //    before M + window: spheres hit later cannot stop the march inside the
 //    window, and those that can are tested at these samples only. A march
 //    that leaves the window without a hit is repeated with a wider one, in
 //    the end the reference's whole march.
+// 3. A ray whose nearest hit is not decided so has its computed hits collected
+//    from the tree, up to a distance that grows until the depth is known. Up to
+//    kRayList of them, only these spheres' cells matter: march_few passes over
+//    the samples far from all of them in strides. (Marching over the window's
+//    cells instead, and adding up t sample by sample, the image of the block at
+//    640 x 480 took 1.11 ms, and 0.99 with this.)
 // The march itself tests each cell once per ray: along every axis both ends
 // of the query box are monotone in t, so a cell that an earlier sample tested
 // and that this box still holds was in the previous box.
-//
-// 3. A ray whose first window is empty has all its computed hits collected
-//    from the tree. Up to kRayList of them, only these spheres' cells matter:
-//    march_few passes over the samples far from all of them in strides. (Without
-//    it such rays marched through ever wider windows; the image of the block
-//    at 640 x 480 took 1.11 ms, now 0.99.)
 //
 // The march alone was bound by instruction issue: most rays miss, and each
 // missing ray took every sample up to max_distance through cells that the
@@ -73,10 +73,12 @@ __device__ __forceinline__ float unordered(unsigned u)
 }
 
 // Radius that bounds the centres of spheres whose COMPUTED test can hit,
-// around the ray, at distances up to d from the camera: the discriminant
-// proj^2 - (|o|^2 - r^2) carries at most 20 roundings (2^-24) of d^2, the
-// direction's length included; 2^-18 (64 roundings) is taken.
-__device__ __forceinline__ float reach(float r, float d) { return sqrtf(fmaf(3.8147e-6f * d, d, r * r)) * 1.0001f; }
+// around the ray, at distances up to d from the camera. With u = 2^-24: proj
+// is within 3u d of the dot product and its square within 7u d^2, |o|^2 within
+// 3u d^2, |o|^2 - r^2 rounds by u d^2, the last difference keeps its sign, and
+// the direction's squared length is within 7u of 1: 18u d^2 in all (24u is
+// taken). The rounding of o moves the centre by u d, inside the last factor.
+__device__ __forceinline__ float reach(float r, float d) { return sqrtf(fmaf(1.4306e-6f * d, d, r * r)) * 1.0001f; }
 
 // whether sphere q can be hit within max_distance of the camera at all (its
 // coordinates and radius finite, the radius positive)
@@ -90,13 +92,15 @@ __device__ __forceinline__ bool in_reach(float4 q, const nsph_raycast_camera& c)
 
 // sorted mirror (x, y, z, radius) of the grid's points, and the bounds of the
 // spheres in reach: bounds[a] = max of ordered(x_a), bounds[3 + a] = max of
-// ordered(-x_a), both 0 at first
-__global__ void k_raycast_gather(const int* __restrict__ ids, const float* __restrict__ x,
+// ordered(-x_a), both 0 at first. (One atomic per block and bound: one per warp
+// kept 500,000 spheres' pass waiting on six addresses, 24 us of 26.)
+__global__ void __launch_bounds__(256) k_raycast_gather(const int* __restrict__ ids, const float* __restrict__ x,
                                  const float* __restrict__ radius, int n, const nsph_raycast_camera cam,
                                  float4* __restrict__ m, unsigned* __restrict__ bounds)
 {
     launch_entry();
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ unsigned block[6][8];
+    const int k = blockIdx.x * 256 + threadIdx.x;
     unsigned b[6] = {0u, 0u, 0u, 0u, 0u, 0u};
     if (k < n) {
         const size_t i = (size_t)ids[k];
@@ -114,7 +118,14 @@ __global__ void k_raycast_gather(const int* __restrict__ ids, const float* __res
 #pragma unroll
     for (int a = 0; a < 6; ++a) {
         const unsigned v = __reduce_max_sync(0xffffffffu, b[a]);
-        if ((threadIdx.x & 31) == a && v > bounds[a]) atomicMax(bounds + a, v);
+        if ((threadIdx.x & 31) == a) block[a][threadIdx.x >> 5] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        unsigned v = 0u;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) v = max(v, block[threadIdx.x][w]);
+        if (v > bounds[threadIdx.x]) atomicMax(bounds + threadIdx.x, v);
     }
 }
 
@@ -354,14 +365,45 @@ struct RayRegion {
 
 // Samples from the one at p on, `move` cells apart along the axis, that are
 // sure to be that far: the distance modulo the dims shrinks by at most `move`
-// per sample. So a march passes over the samples that cannot matter in strides,
-// at one addition each (the sample's t is the repeated sum).
+// per sample. So a march passes over the samples that cannot matter in strides.
 __device__ __forceinline__ int far_samples(float p, float inv, float centre, float half, float dim, float move)
 {
     const float c = p * inv, w = c - centre;
     const float e = fabsf(fmaf(-dim, rintf(w / dim), w)) - half;
     // (a sample whose cells the 2^20 origin may clamp is left to the box)
     return fabsf(c) < 1e6f && e > 0.f ? (int)fminf(e / move, 1e6f) + 1 : 0;
+}
+
+// Up to k samples on: ++s and t = t + step, k times, but not beyond the first
+// t > lim nor past max_steps. Within a binade the rounded sum grows by the same
+// multiple of its last place each time (from the second sum inside the binade
+// on, if step lies half way between two), so all additions that stay inside it
+// are one exact product.
+__device__ __forceinline__ void stride(float& t, int& s, int k, float lim, float step, int max_steps)
+{
+    k = min(k, max_steps - s);
+    while (k > 0) {
+        ++s;
+        t = __fadd_rn(t, step);
+        if (--k == 0 || !(t <= lim)) return;
+        const float before = t;
+        ++s;
+        t = __fadd_rn(t, step);
+        if (--k == 0 || !(t <= lim)) return;
+        if ((__float_as_uint(before) ^ __float_as_uint(t)) & 0x7f800000u) continue;
+        const float grow = __fadd_rn(t, step) - t;
+        if (!(grow > 0.f)) {
+            s += k;
+            return;
+        }
+        const float top = __uint_as_float((__float_as_uint(t) & 0x7f800000u) + 0x00800000u);
+        const int j = min(k - 1, (int)fminf((fminf(top, lim) - t) / grow, 1e9f) - 2);
+        if (j > 0) {
+            s += j;
+            t = fmaf((float)j, grow, t);
+            k -= j;
+        }
+    }
 }
 
 // per-sample movement along the axes, in cells, and the grid's dims
@@ -416,11 +458,7 @@ __device__ __noinline__ bool march(const GridDev& g, const float4* __restrict__ 
             for (int a = 0; a < 3; ++a)
                 far = max(far, far_samples(p[a], g.inv, region.centre[a], region.half[a], mv.dim[a], mv.move[a]));
             if (far > 0) {
-                const float lim = fminf(fminf(max_distance, best), stop);
-                do {
-                    ++s;
-                    t = __fadd_rn(t, march_step);
-                } while (--far > 0 && s < max_steps && t <= lim);
+                stride(t, s, far, fminf(fminf(max_distance, best), stop), march_step, max_steps);
                 continue;
             }
         }
@@ -472,63 +510,80 @@ __device__ __noinline__ bool march(const GridDev& g, const float4* __restrict__ 
     return hit;
 }
 
-// nearest computed hit of the warp's rays over all spheres: a depth-first walk
-// of the tree shared by the warp, nearest child first. `best` is the bound on
-// entry; returns the sphere's Morton position or -1.
-// kList: instead, the Morton positions of all hits below `best` into list (at
-// most kRayList; a ray with more drops out), returning their number.
-constexpr int kRayList = 8;
+// A warp takes four rays, eight lanes to a ray. The walk over the tree is shared
+// by the warp, depth-first and nearest child first; a lane tests one of a node's
+// eight children, or of a leaf's spheres, for its ray. (With a ray per lane a warp
+// went over the children one by one for 32 rays' worth of nodes: the few warps that
+// see the scene's edges walked for 1.4 million cycles while the other SMs were
+// idle, 9.6 % of the warps active. Depth image of 640 x 480 pixels, 515,100
+// spheres: this kernel 930 -> 269 us, now bound by issue at 63 %; the whole
+// update 0.99 -> 0.40 ms.)
+constexpr int kRayLanes = 8;
+constexpr int kRayRays = 32 / kRayLanes;
+constexpr int kRayThreads = 128;
+constexpr int kRayTile = 4;  // pixels along each side of a block's tile
+constexpr int kRayStack = kRayLevels * kRayArity;
+constexpr int kRayList = 32;
+static_assert(kRayLanes == kRayArity && kRayThreads / 32 * kRayRays == kRayTile * kRayTile, "");
 
+// over the ray's lanes
+__device__ __forceinline__ unsigned ray_mask() { return 0xffu << (threadIdx.x & 24); }
+
+// Nearest computed hit: `best` is the bound on entry; returns the sphere's
+// Morton position or -1. kList: the Morton positions of all hits up to `best`
+// into list (the first kRayList of them), returning their number. For the whole
+// warp together; the same result in all lanes of a ray.
 template <bool kList>
-__device__ __forceinline__ int nearest_hit(const RayTree& tree, const float4* __restrict__ sorted, int n,
-                                           const Ray& r, bool live, float max_distance, float& best, int2* stack,
-                                           int* list = nullptr)
+__device__ __forceinline__ int walk_hits(const RayTree& tree, const float4* __restrict__ sorted, int n, const Ray& r,
+                                         bool live, float max_distance, float& best, int2* stack, int* list)
 {
     constexpr unsigned kAll = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, c = lane & (kRayLanes - 1);
     int who = kList ? 0 : -1;
     if (!live) best = -1.f;
     // a zero component would give 0 x inf on a box face
     auto inverse = [](float d) { return 1.f / (fabsf(d) < 1e-12f ? copysignf(1e-12f, d) : d); };
     const float ix = inverse(r.dx), iy = inverse(r.dy), iz = inverse(r.dz);
-    int sp = 0;
     if (lane == 0) stack[0] = make_int2((int)((unsigned)(tree.levels - 1) << 28), 0);
-    sp = 1;
+    int sp = 1;
     __syncwarp();
     while (sp > 0) {
         const int2 top = stack[--sp];
         __syncwarp();
-        const float far = __uint_as_float(__reduce_max_sync(kAll, __float_as_uint(fmaxf(best, 0.f))));
+        float far = fmaxf(best, __shfl_xor_sync(kAll, best, 8));
+        far = fmaxf(far, __shfl_xor_sync(kAll, far, 16));
         if (__int_as_float(top.y) > far) continue;
-        const int level = (int)((unsigned)top.x >> 28), first = kRayArity * (top.x & 0x0fffffff);
+        const int level = (int)((unsigned)top.x >> 28), child = kRayArity * (top.x & 0x0fffffff) + c;
         if (level == 0) {
+            float th = -1.f;
+            if (child < n) {
+                const float4 q = __ldg(sorted + child);
+                if (q.w > 0.f) th = ray_sphere(r, q) + 0.f;  // (no negative zero)
+            }
+            const bool hit = th >= 0.f && th <= max_distance && (kList ? th <= best : th < best);
+            if (kList) {
+                const unsigned hits = __ballot_sync(kAll, hit) & ray_mask();
+                const int at = who + __popc(hits & ((1u << lane) - 1u));
+                if (hit && at < kRayList) list[at] = child;
+                who += __popc(hits);
+                if (who > kRayList) best = -1.f;  // too many: no more of them
+            } else {
+                // a float that is not negative orders as its bits do
+                unsigned near = hit ? __float_as_uint(th) : 0xffffffffu;
 #pragma unroll
-            for (int c = 0; c < kRayArity; ++c) {
-                if (first + c >= n) break;
-                const float4 q = __ldg(sorted + first + c);
-                if (!(q.w > 0.f)) continue;
-                const float th = ray_sphere(r, q);
-                if (th >= 0.f && th <= max_distance && th < best) {
-                    if (kList) {
-                        if (who < kRayList)
-                            list[who] = first + c;
-                        else
-                            best = -1.f;
-                        ++who;
-                    } else {
-                        best = th;
-                        who = first + c;
-                    }
+                for (int o = 1; o < kRayLanes; o <<= 1) near = min(near, __shfl_xor_sync(kAll, near, o));
+                const unsigned first = __ballot_sync(kAll, hit && __float_as_uint(th) == near) & ray_mask();
+                if (first) {
+                    best = __uint_as_float(near);
+                    who = child - c + ((__ffs((int)first) - 1) & (kRayLanes - 1));
                 }
             }
             continue;
         }
-        unsigned key = 0xffffffffu;  // lane c < 8: child c's nearest entry over the warp's rays
-        const int children = min(kRayArity, tree.count[level - 1] - first);
-        for (int c = 0; c < children; ++c) {
-            const float4* node = tree.node(level - 1, first + c);
+        float entry = INFINITY;
+        if (child < tree.count[level - 1]) {
+            const float4* node = tree.node(level - 1, child);
             const float4 lo = __ldg(node), hi = __ldg(node + 1);
-            float entry = INFINITY;
             if (lo.x <= hi.x) {
                 // the farthest point of the box from the camera bounds the rounding of its spheres' tests
                 const float fx = fmaxf(fabsf(lo.x - r.ox), fabsf(hi.x - r.ox));
@@ -546,64 +601,81 @@ __device__ __forceinline__ int nearest_hit(const RayTree& tree, const float4* __
                 const float near = fmaxf(tn - w, 0.f);
                 if (tn <= tf && tf >= -2.f * w && near <= best) entry = near;
             }
-            const unsigned e = __reduce_min_sync(kAll, __float_as_uint(entry));
-            if (lane == c) key = e;
         }
-        const bool take = lane < children && key < 0x7f800000u;
-        const unsigned taken = __ballot_sync(kAll, take);
+        entry = fminf(entry, __shfl_xor_sync(kAll, entry, 8));
+        entry = fminf(entry, __shfl_xor_sync(kAll, entry, 16));
+        const bool take = entry < INFINITY;
+        const unsigned taken = __ballot_sync(kAll, take) & 0xffu;
         int rank = 0;  // farthest first, so that the nearest is popped next
-        for (int c = 0; c < children; ++c) {
-            const unsigned other = __shfl_sync(kAll, key, c);
-            if (((taken >> c) & 1u) && (other > key || (other == key && c > lane))) ++rank;
+#pragma unroll
+        for (int o = 1; o < kRayLanes; ++o) {
+            const float other = __shfl_xor_sync(kAll, entry, o);
+            rank += other < INFINITY && (other > entry || (other == entry && (c ^ o) > c));
         }
-        if (take) stack[sp + rank] = make_int2((int)(((unsigned)(level - 1) << 28) | (unsigned)(first + lane)), (int)key);
+        if (take && lane < kRayLanes)
+            stack[sp + rank] = make_int2((int)(((unsigned)(level - 1) << 28) | (unsigned)child), __float_as_int(entry));
         sp += __popc(taken);
         __syncwarp();
     }
     return who;
 }
 
-// The march of a ray whose computed hits are the spheres list[0 .. count), all
-// of them: which of them a taken sample's box holds decides the depth, and no
-// other candidate matters. False when a sphere's cell may be clamped.
+// The march of a ray whose computed hits up to `stop` are the spheres
+// list[0 .. count), all of them: up to there, which of them a taken sample's
+// box holds decides the depth, and no other candidate matters. A lane of the
+// ray looks after every eighth of them. False when a cell may be clamped.
 __device__ __noinline__ bool march_few(const GridDev& g, const float4* __restrict__ sorted, const int* list, int count,
                                        const Ray& r, float max_distance, float search_radius, float march_step,
-                                       int max_steps, float& best)
+                                       int max_steps, float stop, float& best)
 {
+    constexpr int kMine = kRayList / kRayLanes;
+    const unsigned lanes = ray_mask();
     // (the box's two cells of slack hold the roundings of coordinates this small)
-    if (!(fmaxf(fmaxf(fabsf(r.ox), fabsf(r.oy)), fabsf(r.oz)) * g.inv < 1e6f)) return false;
-    float hit[kRayList], cell[kRayList][3];
-    for (int i = 0; i < count; ++i) {
-        const float4 q = sorted[list[i]];
-        hit[i] = ray_sphere(r, q);
-        const float x[3] = {q.x, q.y, q.z};
-        for (int a = 0; a < 3; ++a) {
-            const float c = __fmul_rn(x[a], g.inv);
-            if (!(fabsf(c) < 1e6f)) return false;
-            cell[i][a] = (float)trunc_sat(c);
+    bool fits = fmaxf(fmaxf(fabsf(r.ox), fabsf(r.oy)), fabsf(r.oz)) * g.inv < 1e6f;
+    float hit[kMine], cell[kMine][3];
+    unsigned left = 0;  // spheres no sample has tested
+#pragma unroll
+    for (int i = 0; i < kMine; ++i) {
+        const int at = i * kRayLanes + (threadIdx.x & (kRayLanes - 1));
+        hit[i] = cell[i][0] = cell[i][1] = cell[i][2] = 0.f;
+        if (at < count) {
+            const float4 q = sorted[list[at]];
+            left |= 1u << i;
+            hit[i] = ray_sphere(r, q) + 0.f;  // (no negative zero)
+            const float x[3] = {q.x, q.y, q.z};
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const float c = __fmul_rn(x[a], g.inv);
+                fits &= fabsf(c) < 1e6f;
+                cell[i][a] = (float)trunc_sat(c);
+            }
         }
     }
+    if (!__all_sync(lanes, fits)) return false;
     const RayMoves mv(g, r, march_step, max_distance);
     const float half = 0.5f + search_radius * g.inv + 2.f;
-    unsigned left = (1u << count) - 1u;  // spheres no sample has tested
     int s = 0;
     float t = 0.f;
-    while (left && s < max_steps && t <= max_distance && t <= best) {
+    while (s < max_steps && t <= max_distance && t <= best && t <= stop && __any_sync(lanes, left != 0u)) {
         int far = 1 << 30;
         const float p[3] = {fmaf(r.dx, t, r.ox), fmaf(r.dy, t, r.oy), fmaf(r.dz, t, r.oz)};
-        for (int i = 0; i < count; ++i) {
-            if (!((left >> i) & 1u)) continue;
+#pragma unroll
+        for (int i = 0; i < kMine; ++i) {
             int f = 0;
+#pragma unroll
             for (int a = 0; a < 3; ++a)
                 f = max(f, far_samples(p[a], g.inv, cell[i][a] + 0.5f, half, mv.dim[a], mv.move[a]));
-            far = min(far, f);
+            if ((left >> i) & 1u) far = min(far, f);
         }
+        far = __reduce_min_sync(lanes, far);
         if (far == 0) {
             int xl, xh, yl, yh, zl, zh;
             box_axis(__fadd_rn(r.ox, __fmul_rn(r.dx, t)), search_radius, g.inv, g.dx, xl, xh);
             box_axis(__fadd_rn(r.oy, __fmul_rn(r.dy, t)), search_radius, g.inv, g.dy, yl, yh);
             box_axis(__fadd_rn(r.oz, __fmul_rn(r.dz, t)), search_radius, g.inv, g.dz, zl, zh);
-            for (int i = 0; i < count; ++i) {
+            float found = INFINITY;
+#pragma unroll
+            for (int i = 0; i < kMine; ++i) {
                 auto holds = [&](int lo, int hi, float c, int dim) {
                     const int pc = wrap_dim((unsigned)((int)c + (int)kOrigin), dim);
                     for (int v = lo; v <= hi; ++v)
@@ -613,22 +685,20 @@ __device__ __noinline__ bool march_few(const GridDev& g, const float4* __restric
                 if (((left >> i) & 1u) && holds(xl, xh, cell[i][0], g.dx) && holds(yl, yh, cell[i][1], g.dy) &&
                     holds(zl, zh, cell[i][2], g.dz)) {
                     left &= ~(1u << i);
-                    best = fminf(best, hit[i]);
+                    found = fminf(found, hit[i]);
                 }
             }
+            __syncwarp(lanes);
+            best = fminf(best, __uint_as_float(__reduce_min_sync(lanes, __float_as_uint(found))));
             far = 1;
         }
-        const float lim = fminf(max_distance, best);
-        do {
-            ++s;
-            t = __fadd_rn(t, march_step);
-        } while (--far > 0 && s < max_steps && t <= lim);
+        stride(t, s, far, fminf(fminf(max_distance, best), stop), march_step, max_steps);
     }
     return true;
 }
 
 // The samples with t <= th are all taken: does the box of one of the last of
-// them hold the cell of sphere q, hit at th?
+// them hold the cell of sphere q, hit at th? A lane of the ray takes a sample.
 __device__ __forceinline__ bool held_before(const GridDev& g, const Ray& r, float4 q, float th, float max_distance,
                                             float search_radius, float march_step, int max_steps)
 {
@@ -643,69 +713,36 @@ __device__ __forceinline__ bool held_before(const GridDev& g, const Ray& r, floa
     };
     int s = 0;
     float t = 0.f;
-    while (s < max_steps && t <= max_distance && t <= th) {
-        if (t + 4.f * march_step > th) {
-            int xl, xh, yl, yh, zl, zh;
-            box_axis(__fadd_rn(r.ox, __fmul_rn(r.dx, t)), search_radius, g.inv, g.dx, xl, xh);
-            box_axis(__fadd_rn(r.oy, __fmul_rn(r.dy, t)), search_radius, g.inv, g.dy, yl, yh);
-            box_axis(__fadd_rn(r.oz, __fmul_rn(r.dz, t)), search_radius, g.inv, g.dz, zl, zh);
-            if (holds(xl, xh, cx, g.dx) && holds(yl, yh, cy, g.dy) && holds(zl, zh, cz, g.dz)) return true;
-        }
+    const float lim = th - 6.f * march_step;
+    if (t <= lim) stride(t, s, max_steps, lim, march_step, max_steps);
+    for (int j = threadIdx.x & (kRayLanes - 1); j > 0; --j) {
         ++s;
         t = __fadd_rn(t, march_step);
     }
-    return false;
+    bool held = false;
+    if (s < max_steps && t <= max_distance && t <= th) {
+        int xl, xh, yl, yh, zl, zh;
+        box_axis(__fadd_rn(r.ox, __fmul_rn(r.dx, t)), search_radius, g.inv, g.dx, xl, xh);
+        box_axis(__fadd_rn(r.oy, __fmul_rn(r.dy, t)), search_radius, g.inv, g.dy, yl, yh);
+        box_axis(__fadd_rn(r.oz, __fmul_rn(r.dz, t)), search_radius, g.inv, g.dz, zl, zh);
+        held = holds(xl, xh, cx, g.dx) && holds(yl, yh, cy, g.dy) && holds(zl, zh, cz, g.dz);
+    }
+    return __any_sync(ray_mask(), held);
 }
 
-constexpr int kRayStack = kRayLevels * kRayArity;
-
-// a warp takes a tile of 8 x 4 pixels, a block one of 16 x 8
-__global__ void __launch_bounds__(128) k_raycast(const __grid_constant__ GridDev g, const float4* __restrict__ m,
-                                                 const float4* __restrict__ sorted, const __grid_constant__ RayTree tree,
-                                                 int n, const __grid_constant__ nsph_raycast_camera cam,
-                                                 float search_radius, float march_step, int max_steps,
-                                                 float* __restrict__ depth)
+// The march over the cells that can hold a hit up to nearest + window, with
+// wider windows until the depth is known. Returns whether there is one.
+__device__ __noinline__ bool march_windows(const GridDev& g, const float4* __restrict__ m, const Ray& r, float rmax,
+                                           float nearest, float window, float max_distance, float search_radius,
+                                           float march_step, int max_steps, float had, float& best)
 {
-    launch_entry();
-    __shared__ int2 stacks[4][kRayStack];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int px = blockIdx.x * 16 + (warp & 1) * 8 + (lane & 7);
-    const int py = blockIdx.y * 8 + (warp >> 1) * 4 + (lane >> 3);
-    const bool live = px < cam.width && py < cam.height;
-    const Ray r = ray_for_pixel(cam, min(px, cam.width - 1), min(py, cam.height - 1));
-    float* out = depth + (live ? (size_t)py * cam.width + px : 0);
-    const float had = live ? (*out < 0.f ? cam.max_distance : *out) : 0.f;
-    float best = had;
-    const int who = nearest_hit<false>(tree, sorted, n, r, live, cam.max_distance, best, stacks[warp]);
-    const float nearest = best, rmax = tree.node(tree.levels - 1, 0)->w;
-    float window = 4.f * (search_radius + march_step);
-    bool open = live && who >= 0;  // the depth is not known yet
-    if (open && held_before(g, r, sorted[who], nearest, cam.max_distance, search_radius, march_step, max_steps)) {
-        *out = nearest;
-        open = false;
-    }
-    // one window, then the ray's hits if they are few, then wider windows
-    for (int round = 0; __any_sync(0xffffffffu, open); ++round) {
-        if (round == 1) {
-            int list[kRayList];
-            best = had;
-            const int count = nearest_hit<true>(tree, sorted, n, r, open, cam.max_distance, best, stacks[warp], list);
-            if (open && count <= kRayList) {
-                best = had;
-                if (march_few(g, sorted, list, count, r, cam.max_distance, search_radius, march_step, max_steps, best)) {
-                    if (best < had) *out = best;
-                    open = false;
-                }
-            }
-            continue;
-        }
-        if (!open) continue;
+    for (;; window *= 4.f) {
         // centres of spheres hit in [nearest, until]: within `w` of the ray's
         // points at [nearest - w, until + w]
         const float until = nearest + window;
         const float w = 1.001f * reach(rmax, until + 2.f * rmax) + 1e-5f * until;
         RayRegion region;
-        region.all = !(until < cam.max_distance && max_steps < (1 << 24) && window * g.inv < 1e6f);
+        region.all = !(until < max_distance && max_steps < (1 << 24) && window * g.inv < 1e6f);
         const float o[3] = {r.ox, r.oy, r.oz}, d[3] = {r.dx, r.dy, r.dz};
         const int dims[3] = {g.dx, g.dy, g.dz};
 #pragma unroll
@@ -721,15 +758,61 @@ __global__ void __launch_bounds__(128) k_raycast(const __grid_constant__ GridDev
             region.all |= !fits;
         }
         best = had;
-        const bool hit = march(g, m, r, cam.max_distance, search_radius, march_step, max_steps, region,
+        const bool hit = march(g, m, r, max_distance, search_radius, march_step, max_steps, region,
                                region.all ? INFINITY : until, best);
         // a march that ended on a hit inside the window is the reference's
-        if (region.all || (hit && best <= until)) {
-            if (hit) *out = best;
-            open = false;
-        }
-        window *= 4.f;
+        if (region.all || (hit && best <= until)) return hit;
     }
+}
+
+// a warp takes a square of four pixels, a block one of kRayTile x kRayTile
+__global__ void __launch_bounds__(kRayThreads) k_raycast(
+    const __grid_constant__ GridDev g, const float4* __restrict__ m, const float4* __restrict__ sorted,
+    const __grid_constant__ RayTree tree, int n, const __grid_constant__ nsph_raycast_camera cam, int tiles_x,
+    float search_radius, float march_step, int max_steps, float* __restrict__ depth)
+{
+    launch_entry();
+    __shared__ int2 stacks[kRayThreads / 32][kRayStack];
+    __shared__ int lists[kRayThreads / 32][kRayRays][kRayList];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ray = lane / kRayLanes;
+    const int px = (int)(blockIdx.x % (unsigned)tiles_x) * kRayTile + (warp & 1) * 2 + (ray & 1);
+    const int py = (int)(blockIdx.x / (unsigned)tiles_x) * kRayTile + (warp >> 1) * 2 + (ray >> 1);
+    const bool live = px < cam.width && py < cam.height;
+    const Ray r = ray_for_pixel(cam, min(px, cam.width - 1), min(py, cam.height - 1));
+    float* out = depth + (live ? (size_t)py * cam.width + px : 0);
+    const float had = live ? (*out < 0.f ? cam.max_distance : *out) : 0.f;
+    float best = had;
+    const int who = walk_hits<false>(tree, sorted, n, r, live, cam.max_distance, best, stacks[warp], nullptr);
+    const float nearest = best;
+    float window = 4.f * (search_radius + march_step);
+    bool open = live && who >= 0, found = false;  // open: the depth is not known yet
+    if (open && held_before(g, r, sorted[who], nearest, cam.max_distance, search_radius, march_step, max_steps)) {
+        found = true;
+        open = false;
+    }
+    // then the ray's hits up to a distance, if they are few, else the march
+    for (; __any_sync(0xffffffffu, open); window *= 4.f) {
+        const bool all = !(nearest + window < fminf(had, cam.max_distance));
+        const float until = all ? fminf(had, cam.max_distance) : nearest + window;
+        float bound = until;
+        const int count = walk_hits<true>(tree, sorted, n, r, open, cam.max_distance, bound, stacks[warp],
+                                          lists[warp][ray]);
+        __syncwarp();
+        if (open) {
+            best = had;
+            if (count > kRayList || !march_few(g, sorted, lists[warp][ray], count, r, cam.max_distance, search_radius,
+                                               march_step, max_steps, all ? INFINITY : until, best)) {
+                const float rmax = tree.node(tree.levels - 1, 0)->w;
+                found = march_windows(g, m, r, rmax, nearest, window, cam.max_distance, search_radius, march_step,
+                                      max_steps, had, best);
+                open = false;
+            } else if (all || best <= until) {
+                found = best < had;
+                open = false;
+            }
+        }
+    }
+    if (found && (lane & (kRayLanes - 1)) == 0) *out = best;
 }
 
 __global__ void k_clamp_no_hits(float* __restrict__ depth, int count, float max_distance)
@@ -816,9 +899,9 @@ extern "C" int nsph_raycast_particles(nsph_grid* grid, const float* x, const flo
                                        tree, level));
         NSPH_LAUNCH_CHECK("k_ray_top");
     }
-    const dim3 blocks((c.width + 15) / 16, (c.height + 7) / 8);
-    NSPH_CUDA_TRY(launch_dependent(k_raycast, blocks, 128, 0, cs,
-                                   g.view(), m, sorted, tree, n, c, search_radius, march_step, max_steps, depth));
+    const int tiles_x = (c.width + kRayTile - 1) / kRayTile, tiles_y = (c.height + kRayTile - 1) / kRayTile;
+    NSPH_CUDA_TRY(launch_dependent(k_raycast, tiles_x * tiles_y, kRayThreads, 0, cs, g.view(), m, sorted, tree, n, c,
+                                   tiles_x, search_radius, march_step, max_steps, depth));
     NSPH_LAUNCH_CHECK("k_raycast");
     return NSPH_OK;
 }
