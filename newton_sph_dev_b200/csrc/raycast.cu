@@ -24,11 +24,11 @@
 // 2. Every sample with t <= M is taken (nothing stops the march before). So
 //    when the box of such a sample holds the nearest sphere's cell, the depth
 //    is M. Otherwise, and if 3 does not apply, the march is run, but only over
-//    the samples whose box overlaps (modulo the grid's dims) the cells that can hold a sphere hit
-//    before M + window: spheres hit later cannot stop the march inside the
-//    window, and those that can are tested at these samples only. A march
-//    that leaves the window without a hit is repeated with a wider one, in
-//    the end the reference's whole march.
+//    the samples whose box overlaps (modulo the grid's dims) the cells that can
+//    hold a sphere hit before M + window: spheres hit later cannot stop the
+//    march inside the window, and those that can are tested at these samples
+//    only. A march that leaves the window without a hit is repeated with a
+//    wider one, in the end the reference's whole march.
 // 3. A ray whose nearest hit is not decided so has its computed hits collected
 //    from the tree, up to a distance that grows until the depth is known. Up to
 //    kRayList of them, only these spheres' cells matter: march_few passes over
@@ -409,7 +409,8 @@ __device__ __forceinline__ void stride(float& t, int& s, int k, float lim, float
 // per-sample movement along the axes, in cells, and the grid's dims
 struct RayMoves {
     float move[3], dim[3];
-    __device__ __forceinline__ RayMoves(const GridDev& g, const Ray& r, float march_step, float max_distance);
+    __device__ __forceinline__ RayMoves(const GridDev& g, const Ray& r, float march_step, float max_distance,
+                                        int max_steps);
 };
 
 __device__ __forceinline__ int wrap_dim(unsigned v, int dim)
@@ -417,9 +418,12 @@ __device__ __forceinline__ int wrap_dim(unsigned v, int dim)
     return (int)((dim & (dim - 1)) == 0 ? v & (unsigned)(dim - 1) : v % (unsigned)dim);
 }
 
-__device__ __forceinline__ RayMoves::RayMoves(const GridDev& g, const Ray& r, float march_step, float max_distance)
+__device__ __forceinline__ RayMoves::RayMoves(const GridDev& g, const Ray& r, float march_step, float max_distance,
+                                              int max_steps)
 {
-    const float step = march_step + 1.2e-7f * fminf(max_distance, 1e30f);  // with the rounding of t
+    // the largest t (2^20 roundings of the sum stay below the factor), and a step with the rounding of t
+    const float last = fminf(fminf(max_distance, 1.1f * march_step * (float)max_steps), 1e30f);
+    const float step = march_step + 1.2e-7f * last;
     const float d[3] = {r.dx, r.dy, r.dz};
     const int dims[3] = {g.dx, g.dy, g.dz};
 #pragma unroll
@@ -447,7 +451,7 @@ __device__ __noinline__ bool march(const GridDev& g, const float4* __restrict__ 
     bool hit = false;
     // previous query box, empty at first (every cell then counts as new)
     int pxl = 0, pxh = -1, pyl = 0, pyh = -1, pzl = 0, pzh = -1;
-    const RayMoves mv(g, r, march_step, max_distance);
+    const RayMoves mv(g, r, march_step, max_distance, max_steps);
     int s = 0;
     float t = 0.f;
     while (s < max_steps && t <= max_distance && t <= best && t <= stop) {
@@ -652,7 +656,7 @@ __device__ __noinline__ bool march_few(const GridDev& g, const float4* __restric
         }
     }
     if (!__all_sync(lanes, fits)) return false;
-    const RayMoves mv(g, r, march_step, max_distance);
+    const RayMoves mv(g, r, march_step, max_distance, max_steps);
     const float half = 0.5f + search_radius * g.inv + 2.f;
     int s = 0;
     float t = 0.f;

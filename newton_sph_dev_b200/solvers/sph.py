@@ -370,7 +370,7 @@ class SolverSPH(SolverBase):
 
     # ---- adjoint ---------------------------------------------------------
     def enable_adjoint(self) -> None:
-        """Allocate the adjoint scratch (36 bytes per particle); called on
+        """Allocate the adjoint scratch (68 bytes per particle); called on
         demand by :meth:`step_backward`, outside graph capture."""
         if self.batched:
             raise ValueError("the adjoint supports single-world solvers only")
