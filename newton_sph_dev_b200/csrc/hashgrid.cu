@@ -330,7 +330,6 @@ __global__ void k_ranges(const int* __restrict__ cells, int n, int2* __restrict_
 // No kernel waits on another block. The result is identical to the stable
 // radix sort's.
 // --------------------------------------------------------------------------
-constexpr int kCcPoints = 4;     // points per thread of k_cc_count / k_cc_scatter
 constexpr int kCsThreads = 256;  // k_cc_scan_ranges
 constexpr int kCsPer = 32;       // cells per thread
 constexpr int kCsTile = kCsThreads * kCsPer;
@@ -342,32 +341,21 @@ __global__ void __launch_bounds__(256) k_cc_count(const float* __restrict__ poin
                                                   unsigned* __restrict__ status)
 {
     launch_entry();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int stride = gridDim.x * blockDim.x;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     // the previous build's cells: the first sorted entry of each clears its range
-    for (int k = t; k < prev_n; k += stride) {
+    for (int k = i; k < prev_n; k += gridDim.x * blockDim.x) {
         const int c = prev_cells[k];
         if (k == 0 || prev_cells[k - 1] != c) ranges[c] = make_int2(0, 0);
     }
     bool bad = false;
-    int c[kCcPoints];
-#pragma unroll
-    for (int u = 0; u < kCcPoints; ++u) {
-        const int i = t + u * stride;
-        c[u] = -1;
-        if (i < n) {
-            const float x = points[3 * (size_t)i + 0];
-            const float y = points[3 * (size_t)i + 1];
-            const float z = points[3 * (size_t)i + 2];
-            bad |= !(isfinite(x) && isfinite(y) && isfinite(z));
-            c[u] = point_cell(x, y, z, inv, dx, dy, dz);
-            cells[i] = c[u];
-        }
-    }
-#pragma unroll
-    for (int u = 0; u < kCcPoints; ++u) {
-        const int i = t + u * stride;
-        if (i < n) slots[i] = atomicAdd(count + c[u], 1);
+    if (i < n) {
+        const float x = points[3 * (size_t)i + 0];
+        const float y = points[3 * (size_t)i + 1];
+        const float z = points[3 * (size_t)i + 2];
+        bad = !(isfinite(x) && isfinite(y) && isfinite(z));
+        const int c = point_cell(x, y, z, inv, dx, dy, dz);
+        cells[i] = c;
+        slots[i] = atomicAdd(count + c, 1);
     }
     if (bad && status) atomicOr(status, (unsigned)NSPH_STATUS_NONFINITE_INPUT);
 }
@@ -476,27 +464,12 @@ __global__ void __launch_bounds__(256) k_cc_scatter(const int* __restrict__ cell
                                                     int* __restrict__ tmp_cells)
 {
     launch_entry();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int stride = gridDim.x * blockDim.x;
-    int c[kCcPoints], s[kCcPoints];
-#pragma unroll
-    for (int u = 0; u < kCcPoints; ++u) {
-        const int i = t + u * stride;
-        c[u] = i < n ? cells[i] : 0;
-        s[u] = i < n ? slots[i] : 0;
-    }
-#pragma unroll
-    for (int u = 0; u < kCcPoints; ++u) {
-        const int i = t + u * stride;
-        if (i < n) s[u] += ranges[c[u]].x;
-    }
-#pragma unroll
-    for (int u = 0; u < kCcPoints; ++u) {
-        const int i = t + u * stride;
-        if (i < n && in_bounds(s[u] >= 0 && s[u] < n)) {
-            tmp[s[u]] = i;
-            tmp_cells[s[u]] = c[u];
-        }
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int c = cells[i], at = ranges[c].x + slots[i];
+    if (in_bounds(at >= 0 && at < n)) {
+        tmp[at] = i;
+        tmp_cells[at] = c;
     }
 }
 
@@ -992,8 +965,10 @@ int count_build(Grid& g, const float* points, int n, float cell_inv, const Gathe
                 cudaStream_t stream, int& nl, int prev_n)
 {
     const int tiles = (int)((g.ncells + kCsTile - 1) / kCsTile);
-    const int per_block = 256 * kCcPoints;
-    const int blocks = (n + per_block - 1) / per_block;
+    // a point per thread: with four, 64k points left half of the SMs without a
+    // block (count kernel 11 us; 64k rollout with its gradient 3.9 -> 3.65 ms,
+    // step of 32,768 60 -> 55 us, of 1M the same)
+    const int blocks = (n + 255) / 256;
     NSPH_CUDA_TRY(launch_dependent(k_cc_count, blocks, 256, 0, stream,
                                    points, n, cell_inv, g.dx, g.dy, g.dz, g.cell_count, g.keys_a, g.vals_a, g.point_cells, prev_n, g.cell_ranges, status));
     NSPH_LAUNCH_CHECK("k_cc_count");
@@ -1006,7 +981,7 @@ int count_build(Grid& g, const float* points, int n, float cell_inv, const Gathe
     NSPH_CUDA_TRY(launch_dependent(k_cc_scatter, blocks, 256, 0, stream,
                                    g.keys_a, g.vals_a, g.cell_ranges, n, g.keys_b, g.vals_b));
     NSPH_LAUNCH_CHECK("k_cc_scatter");
-    NSPH_CUDA_TRY(launch_dependent(k_cc_rank, (n + 255) / 256, 256, 0, stream,
+    NSPH_CUDA_TRY(launch_dependent(k_cc_rank, blocks, 256, 0, stream,
                                    g.vals_b, g.cell_ranges, g.keys_b, n, g.cell_count, g.point_cells, g.point_ids, gather ? *gather : GatherArgs{}, gather != nullptr));
     NSPH_LAUNCH_CHECK("k_cc_rank");
     nl += 5;
