@@ -86,6 +86,11 @@ __global__ void k_contact_gather(const int* __restrict__ ids, int n, const float
 // piles) evaluates its candidates where it finds them.
 constexpr int kContactThreads = 128;
 constexpr int kContactSlots = 24;
+// resident blocks per SM: 48 registers instead of 64 (56 for the XPBD pass), some
+// 90 bytes of spills outside the candidate loop. Contact step of 1M particles
+// 232 -> 219 us, XPBD step of 262k 286 -> 281; 9 blocks 227 and 280, 12 blocks
+// (40 registers) 229 and 298.
+constexpr int kContactBlocks = 10;
 
 // Bound of the contact test: err <= c implies fl(d) <= reach, with err =
 // fl(fl(d - r_i) - r_j) three roundings of quantities no larger than d + r_i
@@ -201,7 +206,7 @@ __device__ __forceinline__ void for_each_near(const GridDev& g, const float4* __
     }
 }
 
-__global__ void __launch_bounds__(kContactThreads) k_contact_forces(GridDev g, int n, const float4* __restrict__ m0,
+__global__ void __launch_bounds__(kContactThreads, kContactBlocks) k_contact_forces(GridDev g, int n, const float4* __restrict__ m0,
                                                                     const float4* __restrict__ m1,
                                                                     const nsph_contact_params p,
                                                                     float* __restrict__ f_out)
@@ -291,7 +296,7 @@ __device__ __forceinline__ void contact_delta(const GridDev& g, const float4* __
 }
 
 // deltas[i] += delta * w1 * relaxation (one writer per particle: no atomics)
-__global__ void __launch_bounds__(kContactThreads) k_contact_deltas(GridDev g, int n, const float4* __restrict__ m0,
+__global__ void __launch_bounds__(kContactThreads, kContactBlocks) k_contact_deltas(GridDev g, int n, const float4* __restrict__ m0,
                                                                     const float4* __restrict__ m1, float k_mu,
                                                                     float k_cohesion, float max_radius, float dt,
                                                                     float relaxation, float* __restrict__ deltas)
@@ -344,7 +349,7 @@ __global__ void k_xpbd_gather(const int* __restrict__ ids, int n, const float* _
     x0[k] = make_float4(x_orig[3 * i], x_orig[3 * i + 1], x_orig[3 * i + 2], 0.f);
 }
 
-__global__ void __launch_bounds__(kContactThreads) k_xpbd_pass(GridDev g, int n, const XpbdPass p,
+__global__ void __launch_bounds__(kContactThreads, kContactBlocks) k_xpbd_pass(GridDev g, int n, const XpbdPass p,
                                                                const float* __restrict__ shape_deltas)
 {
     launch_entry();
