@@ -70,8 +70,9 @@ __global__ void k_contact_gather(const int* __restrict__ ids, int n, const float
     if (k >= n) return;
     const size_t i = (size_t)ids[k];
     const bool active = (flags[i] & NSPH_PARTICLE_ACTIVE) != 0;
-    m0[k] = make_float4(x[3 * i], x[3 * i + 1], x[3 * i + 2], active ? radius[i] : -INFINITY);
-    m1[k] = make_float4(v[3 * i], v[3 * i + 1], v[3 * i + 2], inv_mass ? inv_mass[i] : 0.f);
+    const Row3 xi = load_row(x + 3 * i), vi = load_row(v + 3 * i);
+    m0[k] = make_float4(xi.x, xi.y, xi.z, active ? radius[i] : -INFINITY);
+    m1[k] = make_float4(vi.x, vi.y, vi.z, inv_mass ? inv_mass[i] : 0.f);
 }
 
 // ---- candidates in two phases ----------------------------------------------------
@@ -240,9 +241,7 @@ __global__ void __launch_bounds__(kContactThreads, kContactBlocks) k_contact_for
         }
     });
     const size_t i = (size_t)g.ids[kk];
-    f_out[3 * i] = fx;
-    f_out[3 * i + 1] = fy;
-    f_out[3 * i + 2] = fz;
+    store_row(f_out + 3 * i, fx, fy, fz);
 }
 
 // the correction of solve_particle_particle_contacts (xpbd/kernels.py:225-289)
@@ -344,9 +343,10 @@ __global__ void k_xpbd_gather(const int* __restrict__ ids, int n, const float* _
     if (k >= n) return;
     const size_t i = (size_t)ids[k];
     const bool active = (flags[i] & NSPH_PARTICLE_ACTIVE) != 0;
-    m0[k] = make_float4(x[3 * i], x[3 * i + 1], x[3 * i + 2], active ? radius[i] : -INFINITY);
-    m1[k] = make_float4(v[3 * i], v[3 * i + 1], v[3 * i + 2], inv_mass[i]);
-    x0[k] = make_float4(x_orig[3 * i], x_orig[3 * i + 1], x_orig[3 * i + 2], 0.f);
+    const Row3 xi = load_row(x + 3 * i), vi = load_row(v + 3 * i), oi = load_row(x_orig + 3 * i);
+    m0[k] = make_float4(xi.x, xi.y, xi.z, active ? radius[i] : -INFINITY);
+    m1[k] = make_float4(vi.x, vi.y, vi.z, inv_mass[i]);
+    x0[k] = make_float4(oi.x, oi.y, oi.z, 0.f);
 }
 
 __global__ void __launch_bounds__(kContactThreads, kContactBlocks) k_xpbd_pass(GridDev g, int n, const XpbdPass p,
@@ -388,12 +388,8 @@ __global__ void __launch_bounds__(kContactThreads, kContactBlocks) k_xpbd_pass(G
     }
     p.n0[kk] = make_float4(x, y, z, a.w);
     p.n1[kk] = make_float4(vx, vy, vz, w1);
-    p.x_out[3 * i] = x;
-    p.x_out[3 * i + 1] = y;
-    p.x_out[3 * i + 2] = z;
-    p.v_out[3 * i] = vx;
-    p.v_out[3 * i + 1] = vy;
-    p.v_out[3 * i + 2] = vz;
+    store_row(p.x_out + 3 * i, x, y, z);
+    store_row(p.v_out + 3 * i, vx, vy, vz);
 }
 
 int check_grid(const nsph_grid* grid, int n)

@@ -46,12 +46,11 @@ __device__ __forceinline__ unsigned lanemask_lt()
     return m;
 }
 
-// the sorted mirrors of particle i at sorted position g
-__device__ __forceinline__ void gather_particle(const GatherArgs& gather, int p, int g)
+// the sorted mirrors of particle p
+__device__ __forceinline__ void mirrors_of(const GatherArgs& gather, int p, float4& xs, float4& vs)
 {
     const size_t i = (size_t)p;
-    const float x = gather.x[3 * i + 0], y = gather.x[3 * i + 1], z = gather.x[3 * i + 2];
-    const float vx = gather.v[3 * i + 0], vy = gather.v[3 * i + 1], vz = gather.v[3 * i + 2];
+    const Row3 x = load_row(gather.x + 3 * i), v = load_row(gather.v + 3 * i);
     const int fl = gather.flags[i];
     const bool active = (fl & NSPH_PARTICLE_ACTIVE) != 0;
     const float m = gather.mass[i];
@@ -59,8 +58,16 @@ __device__ __forceinline__ void gather_particle(const GatherArgs& gather, int p,
     int gw = gather.world ? gather.world[i] : 0;
     gw = gw < 0 ? 0 : (gw >= gather.world_count ? gather.world_count - 1 : gw);
     const int attr = (active ? kAttrActive : 0) | (w > 0.f ? kAttrDynamic : 0) | (gw << kAttrGravShift);
-    gather.xs[g] = make_float4(x, y, z, mirror_mass(m, active));
-    gather.vs[g] = make_float4(vx, vy, vz, __int_as_float(attr));
+    xs = make_float4(x.x, x.y, x.z, mirror_mass(m, active));
+    vs = make_float4(v.x, v.y, v.z, __int_as_float(attr));
+}
+
+__device__ __forceinline__ void gather_particle(const GatherArgs& gather, int p, int g)
+{
+    float4 xs, vs;
+    mirrors_of(gather, p, xs, vs);
+    gather.xs[g] = xs;
+    gather.vs[g] = vs;
 }
 
 // the cell of point idx, in its world's part of the table; sets bad for a
@@ -489,20 +496,7 @@ __global__ void __launch_bounds__(256) k_cc_rank(const int* __restrict__ tmp_cel
     const int c = tmp_cells[q];
     if (!in_bounds(i >= 0 && i < n)) return;
     float4 xs, vs;
-    if (do_gather) {  // the gathered loads go out before the rank loop
-        const size_t ii = (size_t)i;
-        const float x = gather.x[3 * ii + 0], y = gather.x[3 * ii + 1], z = gather.x[3 * ii + 2];
-        const float vx = gather.v[3 * ii + 0], vy = gather.v[3 * ii + 1], vz = gather.v[3 * ii + 2];
-        const int fl = gather.flags[ii];
-        const bool active = (fl & NSPH_PARTICLE_ACTIVE) != 0;
-        const float m = gather.mass[ii];
-        const float w = gather.inv_mass[ii];
-        int gw = gather.world ? gather.world[ii] : 0;
-        gw = gw < 0 ? 0 : (gw >= gather.world_count ? gather.world_count - 1 : gw);
-        const int attr = (active ? kAttrActive : 0) | (w > 0.f ? kAttrDynamic : 0) | (gw << kAttrGravShift);
-        xs = make_float4(x, y, z, mirror_mass(m, active));
-        vs = make_float4(vx, vy, vz, __int_as_float(attr));
-    }
+    if (do_gather) mirrors_of(gather, i, xs, vs);  // the gathered loads go out before the rank loop
     const int2 se = ranges[c];
     if (!in_bounds(se.x >= 0 && se.x <= q && q < se.y && se.y <= n)) return;
     int rank = 0;

@@ -117,6 +117,30 @@ cudaError_t launch_plain(void (*kernel)(P...), dim3 grid, dim3 block, size_t sme
     return cudaGetLastError();
 }
 
+// A row of three floats (any 4-byte aligned address) as one 8-byte access and
+// one 4-byte one. A scattered row costs the L1 a wavefront per access and line,
+// whatever its width. Two accesses instead of three: force pass of 1M particles
+// 151.6 -> 145.4 us, build 73.7 -> 70.2, contact step of 1M 219.6 -> 210.7, XPBD
+// step of 262k 281 -> 267.
+struct Row3 {
+    float x, y, z;
+};
+
+__device__ __forceinline__ Row3 load_row(const float* p)
+{
+    const bool odd = (reinterpret_cast<size_t>(p) & 4u) != 0;
+    const float2 pair = *reinterpret_cast<const float2*>(p + (odd ? 1 : 0));
+    const float one = p[odd ? 0 : 2];
+    return odd ? Row3{one, pair.x, pair.y} : Row3{pair.x, pair.y, one};
+}
+
+__device__ __forceinline__ void store_row(float* p, float x, float y, float z)
+{
+    const bool odd = (reinterpret_cast<size_t>(p) & 4u) != 0;
+    *reinterpret_cast<float2*>(p + (odd ? 1 : 0)) = odd ? make_float2(y, z) : make_float2(x, y);
+    p[odd ? 0 : 2] = odd ? x : z;
+}
+
 __device__ __forceinline__ void launch_entry()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -104,7 +104,8 @@ __global__ void __launch_bounds__(256) k_raycast_gather(const int* __restrict__ 
     unsigned b[6] = {0u, 0u, 0u, 0u, 0u, 0u};
     if (k < n) {
         const size_t i = (size_t)ids[k];
-        const float4 q = make_float4(x[3 * i], x[3 * i + 1], x[3 * i + 2], radius[i]);
+        const Row3 xi = load_row(x + 3 * i);
+        const float4 q = make_float4(xi.x, xi.y, xi.z, radius[i]);
         m[k] = q;
         if (in_reach(q, cam)) {
             b[0] = ordered(q.x);

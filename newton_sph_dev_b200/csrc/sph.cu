@@ -898,9 +898,7 @@ __device__ __forceinline__ void integrate_out(size_t i, float4 xi, float4 vi, in
     }
     const float ax = acc.ax, ay = acc.ay, az = acc.az;
     if (o.a_out) {
-        o.a_out[3 * i + 0] = ax;
-        o.a_out[3 * i + 1] = ay;
-        o.a_out[3 * i + 2] = az;
+        store_row(o.a_out + 3 * i, ax, ay, az);
     }
     float v1x = vi.x, v1y = vi.y, v1z = vi.z;
     const bool dynamic = (attr & kAttrDynamic) != 0;
@@ -909,9 +907,10 @@ __device__ __forceinline__ void integrate_out(size_t i, float4 xi, float4 vi, in
         float fx = 0.f, fy = 0.f, fz = 0.f;
         if (o.f_ext) {
             const float w = o.inv_mass[i];
-            fx = __fmul_rn(o.f_ext[3 * i + 0], w);
-            fy = __fmul_rn(o.f_ext[3 * i + 1], w);
-            fz = __fmul_rn(o.f_ext[3 * i + 2], w);
+            const Row3 f = load_row(o.f_ext + 3 * i);
+            fx = __fmul_rn(f.x, w);
+            fy = __fmul_rn(f.y, w);
+            fz = __fmul_rn(f.z, w);
         }
         const float gx = o.gravity[3 * gw + 0], gy = o.gravity[3 * gw + 1], gz = o.gravity[3 * gw + 2];
         // v1 = fma(eps, dv, fma((a + f w) + g, dt, v0))
@@ -938,12 +937,8 @@ __device__ __forceinline__ void integrate_out(size_t i, float4 xi, float4 vi, in
     if (o.status && !(isfinite(x1x) && isfinite(x1y) && isfinite(x1z) && isfinite(v1x) && isfinite(v1y) &&
                       isfinite(v1z)))
         atomicOr(o.status, (unsigned)NSPH_STATUS_NONFINITE_OUTPUT);
-    o.x_out[3 * i + 0] = x1x;
-    o.x_out[3 * i + 1] = x1y;
-    o.x_out[3 * i + 2] = x1z;
-    o.v_out[3 * i + 0] = v1x;
-    o.v_out[3 * i + 1] = v1y;
-    o.v_out[3 * i + 2] = v1z;
+    store_row(o.x_out + 3 * i, x1x, x1y, x1z);
+    store_row(o.v_out + 3 * i, v1x, v1y, v1z);
 }
 
 // ---- the density pass of a small scene: eight lanes per particle -----------------
@@ -1645,8 +1640,8 @@ __global__ void __launch_bounds__(kSphThreads, 2) k_adj_local(GridDev g, const f
         const float4 xi = xs[k], vi = vs[k];
         const int attr = __float_as_int(vi.w);
         const size_t i = (size_t)g.ids[k];
-        const float xb1[3] = {io.x_out_adj[3 * i], io.x_out_adj[3 * i + 1], io.x_out_adj[3 * i + 2]};
-        const float vb1[3] = {io.v_out_adj[3 * i], io.v_out_adj[3 * i + 1], io.v_out_adj[3 * i + 2]};
+        const Row3 xo = load_row(io.x_out_adj + 3 * i), vo = load_row(io.v_out_adj + 3 * i);
+        const float xb1[3] = {xo.x, xo.y, xo.z}, vb1[3] = {vo.x, vo.y, vo.z};
         float fb[3] = {0.f, 0.f, 0.f};
         float4 gk = make_float4(0.f, 0.f, 0.f, 0.f), dk = gk;
         if (!(attr & kAttrActive)) {
@@ -1802,9 +1797,8 @@ __global__ void __launch_bounds__(kSphThreads, 2) k_adj_pair(GridDev g, const fl
         }
         if (sub != 0 || kt >= n) continue;
         const float4 x0 = io.xv[2 * (size_t)k], v0 = io.xv[2 * (size_t)k + 1];
-        io.v_in_adj[3 * i + 0] = active ? v0.x + vb[0] : v0.x;
-        io.v_in_adj[3 * i + 1] = active ? v0.y + vb[1] : v0.y;
-        io.v_in_adj[3 * i + 2] = active ? v0.z + vb[2] : v0.z;
+        store_row(io.v_in_adj + 3 * i, active ? v0.x + vb[0] : v0.x, active ? v0.y + vb[1] : v0.y,
+                  active ? v0.z + vb[2] : v0.z);
         if (!active) {
             io.rho[k] = 0.f;
             continue;
@@ -1866,9 +1860,8 @@ __global__ void __launch_bounds__(kSphThreads, 3) k_adj_density(GridDev g, const
         if (sub != 0 || kt >= n) continue;
         const size_t i = (size_t)g.ids[k];
         const float4 x0 = xv[2 * (size_t)k];
-        x_in_adj[3 * i + 0] = active ? x0.x + xb[0] : x0.x;
-        x_in_adj[3 * i + 1] = active ? x0.y + xb[1] : x0.y;
-        x_in_adj[3 * i + 2] = active ? x0.z + xb[2] : x0.z;
+        store_row(x_in_adj + 3 * i, active ? x0.x + xb[0] : x0.x, active ? x0.y + xb[1] : x0.y,
+                  active ? x0.z + xb[2] : x0.z);
     }
 }
 
