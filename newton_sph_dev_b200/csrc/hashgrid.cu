@@ -517,10 +517,10 @@ __global__ void __launch_bounds__(256) k_cc_rank(const int* __restrict__ tmp_cel
 // counts, for each point, the points of smaller cells and those of its own:
 // the counts are the point's place in the stable order and its cell's range.
 // n^2 comparisons, but in one pass; such a build is bound by its launches (five
-// of the counting build, ten of the radix sort). Step of 2,197 particles on a
-// B200, alone: 44 us instead of 50; build phase of a step, with this build and
-// without: 12 and 18 us (counting) or 28 (radix) at 1,000 particles, 14 and 20
-// or 29 at 4,096; at 8,000 it loses (24 and 20). A bitonic sort in one block
+// of the counting build, ten of the radix sort). Whole step on
+// a B200, with this build and without: 23 us and 27 (counting) or 38 (radix) at
+// 1,000 particles, 25 and 28 or 39 at 2,197, 28 and 29.5 or 42 at 4,096; at
+// 8,000 it loses (build phase 24 us, counting 16). A bitonic sort in one block
 // took 46 us at 2,197.
 // --------------------------------------------------------------------------
 constexpr int kRankThreads = 256;
