@@ -77,7 +77,10 @@ __device__ __forceinline__ float unordered(unsigned u)
 // is within 3u d of the dot product and its square within 7u d^2, |o|^2 within
 // 3u d^2, |o|^2 - r^2 rounds by u d^2, the last difference keeps its sign, and
 // the direction's squared length is within 7u of 1: 18u d^2 in all (24u is
-// taken). The rounding of o moves the centre by u d, inside the last factor.
+// taken). The centre is the rounded difference o itself: the boxes are formed
+// from the same differences, and rounding is monotone. The box test's own
+// roundings (5u of the distance) lie inside the last factor where the radius is
+// the larger part, and between 18u and 24u (1.6e-4 d) where the distance is.
 __device__ __forceinline__ float reach(float r, float d) { return sqrtf(fmaf(1.4306e-6f * d, d, r * r)) * 1.0001f; }
 
 // whether sphere q can be hit within max_distance of the camera at all (its
@@ -595,9 +598,11 @@ __device__ __forceinline__ int walk_hits(const RayTree& tree, const float4* __re
                 const float fy = fmaxf(fabsf(lo.y - r.oy), fabsf(hi.y - r.oy));
                 const float fz = fmaxf(fabsf(lo.z - r.oz), fabsf(hi.z - r.oz));
                 const float w = reach(lo.w, sqrtf(fx * fx + fy * fy + fz * fz) * 1.0001f);
-                const float ax = (lo.x - w - r.ox) * ix, bx = (hi.x + w - r.ox) * ix;
-                const float ay = (lo.y - w - r.oy) * iy, by = (hi.y + w - r.oy) * iy;
-                const float az = (lo.z - w - r.oz) * iz, bz = (hi.z + w - r.oz) * iz;
+                // differences first: those of the sphere test, so no centre leaves its box, however coarse the
+                // coordinates; the radius then rounds by 1u of the distance, the slab's ends by 2u each
+                const float ax = (lo.x - r.ox - w) * ix, bx = (hi.x - r.ox + w) * ix;
+                const float ay = (lo.y - r.oy - w) * iy, by = (hi.y - r.oy + w) * iy;
+                const float az = (lo.z - r.oz - w) * iz, bz = (hi.z - r.oz + w) * iz;
                 const float tn = fmaxf(fmaxf(fminf(ax, bx), fminf(ay, by)), fminf(az, bz));
                 const float tf = fminf(fminf(fmaxf(ax, bx), fmaxf(ay, by)), fmaxf(az, bz));
                 // the ray's nearest point to a centre lies in the inflated
