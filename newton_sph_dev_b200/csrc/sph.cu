@@ -407,10 +407,11 @@ __device__ __noinline__ int scan_general(const GridDev* g, const float4* xs, con
 // against all 32 particles at once, as the contraction
 //   r2 - T = |a|^2 - T + |b|^2 - 2 a.b
 // of fp16 coordinates relative to the group's origin in units of h
-// (mma.m16n8k8, fp16 accumulators: eight instructions per chunk; the norms
-// are split into fp16 hi + lo parts along K). The sign of r2 - T marks a
-// possible neighbour: T exceeds 1 by a bound on the rounding errors, so no
-// neighbour is missed. A chunk's marks (one 32-bit word per particle) wait in
+// (mma.m16n8k8, fp32 sums: eight instructions per chunk; the norms are split
+// into fp16 hi + lo parts along K). The sign of r2 - T marks a possible
+// neighbour: T exceeds 1 by a bound on the rounding errors, so no neighbour is
+// missed. (fp16 sums, of which only half precision is specified, would save
+// 8 of the 440 us of the 1M tank's step, 2 of 57 at 32,768 particles.) A chunk's marks (one 32-bit word per particle) wait in
 // shared memory; then each lane walks its own marks in order, repeats the
 // exact fp32 test of the definition, sums rho and appends to the list. Sets,
 // order and every rounding are therefore those of the general scan.
@@ -458,13 +459,25 @@ __device__ __forceinline__ float2 unpack_h2(unsigned u)
     return __half22float2(*reinterpret_cast<const __half2*>(&u));
 }
 
-// D = A (16 x 8) B (8 x 8), fp16: d0 = row lane / 4, d1 = row lane / 4 + 8,
-// columns 2 (lane % 4) and + 1
-__device__ __forceinline__ void mma_16x8x8(unsigned& d0, unsigned& d1, unsigned a0, unsigned a1, unsigned b)
+// D = A (16 x 8) B (8 x 8), fp16 operands and fp32 sums: d[0], d[1] = row
+// lane / 4, columns 2 (lane % 4) and + 1; d[2], d[3] = row lane / 4 + 8
+__device__ __forceinline__ void mma_16x8x8(float (&d)[4], unsigned a0, unsigned a1, unsigned b)
 {
-    asm("mma.sync.aligned.m16n8k8.row.col.f16.f16.f16.f16 {%0,%1}, {%2,%3}, {%4}, {%5,%5};"
-        : "=r"(d0), "=r"(d1)
-        : "r"(a0), "r"(a1), "r"(b), "r"(0u));
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(b), "f"(0.f));
+}
+
+// A byte per entry of d, in order: 0 where it is negative, 0xff above a
+// hundred denormals (as integers, saturated to eight bits). Two instructions
+// instead of three byte permutations: 1M tank's step 440 us against 447.
+__device__ __forceinline__ unsigned sign_bytes(const float (&d)[4])
+{
+    unsigned s;
+    asm("{.reg .b32 t;\n\tcvt.pack.sat.u8.s32.b32 t, %4, %3, 0;\n\tcvt.pack.sat.u8.s32.b32 %0, %2, %1, t;}"
+        : "=r"(s)
+        : "r"(__float_as_int(d[0])), "r"(__float_as_int(d[1])), "r"(__float_as_int(d[2])), "r"(__float_as_int(d[3])));
+    return s;
 }
 
 // Neighbour list and rho of the warp's particles k (one per lane; lanes with
@@ -509,6 +522,12 @@ __device__ __forceinline__ int tile_neighbors(const GridDev& g, const float4* __
     int nw = kTileWords;             // words free
     unsigned any = 0u;               // those with marks of this lane
     int total = 0;                   // this lane's waiting marks
+    // The lane's candidate of a chunk's half, last first, so that bit l of a
+    // ballot and of a word of marks is lane l's and the words are walked from the
+    // top bit down; and its column among the tiles: a word's byte b has the four
+    // tiles' columns b below those of columns b + 4.
+    const int cand = 31 - lane;
+    const int slot = 4 * ((lane >> 3) + (lane & 4)) + (lane & 3);
 
     int groups = 0;
     while (todo) {
@@ -592,9 +611,15 @@ __device__ __forceinline__ int tile_neighbors(const GridDev& g, const float4* __
                 __uint_as_float(__reduce_max_sync(kAll, __float_as_uint(fmaxf(fabsf(uy), fabsf(uz))))) + 1.01f;
             const float d = 9.765625e-4f * sqrtf(mx * mx + 2.f * myz * myz);  // 2 x 2^-11
             const float big = mx * mx + 2.f * myz * myz;
-            // (1 + d)^2, and 2^-16 of the largest partial sum for the
-            // products' sum and the splits
-            const float thr = (1.f + d) * (1.f + d) + 6.2e-5f * big;
+            // (1 + d)^2 of the rounded coordinates, and for the sum, of which the
+            // PTX specification promises products and additions in at least
+            // single precision, in any order, subnormal operands kept or not:
+            // per axis the product of a coordinate below 2^-14, at most 2^-13 of
+            // the other; the norms' parts below 2^-14, 2^-13 in all; eight
+            // additions of at most 5 big, 2^-23 each (4.8e-6 big); and the norms'
+            // splits and the fp32 roundings of coordinates, norms and the
+            // definition's test (under 1.2e-6 big)
+            const float thr = (1.f + d) * (1.f + d) + 1.3e-4f * (mx + 2.f * myz + 1.f) + 8e-6f * big;
             const float n2 = fmaf(fz, fz, fmaf(fxy.y, fxy.y, fxy.x * fxy.x)) - thr;
             const float n2h = unpack_h2(pack_h2(n2, 0.f)).x;
             const unsigned w0 = pack_h2(-2.f * fxy.x, -2.f * fxy.y), w1 = pack_h2(-2.f * fz, 1.f);
@@ -629,8 +654,8 @@ __device__ __forceinline__ int tile_neighbors(const GridDev& g, const float4* __
                 c0 = __shfl_sync(kAll, lo, r);
                 end = __shfl_sync(kAll, hi, r);
             }
-            q[0] = __ldg(xs + min(c0 + lane, end - 1));
-            q[1] = __ldg(xs + min(c0 + 32 + lane, end - 1));
+            q[0] = __ldg(xs + min(c0 + cand, end - 1));
+            q[1] = __ldg(xs + min(c0 + 32 + cand, end - 1));
         };
         q[0] = q[1] = make_float4(0.f, 0.f, 0.f, 0.f);
         more = true;
@@ -649,32 +674,28 @@ __device__ __forceinline__ int tile_neighbors(const GridDev& g, const float4* __
                     const float fz = unpack_h2(pack_h2(uz, 0.f)).x;
                     const float n2 = fmaf(fz, fz, fmaf(fxy.y, fxy.y, fxy.x * fxy.x));
                     const unsigned w1 = pack_h2(fz, n2);
-                    sm.frag[h][0][lane] = hxy;
-                    sm.frag[h][1][lane] = w1;
-                    sm.frag[h][2][lane] = pack_h2(n2 - unpack_h2(w1).y, 1.f);
+                    sm.frag[h][0][slot] = hxy;
+                    sm.frag[h][1][slot] = w1;
+                    sm.frag[h][2][slot] = pack_h2(n2 - unpack_h2(w1).y, 1.f);
                     // past the run's end and inactive (in no list): no mark
-                    counted[h] = __ballot_sync(kAll, 32 * h + lane < m && !mirror_inactive(q[h]));
+                    counted[h] = __ballot_sync(kAll, 32 * h + cand < m && !mirror_inactive(q[h]));
                 }
                 next_chunk();
                 __syncwarp();
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     if (h >= halves) break;
-                    // column j of tile i is candidate 4 j + i
+                    // column j of tile i is the candidate in slot 4 j + i
                     const uint4 b = *reinterpret_cast<const uint4*>(&sm.frag[h][lane & 3][lane & ~3]);
                     unsigned acc = 0u;
                     const unsigned bw[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
-                        unsigned d0, d1, d2, d3;
-                        mma_16x8x8(d0, d1, a0, a1, bw[i]);
-                        mma_16x8x8(d2, d3, a2, a3, bw[i]);
-                        // the four signs as bytes 0 or 0xff (sign-replicating selectors)
-                        unsigned s01, s23;
-                        asm("prmt.b32 %0, %1, %2, 0xfdb9;" : "=r"(s01) : "r"(d0), "r"(d1));
-                        asm("prmt.b32 %0, %1, %2, 0xfdb9;" : "=r"(s23) : "r"(d2), "r"(d3));
-                        acc |= s01 & (0x01010101u << i);
-                        acc |= s23 & (0x10101010u << i);
+                        float d01[4], d23[4];
+                        mma_16x8x8(d01, a0, a1, bw[i]);
+                        mma_16x8x8(d23, a2, a3, bw[i]);
+                        acc |= sign_bytes(d01) & (0x01010101u << i);
+                        acc |= sign_bytes(d23) & (0x10101010u << i);
                     }
                     sm.bits[h][lane] = acc;
                 }
@@ -686,14 +707,10 @@ __device__ __forceinline__ int tile_neighbors(const GridDev& g, const float4* __
                     const uint4 v = *reinterpret_cast<const uint4*>(&sm.bits[h][4 * (lane & 7)]);
                     const unsigned sel = (lane & 8) ? 0x7632u : 0x5410u;
                     const int sh = (lane & 16) ? 4 : 0;
-                    unsigned y0 = (__byte_perm(v.x, v.y, sel) >> sh) & 0x0f0f0f0fu;
-                    unsigned y1 = (__byte_perm(v.z, v.w, sel) >> sh) & 0x0f0f0f0fu;
-                    y0 |= y0 >> 4;
-                    y1 |= y1 >> 4;
-                    const unsigned marks = __byte_perm(y0, y1, 0x6420u) & (mine ? counted[h] : 0u);
-                    // kept so that the order is from the top bit down
+                    const unsigned y0 = __byte_perm(v.x, v.y, sel) >> sh, y1 = __byte_perm(v.z, v.w, sel) << (4 - sh);
+                    const unsigned marks = ~((y0 & 0x0f0f0f0fu) | (y1 & 0xf0f0f0f0u)) & (mine ? counted[h] : 0u);
                     --nw;
-                    sm.marks[nw][lane] = __brev(marks);
+                    sm.marks[nw][lane] = marks;
                     if (lane == 0) sm.first[nw] = at + 32 * h + 31;
                     any |= (marks != 0u ? 1u : 0u) << nw;
                     total += __popc(marks);
