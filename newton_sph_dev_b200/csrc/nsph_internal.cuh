@@ -342,7 +342,9 @@ struct Grid {
     int built = 0;
     float cell_width = 0.f;
     float cell_inv = 0.f;
-    // sort buffers (capacity each)
+    // one allocation of grid_reserve: the sort buffers (capacity each, rounded up
+    // to whole tree nodes of the raycast), the histograms, the raycast's bounds
+    char* block = nullptr;
     int* keys_a = nullptr;
     int* vals_a = nullptr;
     int* keys_b = nullptr;
@@ -350,6 +352,7 @@ struct Grid {
     int* point_cells = nullptr;  // sorted cell ids of the last build
     int* point_ids = nullptr;    // sorted original ids of the last build
     unsigned int* hist = nullptr;  // kRadix * ntiles(capacity)
+    unsigned int* bounds = nullptr;  // 6: of the spheres of a raycast
     // cell table (ncells entries of {start, end})
     int2* cell_ranges = nullptr;
     // counting build (single world, at most kCountMaxCells cells): per-cell
@@ -409,12 +412,7 @@ int grid_sort_keys(Grid& g, int n, int bits, cudaStream_t stream);
 struct nsph_grid {
     nsph::Grid g;
     // scratch of the contact and raycast kernels: 2 x mirror_cap sorted float4
-    // ((x, r), (v, inv_mass); or the spheres in grid and in tree order), then
-    // the raycast's bounds
+    // ((x, r), (v, inv_mass); or the spheres in grid and in tree order)
     float4* mirror = nullptr;
     int mirror_cap = 0;
 };
-
-namespace nsph {
-constexpr size_t mirror_bytes(int capacity) { return sizeof(float4) * 2 * (size_t)capacity + 256; }
-}  // namespace nsph

@@ -865,13 +865,13 @@ extern "C" int nsph_raycast_particles(nsph_grid* grid, const float* x, const flo
         cudaFree(grid->mirror);
         grid->mirror = nullptr;
         grid->mirror_cap = 0;
-        NSPH_CUDA_TRY(cudaMalloc(&grid->mirror, mirror_bytes(g.capacity)));
+        NSPH_CUDA_TRY(cudaMalloc(&grid->mirror, sizeof(float4) * 2 * (size_t)g.capacity));
         grid->mirror_cap = g.capacity;
     }
     cudaStream_t cs = (cudaStream_t)stream;
     float4* m = grid->mirror;
     float4* sorted = grid->mirror + grid->mirror_cap;
-    unsigned* bounds = reinterpret_cast<unsigned*>(grid->mirror + 2 * (size_t)grid->mirror_cap);
+    unsigned* bounds = g.bounds;
     NSPH_CUDA_TRY(cudaMemsetAsync(bounds, 0, 6 * sizeof(unsigned), cs));
     const int blocks_n = (n + 255) / 256;
     NSPH_CUDA_TRY(launch_dependent(k_raycast_gather, blocks_n, 256, 0, cs,

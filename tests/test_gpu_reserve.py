@@ -1,0 +1,31 @@
+"""What reservations take, and that a step asks for no memory that its solver
+could have had from the start."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda:0"
+
+
+def test_grid_reservation_stays_within_its_granules():
+    """2^20 points: six sort buffers of 4 MiB, half a MiB of histograms and a
+    mirror of 32 MiB, in granules of 2 MiB."""
+    from newton_sph_dev_b200 import HashGrid
+
+    HashGrid(16, 16, 16, device=DEV).reserve(1000)  # the kernels are loaded
+    grid = HashGrid(16, 16, 16, device=DEV)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    grid.reserve(1 << 20)
+    assert free - torch.cuda.mem_get_info()[0] <= 60 << 20
+    grid.build(torch.rand((1 << 20, 3), device=DEV), 0.05)
+    assert torch.equal(grid.point_ids.sort().values, torch.arange(1 << 20, dtype=torch.int32, device=DEV))
+    before = grid.point_ids.clone()
+    del grid
+    assert torch.cuda.mem_get_info()[0] > free - (16 << 20)
+    assert before.numel() == 1 << 20
