@@ -56,6 +56,11 @@ class SolverXPBD(SolverBase):
             self._qd_init = torch.empty_like(model.particle_q)
         if model.particle_count > 1 and model.particle_grid is not None:
             model.particle_grid.reserve(model.particle_count)
+            self._scratch = self._new_scratch()
+
+    def _new_scratch(self):
+        """Work memory of the iterations in one call (nsph_xpbd_solve)."""
+        return torch.empty((self.model.particle_count, 12), dtype=torch.float32, device=self.model.device)
 
     def _apply_particle_deltas(self, model: Model, state_in: State, state_out: State, dt: float):
         """One apply_particle_deltas, alternating the buffers as the reference does."""
@@ -79,14 +84,14 @@ class SolverXPBD(SolverBase):
                 and state_in.particle_qd.data_ptr() != state_out.particle_qd.data_ptr())
 
     def _step_one_call(self, state_in: State, state_out: State, contacts, dt: float) -> None:
-        model, n = self.model, self.model.particle_count
+        model = self.model
         if self.enable_restitution:
             self._q_init.copy_(state_in.particle_q)
             self._qd_init.copy_(state_in.particle_qd)
         self.integrate_particles(model, state_in, state_out, dt)
         model.particle_grid.build(state_out.particle_q, radius=model.particle_max_radius * 2.0 + model.particle_cohesion)
-        if self._scratch is None:
-            self._scratch = torch.empty((n, 12), dtype=torch.float32, device=model.device)
+        if self._scratch is None:  # the model's grid came after the solver
+            self._scratch = self._new_scratch()
         pc.solve_xpbd_iterations(model, contacts, self.iterations, state_in, state_out, self._deltas, self._scratch, dt,
                                  self.soft_contact_relaxation)
         final_qd = state_out.particle_qd

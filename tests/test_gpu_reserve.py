@@ -29,3 +29,25 @@ def test_grid_reservation_stays_within_its_granules():
     del grid
     assert torch.cuda.mem_get_info()[0] > free - (16 << 20)
     assert before.numel() == 1 << 20
+
+
+def test_first_xpbd_step_allocates_nothing():
+    import newton_sph_dev_b200 as nsph
+    from newton_sph_dev_b200.solvers import SolverXPBD
+
+    n = 3000
+    b = nsph.ModelBuilder()
+    b.add_particles(pos=(np.random.default_rng(1).random((n, 3)) * 0.2).astype(np.float32),
+                    vel=np.zeros((n, 3), np.float32), mass=np.full(n, 1.0), radius=np.full(n, 0.005))
+    b.add_ground_plane()
+    model = b.finalize(DEV)
+    solver = SolverXPBD(model, iterations=3)
+    s0, s1, contacts = model.state(), model.state(), model.contacts()
+    model.collide(s0, contacts)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    held = torch.cuda.memory_allocated()
+    solver.step(s0, s1, None, contacts, 1e-3)
+    torch.cuda.synchronize()
+    assert torch.cuda.memory_allocated() == held
+    assert torch.cuda.max_memory_allocated() == held
