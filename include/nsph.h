@@ -327,7 +327,7 @@ NSPH_API int nsph_sph_rollout_adjoint(nsph_sph* solver, const nsph_sph_params* p
  *   accumulate as in nsph_sph_step_adjoint. Afterwards the solver's grid
  *   describes the last step's input.
  * nsph_sph_reserve_segment: allocates the tape for segments of up to
- *   `steps` steps (380 bytes per particle of capacity plus 8 bytes per grid
+ *   `steps` steps (372 bytes per particle of capacity plus 8 bytes per grid
  *   cell, per step, and two states); nsph_sph_segment_adjoint reserves on
  *   demand, so call this first where the call is captured in a graph. */
 NSPH_API int nsph_sph_reserve_segment(nsph_sph* solver, int steps);

@@ -16,7 +16,9 @@
 // Layout in HBM (sorted by cell, written by the last radix pass):
 //   xs[k]  float4 (x, y, z, m_eff)   m_eff = -0 for inactive particles
 //   vs[k]  float4 (vx, vy, vz, attr) attr = active | dynamic<<1 | gravity<<2
-//   aux[k] float2 (m/rho, p/rho^2)   written by the density pass
+//   rec[k] 2 float4 (x, y, z, m_eff), (vx, vy, vz, m/rho), and
+//   pr2[k] float p/rho^2             what the force passes gather of a neighbour,
+//                                    written by the density pass
 //   rp[k]  float2 (rho, p)           written by the density pass
 // Outputs are scattered back to original particle order through point_ids.
 #include <algorithm>
@@ -185,7 +187,7 @@ __device__ __forceinline__ Neighbour load_neighbour(const float4* __restrict__ r
 
 template <bool Fast = false>
 __device__ __forceinline__ void density_finish(int k, float4 xi, float4 vi, float rho, const nsph_sph_params& p,
-                                               float2* __restrict__ aux, float2* __restrict__ rp, const ForceRec& fr,
+                                               float2* __restrict__ rp, const ForceRec& fr,
                                                unsigned* __restrict__ status)
 {
     const float m = xi.w;
@@ -203,7 +205,6 @@ __device__ __forceinline__ void density_finish(int k, float4 xi, float4 vi, floa
     } else if (status) {
         atomicOr(status, (unsigned)NSPH_STATUS_ZERO_DENSITY);
     }
-    aux[k] = make_float2(mor, pr2);
     rp[k] = make_float2(rho, pr);
     fr.rec[2 * (size_t)k] = xi;
     fr.rec[2 * (size_t)k + 1] = make_float4(vi.x, vi.y, vi.z, mor);
@@ -1130,7 +1131,7 @@ __device__ __forceinline__ int octet_neighbors(const GridDev& g, const float4* _
 template <bool Fast>
 __global__ void __launch_bounds__(kSphThreads, kDensityBlocks) k_density_list(
     const __grid_constant__ GridDev g, const float4* __restrict__ xs, const float4* __restrict__ vs, int n,
-    const __grid_constant__ nsph_sph_params p, float2* __restrict__ aux, float2* __restrict__ rp,
+    const __grid_constant__ nsph_sph_params p, float2* __restrict__ rp,
     int4* __restrict__ nbr, int* __restrict__ ncnt, const ForceRec fr, unsigned* __restrict__ status)
 {
     launch_entry();
@@ -1152,9 +1153,8 @@ __global__ void __launch_bounds__(kSphThreads, kDensityBlocks) k_density_list(
             if (cnt < 0) cnt = scan_general<Fast>(&g, xs, &p, xi, nbr, n, k, &rho);
             ncnt[k] = cnt;
             if (cnt > kNbrSlots && fr.overflow) atomicOr(fr.overflow, 1u);
-            density_finish<Fast>(k, xi, vs[k], rho, p, aux, rp, fr, status);
+            density_finish<Fast>(k, xi, vs[k], rho, p, rp, fr, status);
         } else if (live) {
-            aux[k] = make_float2(0.f, 0.f);
             rp[k] = make_float2(0.f, 0.f);
             fr.rec[2 * (size_t)k] = xi;  // (marked inactive)
             ncnt[k] = 0;
@@ -1165,7 +1165,7 @@ __global__ void __launch_bounds__(kSphThreads, kDensityBlocks) k_density_list(
 template <bool Fast>
 __global__ void __launch_bounds__(kOctetThreads) k_density_octet(
     const __grid_constant__ GridDev g, const float4* __restrict__ xs, const float4* __restrict__ vs, int n,
-    const __grid_constant__ nsph_sph_params p, float2* __restrict__ aux, float2* __restrict__ rp,
+    const __grid_constant__ nsph_sph_params p, float2* __restrict__ rp,
     int4* __restrict__ nbr, int* __restrict__ ncnt, const ForceRec fr, unsigned* __restrict__ status)
 {
     launch_entry();
@@ -1180,9 +1180,8 @@ __global__ void __launch_bounds__(kOctetThreads) k_density_octet(
         if (cnt < 0) cnt = scan_general<Fast>(&g, xs, &p, xi, nbr, n, k, &rho);
         ncnt[k] = cnt;
         if (cnt > kNbrSlots && fr.overflow) atomicOr(fr.overflow, 1u);
-        density_finish<Fast>(k, xi, vi, rho, p, aux, rp, fr, status);
+        density_finish<Fast>(k, xi, vi, rho, p, rp, fr, status);
     } else {
-        aux[k] = make_float2(0.f, 0.f);
         rp[k] = make_float2(0.f, 0.f);
         fr.rec[2 * (size_t)k] = xi;  // (marked inactive)
         ncnt[k] = 0;
@@ -1387,7 +1386,7 @@ __device__ __noinline__ int scan_general_world(const WorldCells* wc, const nsph_
 __global__ void __launch_bounds__(kSphThreads, kDensityBlocks) k_density_worlds(
     const WorldCells* __restrict__ wc, const nsph_sph_params* __restrict__ wp, const int2* __restrict__ ranges,
     const int* __restrict__ ids, const float4* __restrict__ xs, const float4* __restrict__ vs, int n,
-    float2* __restrict__ aux, float2* __restrict__ rp, int4* __restrict__ nbr, int* __restrict__ ncnt,
+    float2* __restrict__ rp, int4* __restrict__ nbr, int* __restrict__ ncnt,
     const ForceRec fr, unsigned* __restrict__ status)
 {
     launch_entry();
@@ -1411,9 +1410,8 @@ __global__ void __launch_bounds__(kSphThreads, kDensityBlocks) k_density_worlds(
         if (active) {
             if (cnt < 0) cnt = scan_general_world(wc, wp, ranges, ids, w, xs, xi, nbr, n, k, &rho);
             ncnt[k] = cnt;
-            density_finish(k, xi, vs[k], rho, p, aux, rp, fr, status);
+            density_finish(k, xi, vs[k], rho, p, rp, fr, status);
         } else if (live) {
-            aux[k] = make_float2(0.f, 0.f);
             rp[k] = make_float2(0.f, 0.f);
             fr.rec[2 * (size_t)k] = xi;  // (marked inactive)
             ncnt[k] = 0;
@@ -1424,7 +1422,7 @@ __global__ void __launch_bounds__(kSphThreads, kDensityBlocks) k_density_worlds(
 __global__ void __launch_bounds__(kOctetThreads) k_density_octet_worlds(
     const WorldCells* __restrict__ wc, const nsph_sph_params* __restrict__ wp, const int2* __restrict__ ranges,
     const int* __restrict__ ids, const float4* __restrict__ xs, const float4* __restrict__ vs, int n,
-    float2* __restrict__ aux, float2* __restrict__ rp, int4* __restrict__ nbr, int* __restrict__ ncnt,
+    float2* __restrict__ rp, int4* __restrict__ nbr, int* __restrict__ ncnt,
     const ForceRec fr, unsigned* __restrict__ status)
 {
     launch_entry();
@@ -1441,9 +1439,8 @@ __global__ void __launch_bounds__(kOctetThreads) k_density_octet_worlds(
     if (active) {
         if (cnt < 0) cnt = scan_general_world(wc, wp, ranges, ids, w, xs, xi, nbr, n, k, &rho);
         ncnt[k] = cnt;
-        density_finish(k, xi, vi, rho, p, aux, rp, fr, status);
+        density_finish(k, xi, vi, rho, p, rp, fr, status);
     } else {
-        aux[k] = make_float2(0.f, 0.f);
         rp[k] = make_float2(0.f, 0.f);
         fr.rec[2 * (size_t)k] = xi;  // (marked inactive)
         ncnt[k] = 0;
@@ -1754,7 +1751,7 @@ __device__ __forceinline__ float block_sum(float v)
 template <int kLanes>
 __global__ void __launch_bounds__(kSphThreads, 2) k_adj_pair(GridDev g, const float4* __restrict__ xs,
                                                              const float4* __restrict__ vs,
-                                                             const float2* __restrict__ aux, const ForceRec fr,
+                                                             const ForceRec fr,
                                                              const float2* __restrict__ rp, int n,
                                                              const __grid_constant__ nsph_sph_params p,
                                                              const int4* __restrict__ nbr,
@@ -1770,7 +1767,7 @@ __global__ void __launch_bounds__(kSphThreads, 2) k_adj_pair(GridDev g, const fl
         const float4 xi = xs[k], vi = vs[k];
         const size_t i = (size_t)g.ids[k];
         const bool active = kt < n && (__float_as_int(vi.w) & kAttrActive);
-        const float2 ak = aux[k];
+        const float2 ak = make_float2(fr.rec[2 * (size_t)k + 1].w, fr.pr2[k]);  // (m/rho, p/rho^2)
         const float4 gk = io.gd[2 * (size_t)k], dk = io.gd[2 * (size_t)k + 1];
         const float mk = xi.w;
         float pr2b = 0.f, morb = 0.f;
@@ -1981,7 +1978,7 @@ __device__ __forceinline__ void force_features_from_list(const GridDev& g, const
 // The 16 features of sorted particle k (all zero for an inactive one) and
 // its force sums; adds the particle's compression max(0, rho/rho0 - 1) and
 // 1 to (csum, ccount) when it is active.
-__device__ __forceinline__ void particle_features(const GridDev& g, const ForceRec& fr, const float2* __restrict__ aux,
+__device__ __forceinline__ void particle_features(const GridDev& g, const ForceRec& fr,
                                                   const float2* __restrict__ rp, const int4* __restrict__ nbr,
                                                   const int* __restrict__ ncnt, int n, int k, float4 xi, float4 vi,
                                                   const nsph_sph_params& p, float (&f)[kFeat], ForceAcc& acc,
@@ -1996,7 +1993,7 @@ __device__ __forceinline__ void particle_features(const GridDev& g, const ForceR
     const float c0sq = fmaxf(p.eos_b * (float)p.eos_gamma * p.inv_rho0, 1e-30f);
     const float inv_c0 = rsqrtf(c0sq);
     const float ascale = p.h / c0sq;
-    const float2 ak = aux[k];
+    const float2 ak = make_float2(fr.rec[2 * (size_t)k + 1].w, fr.pr2[k]);  // (m/rho, p/rho^2)
     FeatAcc fa{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     force_features_from_list(g, fr, nbr, ncnt[k], n, k, xi, vi, ak.y, p, acc, fa);
     const float2 rpk = rp[k];
@@ -2026,7 +2023,7 @@ __device__ __forceinline__ void particle_features(const GridDev& g, const ForceR
 // active count)
 __global__ void __launch_bounds__(kSphThreads, 4) k_force_features_list(GridDev g, const float4* __restrict__ xs,
                                                                         const float4* __restrict__ vs,
-                                                                        const ForceRec fr, const float2* __restrict__ aux,
+                                                                        const ForceRec fr,
                                                                         const float2* __restrict__ rp, int n,
                                                                         const __grid_constant__ nsph_sph_params p,
                                                                         const int4* __restrict__ nbr,
@@ -2041,7 +2038,7 @@ __global__ void __launch_bounds__(kSphThreads, 4) k_force_features_list(GridDev 
         const float4 xi = xs[k], vi = vs[k];
         float f[kFeat];
         ForceAcc acc;
-        particle_features(g, fr, aux, rp, nbr, ncnt, n, k, xi, vi, p, f, acc, csum, ccount);
+        particle_features(g, fr, rp, nbr, ncnt, n, k, xi, vi, p, f, acc, csum, ccount);
         float4* fo = reinterpret_cast<float4*>(feat + (size_t)k * kFeat);
 #pragma unroll
         for (int j = 0; j < kFeat; j += 4) fo[j / 4] = make_float4(f[j], f[j + 1], f[j + 2], f[j + 3]);
@@ -2094,7 +2091,7 @@ __global__ void __launch_bounds__(kMlpTile, 6) k_surrogate_fused(const float* __
                                                                  int wait_limit, GridDev g,
                                                                  const float4* __restrict__ xs,
                                                                  const float4* __restrict__ vs,
-                                                                 const ForceRec fr, const float2* __restrict__ aux,
+                                                                 const ForceRec fr,
                                                                  const float2* __restrict__ rp, int n,
                                                                  const __grid_constant__ nsph_sph_params p,
                                                                  const int4* __restrict__ nbr,
@@ -2116,7 +2113,7 @@ __global__ void __launch_bounds__(kMlpTile, 6) k_surrogate_fused(const float* __
         float f[kFeat];
         ForceAcc acc;
         if (k < n) {
-            particle_features(g, fr, aux, rp, nbr, ncnt, n, k, xi, vi, p, f, acc, csum, ccount);
+            particle_features(g, fr, rp, nbr, ncnt, n, k, xi, vi, p, f, acc, csum, ccount);
         } else {
             acc = ForceAcc{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -2161,7 +2158,7 @@ template <int kGroups>
 __global__ void __launch_bounds__(kGroups * kMlpTile, 6 / kGroups)
     k_surrogate_fused_groups(const float* __restrict__ model, float acc_scale, int wait_limit, GridDev g,
                              const float4* __restrict__ xs, const float4* __restrict__ vs,
-                             const ForceRec fr, const float2* __restrict__ aux, const float2* __restrict__ rp, int n,
+                             const ForceRec fr, const float2* __restrict__ rp, int n,
                              const __grid_constant__ nsph_sph_params p, const int4* __restrict__ nbr,
                              const int* __restrict__ ncnt, const StepOut o, float* __restrict__ cpart)
 {
@@ -2185,7 +2182,7 @@ __global__ void __launch_bounds__(kGroups * kMlpTile, 6 / kGroups)
         float f[kFeat];
         ForceAcc acc;
         if (k < n) {
-            particle_features(g, fr, aux, rp, nbr, ncnt, n, k, xi, vi, p, f, acc, csum, ccount);
+            particle_features(g, fr, rp, nbr, ncnt, n, k, xi, vi, p, f, acc, csum, ccount);
         } else {
             acc = ForceAcc{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -2297,7 +2294,6 @@ struct nsph_sph {
     int capacity = 0;
     float4* xs = nullptr;
     float4* vs = nullptr;
-    float2* aux = nullptr;
     float2* rp = nullptr;
     ForceRec fr{nullptr, nullptr, nullptr};  // the force pass's records
     int4* nbr = nullptr;       // kNbrGroups x capacity neighbour lists (group-major), every step form
@@ -2336,7 +2332,6 @@ struct nsph_sph {
 struct TapeStep {
     float4* xs;
     float4* vs;
-    float2* aux;
     float2* rp;
     ForceRec fr;
     int4* nbr;
@@ -2350,7 +2345,7 @@ static size_t tape_align(size_t b) { return (b + 255) & ~(size_t)255; }
 
 static size_t tape_slot_bytes(size_t c, long long ncells)
 {
-    return 2 * tape_align(sizeof(float4) * c) + 2 * tape_align(sizeof(float2) * c) +
+    return 2 * tape_align(sizeof(float4) * c) + tape_align(sizeof(float2) * c) +
            tape_align(sizeof(float4) * 2 * c) + tape_align(sizeof(float) * c) +
            tape_align(sizeof(int4) * kNbrGroups * c) + 2 * tape_align(sizeof(int) * c) +
            tape_align(sizeof(int2) * (size_t)ncells) + tape_align(sizeof(float4) * 2 * c);
@@ -2365,8 +2360,6 @@ static TapeStep tape_slot(const nsph_sph* s, int t)
     b += tape_align(sizeof(float4) * c);
     ts.vs = reinterpret_cast<float4*>(b);
     b += tape_align(sizeof(float4) * c);
-    ts.aux = reinterpret_cast<float2*>(b);
-    b += tape_align(sizeof(float2) * c);
     ts.rp = reinterpret_cast<float2*>(b);
     b += tape_align(sizeof(float2) * c);
     ts.fr.rec = reinterpret_cast<float4*>(b);
@@ -2453,18 +2446,18 @@ static cudaError_t launch_tiles(const nsph_sph* s, void (*kernel)(P...), int blo
 
 // the density pass of a single-world step into the given arrays
 static int density_enqueue(const nsph_sph* s, const GridDev& g, const nsph_sph_params* p, int n, bool fast,
-                           const float4* xs, const float4* vs, float2* aux, float2* rp, int4* nbr, int* ncnt,
+                           const float4* xs, const float4* vs, float2* rp, int4* nbr, int* ncnt,
                            const ForceRec& fr, cudaStream_t cs, int& launches)
 {
     if (octet_pass(s, n)) {
         const int blocks = (n + kOctetParticles - 1) / kOctetParticles;
         NSPH_CUDA_TRY(launch_plain(fast ? k_density_octet<true> : k_density_octet<false>, blocks, kOctetThreads,
-                                   0, cs, g, xs, vs, n, *p, aux, rp, nbr, ncnt, fr, s->status));
+                                   0, cs, g, xs, vs, n, *p, rp, nbr, ncnt, fr, s->status));
     } else {
         int blocks, threads;
         pass_launch(s, n, false, blocks, threads);
         NSPH_CUDA_TRY(launch_tiles(s, fast ? k_density_list<true> : k_density_list<false>, blocks, threads, cs, g, xs,
-                                   vs, n, *p, aux, rp, nbr, ncnt, fr, s->status));
+                                   vs, n, *p, rp, nbr, ncnt, fr, s->status));
     }
     ++launches;
     return NSPH_OK;
@@ -2496,7 +2489,6 @@ static void sph_free(nsph_sph* s)
         }
     cudaFree(s->xs);
     cudaFree(s->vs);
-    cudaFree(s->aux);
     cudaFree(s->rp);
     cudaFree(s->fr.rec);
     cudaFree(s->fr.pr2);
@@ -2603,7 +2595,6 @@ static int sph_create_common(nsph_sph* s, int device, int capacity)
         cudaError_t e = cudaMalloc(&s->xs, sizeof(float4) * (c + kXsPad));
         if (e == cudaSuccess) e = cudaMemset(s->xs + c, 0, sizeof(float4) * kXsPad);
         if (e == cudaSuccess) e = cudaMalloc(&s->vs, sizeof(float4) * c);
-        if (e == cudaSuccess) e = cudaMalloc(&s->aux, sizeof(float2) * c);
         if (e == cudaSuccess) e = cudaMalloc(&s->rp, sizeof(float2) * c);
         if (e == cudaSuccess) e = cudaMalloc(&s->fr.rec, sizeof(float4) * 2 * c);
         if (e == cudaSuccess) e = cudaMalloc(&s->fr.pr2, sizeof(float) * c);
@@ -2674,7 +2665,7 @@ static int step_enqueue(nsph_sph* s, const nsph_sph_params* p, int n, const floa
     if (n > 0) {
         const GridDev g = s->grid.view();
         int blocks, threads;
-        st = density_enqueue(s, g, p, n, s->fast != 0, s->xs, s->vs, s->aux, s->rp, s->nbr, s->ncnt, s->fr, cs, launches);
+        st = density_enqueue(s, g, p, n, s->fast != 0, s->xs, s->vs, s->rp, s->nbr, s->ncnt, s->fr, cs, launches);
         if (st != NSPH_OK) return st;
         if (s->ev[2]) NSPH_CUDA_TRY(record_mark(s->ev[2], cs));
         pass_launch(s, n, false, blocks, threads);
@@ -2819,12 +2810,12 @@ extern "C" int nsph_sph_step_worlds(nsph_sph* s, float dt, int n, const float* x
         if (octet_pass(s, n)) {
             NSPH_CUDA_TRY(launch_plain(k_density_octet_worlds, (n + kOctetParticles - 1) / kOctetParticles,
                                        kOctetThreads, 0, cs, s->grid.worlds, s->wparams, s->grid.cell_ranges,
-                                       s->grid.point_ids, s->xs, s->vs, n, s->aux, s->rp, s->nbr, s->ncnt, s->fr,
+                                       s->grid.point_ids, s->xs, s->vs, n, s->rp, s->nbr, s->ncnt, s->fr,
                                        s->status));
         } else {
             pass_launch(s, n, true, blocks, threads);
             NSPH_CUDA_TRY(launch_tiles(s, k_density_worlds, blocks, threads, cs, s->grid.worlds, s->wparams,
-                                       s->grid.cell_ranges, s->grid.point_ids, s->xs, s->vs, n, s->aux, s->rp, s->nbr,
+                                       s->grid.cell_ranges, s->grid.point_ids, s->xs, s->vs, n, s->rp, s->nbr,
                                        s->ncnt, s->fr, s->status));
         }
         ++launches;
@@ -3015,10 +3006,10 @@ static int adjoint_kernels(nsph_sph* s, const nsph_sph_params* p, int n, const G
     const int pair_threads = quad ? kSphThreads : threads;
     if (quad)
         NSPH_CUDA_TRY(launch_dependent(k_adj_pair<4>, pair_blocks, pair_threads, 0, cs,
-                                       g, ts.xs, ts.vs, ts.aux, ts.fr, ts.rp, n, *p, ts.nbr, ts.ncnt, io));
+                                       g, ts.xs, ts.vs, ts.fr, ts.rp, n, *p, ts.nbr, ts.ncnt, io));
     else
         NSPH_CUDA_TRY(launch_dependent(k_adj_pair<1>, pair_blocks, pair_threads, 0, cs,
-                                       g, ts.xs, ts.vs, ts.aux, ts.fr, ts.rp, n, *p, ts.nbr, ts.ncnt, io));
+                                       g, ts.xs, ts.vs, ts.fr, ts.rp, n, *p, ts.nbr, ts.ncnt, io));
     NSPH_LAUNCH_CHECK("k_adj_pair");
     if (mark && s->eva[4]) NSPH_CUDA_TRY(record_mark(s->eva[4], cs));
     if (quad)
@@ -3053,12 +3044,12 @@ static int adjoint_enqueue(nsph_sph* s, const nsph_sph_params* p, int n, const f
     if (s->eva[1]) NSPH_CUDA_TRY(record_mark(s->eva[1], cs));
     if (n > 0) {
         const GridDev g = s->grid.view();
-        st = density_enqueue(s, g, p, n, false, s->xs, s->vs, s->aux, s->rp, s->nbr, s->ncnt, s->fr, cs, launches);
+        st = density_enqueue(s, g, p, n, false, s->xs, s->vs, s->rp, s->nbr, s->ncnt, s->fr, cs, launches);
         if (st != NSPH_OK) return st;
         if (s->eva[2]) NSPH_CUDA_TRY(record_mark(s->eva[2], cs));
         const AdjIO io{x_out_adj, v_out_adj, rho_out_adj, x_in_adj, v_in_adj, f_ext_adj, f_ext, inv_mass, gravity,
                        s->adj_gd, s->adj_xv, s->adj_rho, s->adj_bpart};
-        const TapeStep ts{s->xs, s->vs, s->aux, s->rp, s->fr, s->nbr, s->ncnt, nullptr, nullptr, nullptr};
+        const TapeStep ts{s->xs, s->vs, s->rp, s->fr, s->nbr, s->ncnt, nullptr, nullptr, nullptr};
         st = adjoint_kernels(s, p, n, g, ts, io, eos_b_adj, cs, launches, true);
         if (st != NSPH_OK) return st;
     } else {
@@ -3212,7 +3203,7 @@ extern "C" int nsph_sph_segment_adjoint(nsph_sph* s, const nsph_sph_params* p, i
         st = grid_build(s->grid, xi, n, p->cell_width, p->cell_inv, &ga, s->status, cs, &launches);
         if (st != NSPH_OK) return st;
         const GridDev g = s->grid.view();
-        st = density_enqueue(s, g, p, n, false, ts.xs, ts.vs, ts.aux, ts.rp, ts.nbr, ts.ncnt, ts.fr, cs, launches);
+        st = density_enqueue(s, g, p, n, false, ts.xs, ts.vs, ts.rp, ts.nbr, ts.ncnt, ts.fr, cs, launches);
         if (st != NSPH_OK) return st;
         float* xo = tape_state(s, (t + 1) & 1);
         float* vo = xo + len;
@@ -3389,13 +3380,13 @@ static int features_enqueue(nsph_sph* s, const nsph_sph_params* p, int n, const 
     if (n > 0) {
         const GridDev g = s->grid.view();
         int threads;
-        st = density_enqueue(s, g, p, n, false, s->xs, s->vs, s->aux, s->rp, s->nbr, s->ncnt, s->fr, cs, launches);
+        st = density_enqueue(s, g, p, n, false, s->xs, s->vs, s->rp, s->nbr, s->ncnt, s->fr, cs, launches);
         if (st != NSPH_OK) return st;
         if (mark && s->eva[2]) NSPH_CUDA_TRY(record_mark(s->eva[2], cs));
         pass_launch(s, n, false, blocks, threads);
         if (features) {
             NSPH_CUDA_TRY(launch_plain(k_force_features_list, blocks, threads, 0, cs,
-                                           g, s->xs, s->vs, s->fr, s->aux, s->rp, n, *p, s->nbr, s->ncnt, s->sfeat, s->sacc, s->cpart));
+                                           g, s->xs, s->vs, s->fr, s->rp, n, *p, s->nbr, s->ncnt, s->sfeat, s->sacc, s->cpart));
             NSPH_LAUNCH_CHECK("k_force_features_list");
             ++launches;
         }
@@ -3478,12 +3469,12 @@ extern "C" int nsph_sph_step_surrogate(nsph_sph* s, const nsph_sph_params* p, co
         if (s->surr_groups == 2) {
             grid = std::min((tiles + 1) / 2, std::max(1, s->surr_ctas));
             NSPH_CUDA_TRY(launch_plain(k_surrogate_fused_groups<2>, grid, 2 * kMlpTile, sizeof(MlpFwdGroupSmem<2>), cs,
-                                           model, acc_scale, wait_limit, s->grid.view(), s->xs, s->vs, s->fr, s->aux, s->rp, n, *p, s->nbr, s->ncnt, o, s->cpart));
+                                           model, acc_scale, wait_limit, s->grid.view(), s->xs, s->vs, s->fr, s->rp, n, *p, s->nbr, s->ncnt, o, s->cpart));
             NSPH_LAUNCH_CHECK("k_surrogate_fused_groups");
         } else {
             grid = std::min(tiles, std::max(1, s->surr_ctas));
             NSPH_CUDA_TRY(launch_plain(k_surrogate_fused, grid, kMlpTile, sizeof(MlpFwdSmem), cs,
-                                           model, acc_scale, wait_limit, s->grid.view(), s->xs, s->vs, s->fr, s->aux, s->rp, n, *p, s->nbr, s->ncnt, o, s->cpart));
+                                           model, acc_scale, wait_limit, s->grid.view(), s->xs, s->vs, s->fr, s->rp, n, *p, s->nbr, s->ncnt, o, s->cpart));
             NSPH_LAUNCH_CHECK("k_surrogate_fused");
         }
         if (s->eva[3]) NSPH_CUDA_TRY(record_mark(s->eva[3], cs));

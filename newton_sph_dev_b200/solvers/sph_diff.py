@@ -139,7 +139,7 @@ def sph_rollout(solver: SolverSPH, x0: torch.Tensor, v0: torch.Tensor, steps: in
     The backward pass costs one extra forward step per step (the segment
     recompute, whose grid build, density pass and force sums the adjoint
     step then reuses) plus the adjoint step, and holds steps /
-    checkpoint_every checkpoints plus one segment's tape (380 bytes per
+    checkpoint_every checkpoints plus one segment's tape (372 bytes per
     particle and 8 per grid cell, per step).
 
     Returns:

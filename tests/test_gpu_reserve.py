@@ -47,3 +47,25 @@ def test_first_xpbd_step_allocates_nothing():
     torch.cuda.synchronize()
     assert torch.cuda.memory_allocated() == held
     assert torch.cuda.max_memory_allocated() == held
+
+
+def test_segment_tape_takes_what_it_says():
+    """372 bytes per particle and 8 per cell, per step (64 steps of 16,384
+    particles on 16^3 cells: 8 bytes more each would be 8 MiB)."""
+    import newton_sph_dev_b200 as nsph
+    from newton_sph_dev_b200.solvers import SolverSPH
+
+    n, steps = 16384, 64
+    b = nsph.ModelBuilder()
+    b.add_particles(pos=(np.random.default_rng(1).random((n, 3)) * 0.3).astype(np.float32),
+                    vel=np.zeros((n, 3), np.float32), mass=np.full(n, 1e-3))
+    model = b.finalize(DEV)
+    solver = SolverSPH(model, SolverSPH.Config(smoothing_length=0.02, grid_dims=(16, 16, 16)))
+    solver.enable_adjoint()
+    solver.reserve_segment(1)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    solver.reserve_segment(steps)
+    first = (372 * n + 8 * 16**3) + 48 * n  # the tape of one step, given back
+    took = free - torch.cuda.mem_get_info()[0]
+    assert took <= steps * (372 * n + 8 * 16**3) + 48 * n - first + (6 << 20)
