@@ -81,16 +81,21 @@ __device__ __forceinline__ float unordered(unsigned u)
 // from the same differences, and rounding is monotone. The box test's own
 // roundings (5u of the distance) lie inside the last factor where the radius is
 // the larger part, and between 18u and 24u (1.6e-4 d) where the distance is.
-__device__ __forceinline__ float reach(float r, float d) { return sqrtf(fmaf(1.4306e-6f * d, d, r * r)) * 1.0001f; }
+// (1e-43: 71 denormals, for what the products round by below the normal range.)
+__device__ __forceinline__ float reach(float r, float d)
+{
+    return sqrtf(fmaf(1.4306e-6f * d, d, fmaf(r, r, 1e-43f))) * 1.0001f;
+}
 
-// whether sphere q can be hit within max_distance of the camera at all (its
-// coordinates and radius finite, the radius positive)
+// Whether sphere q can be hit within max_distance of the camera at all: not
+// without a positive, finite radius, nor where the square of the distance
+// overflows (the test's discriminant is then no number, or its root infinite).
 __device__ __forceinline__ bool in_reach(float4 q, const nsph_raycast_camera& c)
 {
-    if (!(q.w > 0.f && isfinite(q.w) && fabsf(q.x) < 1e18f && fabsf(q.y) < 1e18f && fabsf(q.z) < 1e18f)) return false;
     const float ox = q.x - c.position[0], oy = q.y - c.position[1], oz = q.z - c.position[2];
-    const float d = sqrtf(ox * ox + oy * oy + oz * oz);
-    return !(d * 0.99999f - reach(q.w, d) > c.max_distance);
+    const float d2 = dot3(ox, oy, oz, ox, oy, oz);
+    if (!(q.w > 0.f && isfinite(q.w) && isfinite(d2))) return false;
+    return !(sqrtf(d2) * 0.99999f - reach(q.w, sqrtf(d2)) > c.max_distance);
 }
 
 // sorted mirror (x, y, z, radius) of the grid's points, and the bounds of the

@@ -63,3 +63,23 @@ def test_block_far_from_the_origin(oracle_mod, offset):
     far = 3 * size
     hits = _equal(oracle_mod, x, r, pos, (1.1, 0.1, -0.2), 0.9, sr, 0.4 * sr, far, int(far / (0.4 * sr)) + 2)
     assert hits.sum() > 100 and not hits.all()
+
+
+@pytest.mark.parametrize("power", [62, 40, -40, -62, -70])
+@pytest.mark.parametrize("name", ["inside", "overlap", "long_step", "truncated", "axis", "one"])
+def test_scales(oracle_mod, name, power):
+    """The same scenes in units in which distances are 10^18 and more, or their
+    squares are denormal."""
+    from newton_sph_dev_b200.sensors import march_steps
+    from test_gpu_raycast_tree import CASES
+
+    x, radius, pos, direction, fov, dims, sr, step, far, steps = CASES[name]()
+    scale = 2.0**power
+    sr = 1.0001 * radius
+    if not steps:
+        steps = march_steps(far, step * sr)[0]
+    x = (x.astype(np.float64) * scale).astype(np.float32)
+    r = np.full(len(x), radius * scale, np.float32)
+    hits = _equal(oracle_mod, x, r, tuple(c * scale for c in pos), direction, fov, sr * scale, step * sr * scale,
+                  far * scale, steps, dims=dims)
+    assert hits.any()
