@@ -679,8 +679,12 @@ NSPH_API int nsph_sph_set_arithmetic(nsph_sph* solver, int mode);
  * block (0 = default 256; else a multiple of 32 up to 256) and
  * `blocks_per_sm` (-1 = default: one thread per particle for a single world,
  * a persistent grid for batched worlds; 0 = one thread per particle; k > 0 =
- * a persistent grid of k blocks per SM striding over the particles). Results
- * do not depend on the shape; SolverSPH.autotune picks the fastest. */
+ * a persistent grid of k blocks per SM striding over the particles). With both
+ * at their defaults small scenes take kernels with several threads per particle
+ * (density up to 16,384 particles, single-world forces and adjoints up to
+ * 24,576); a shape set here turns these off. Results do not depend on the
+ * shape, but for the order of an adjoint's sums; SolverSPH.autotune picks the
+ * fastest. */
 NSPH_API int nsph_sph_set_launch(nsph_sph* solver, int threads, int blocks_per_sm);
 
 /* Number of kernels the last nsph_sph_step launched. */

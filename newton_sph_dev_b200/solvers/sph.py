@@ -726,7 +726,8 @@ class SolverSPH(SolverBase):
         return tuple(float(v) for v in ms)
 
     def set_launch(self, threads: int = 0, blocks_per_sm: int = -1) -> None:
-        """Launch shape of the density and force passes (see nsph_sph_set_launch)."""
+        """Launch shape of the density and force passes (see nsph_sph_set_launch);
+        no arguments: the default."""
         _lib.check(self._lib.nsph_sph_set_launch(self._handle, int(threads), int(blocks_per_sm)),
                    "SolverSPH.set_launch")
         self.launch = (int(threads), int(blocks_per_sm))
@@ -735,7 +736,8 @@ class SolverSPH(SolverBase):
         """Pick the fastest launch shape of the neighbour passes.
 
         Runs `repeats` steps state_in -> state_out per candidate (threads per
-        block, persistent blocks per SM; 0 = one thread per particle), timed
+        block, persistent blocks per SM; 0 = one thread per particle; (0, -1) =
+        the default, see nsph_sph_set_launch), timed
         on the device with the library's phase events, and keeps the fastest
         density + force time. Outside a CUDA graph capture only. Results do not
         depend on the launch shape.
@@ -745,7 +747,8 @@ class SolverSPH(SolverBase):
              "best": (threads, blocks_per_sm)}
         """
         if candidates is None:
-            candidates = [(t, b) for t in (128, 256) for b in (0, 2, 3, 4, 8)]
+            # the default first: the kernels of small scenes go with it, an explicit shape turns them off
+            candidates = [(0, -1)] + [(t, b) for t in (128, 256) for b in (0, 2, 3, 4, 8)]
         self.enable_phase_timing(True)
         results = {}
         for t, b in candidates:
