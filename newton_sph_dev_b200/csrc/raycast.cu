@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(256) k_ray_upper(const __grid_constant__ RayTr
     if (i < tree.count[level - 1] && (threadIdx.x & (kRayArity - 1)) == 0) store_box(tree.node(level, i / kRayArity), b);
 }
 
-// the levels from `first` up, in one block (the first has at most 256 x 8 children)
+// the levels from `first` up, in one block (the first has at most 4,096 children)
 __global__ void __launch_bounds__(1024) k_ray_top(const __grid_constant__ RayTree tree, int first)
 {
     launch_entry();
