@@ -203,7 +203,7 @@ __device__ __forceinline__ void query_bounds(float p, float r, float inv, int di
 // physical coordinate of virtual cell c (not clamped: c + 2^20 >= 0)
 __device__ __forceinline__ int wrap_cell(int c, int dim)
 {
-    const unsigned v = (unsigned)(c + (int)kOrigin);
+    const unsigned v = (unsigned)c + (unsigned)kOrigin;
     return (int)((dim & (dim - 1)) == 0 ? v & (unsigned)(dim - 1) : v % (unsigned)dim);
 }
 

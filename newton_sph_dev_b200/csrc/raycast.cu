@@ -422,11 +422,6 @@ struct RayMoves {
                                         int max_steps);
 };
 
-__device__ __forceinline__ int wrap_dim(unsigned v, int dim)
-{
-    return (int)((dim & (dim - 1)) == 0 ? v & (unsigned)(dim - 1) : v % (unsigned)dim);
-}
-
 __device__ __forceinline__ RayMoves::RayMoves(const GridDev& g, const Ray& r, float march_step, float max_distance,
                                               int max_steps)
 {
@@ -446,7 +441,7 @@ __device__ __forceinline__ RayMoves::RayMoves(const GridDev& g, const Ray& r, fl
 __device__ __forceinline__ bool axis_meets(const RayRegion& g, int a, int lo, int hi, int dim)
 {
     if ((long long)lo + kOrigin < 0 || g.span[a] + (hi - lo) + 2 > dim) return true;
-    const int p = wrap_dim((unsigned)(lo + (int)kOrigin), dim);
+    const int p = wrap_cell(lo, dim);
     const int d = p >= g.first[a] ? p - g.first[a] : p - g.first[a] + dim;  // from the region's first to lo
     return d <= g.span[a] || dim - d <= hi - lo;
 }
@@ -692,7 +687,7 @@ __device__ __noinline__ bool march_few(const GridDev& g, const float4* __restric
 #pragma unroll
             for (int i = 0; i < kMine; ++i) {
                 auto holds = [&](int lo, int hi, float c, int dim) {
-                    const int pc = wrap_dim((unsigned)((int)c + (int)kOrigin), dim);
+                    const int pc = wrap_cell((int)c, dim);
                     for (int v = lo; v <= hi; ++v)
                         if (phys_axis(v, dim) == pc) return true;
                     return false;
@@ -722,7 +717,7 @@ __device__ __forceinline__ bool held_before(const GridDev& g, const Ray& r, floa
               cz = phys_axis(trunc_sat(__fmul_rn(q.z, g.inv)), g.dz);
     auto holds = [](int lo, int hi, int c, int dim) {
         if ((long long)lo + kOrigin < 0) return false;  // clamped cells: left to the march
-        int d = c - wrap_dim((unsigned)(lo + (int)kOrigin), dim);
+        int d = c - wrap_cell(lo, dim);
         if (d < 0) d += dim;
         return d <= hi - lo;
     };
@@ -769,7 +764,7 @@ __device__ __noinline__ bool march_windows(const GridDev& g, const float4* __res
             region.span[a] = vhi - vlo;
             region.centre[a] = 0.5f * ((float)vlo + (float)vhi + 1.f);
             region.half[a] = 0.5f * (float)(vhi - vlo + 1) + search_radius * g.inv + 2.f;
-            region.first[a] = wrap_dim((unsigned)(vlo + (int)kOrigin), dims[a]);
+            region.first[a] = wrap_cell(vlo, dims[a]);
             region.all |= !fits;
         }
         best = had;

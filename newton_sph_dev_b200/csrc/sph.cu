@@ -331,11 +331,8 @@ __device__ __forceinline__ int group_item(const int4& gr, int u)
 // register (no per-item select, as a reader returning one item at a time
 // needs) and the visits' loads can issue together. kReadOnly: the list was
 // written by an earlier kernel (read-only path); otherwise it is read back by
-// the thread that wrote it (plain loads). kUnrolled = false keeps a rolled
-// loop over a group's items (one item per iteration, selected at run time):
-// the batched worlds' force pass spills more when unrolled (2.16 -> 2.38 ms
-// on worlds_4096).
-template <bool kReadOnly, bool kUnrolled = true, class F>
+// the thread that wrote it (plain loads).
+template <bool kReadOnly, class F>
 __device__ __forceinline__ void for_each_listed(const int4* __restrict__ nbr, int n, int k, int cnt, F&& visit)
 {
     in_bounds(cnt >= 0 && cnt <= kNbrSlots);
@@ -347,18 +344,12 @@ __device__ __forceinline__ void for_each_listed(const int4* __restrict__ nbr, in
         const int4 gr = cur;
         cur = nxt;
         if (t + 8 < cnt) nxt = load((t >> 2) + 2);
-        auto item = [&](int u) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
             if (t + u < cnt) {
                 const int j = group_item(gr, u);
                 visit(in_bounds(j >= 0 && j < n) ? j : 0);
             }
-        };
-        if constexpr (kUnrolled) {
-#pragma unroll
-            for (int u = 0; u < 4; ++u) item(u);
-        } else {
-#pragma unroll 1
-            for (int u = 0; u < 4; ++u) item(u);
         }
     }
 }
