@@ -402,8 +402,8 @@ __device__ __noinline__ int scan_general(const GridDev* g, const float4* xs, con
 // (mma.m16n8k8, fp32 sums: eight instructions per chunk; the norms are split
 // into fp16 hi + lo parts along K). The sign of r2 - T marks a possible
 // neighbour: T exceeds 1 by a bound on the rounding errors, so no neighbour is
-// missed. (fp16 sums, of which only half precision is specified, would save
-// 8 of the 440 us of the 1M tank's step, 2 of 57 at 32,768 particles.) A chunk's marks (one 32-bit word per particle) wait in
+// missed. (fp16 sums, of which only half precision is specified, would save 3 of
+// the 434 us of the 1M tank's step.) A chunk's marks (one 32-bit word per particle) wait in
 // shared memory; then each lane walks its own marks in order, repeats the
 // exact fp32 test of the definition, sums rho and appends to the list. Sets,
 // order and every rounding are therefore those of the general scan.
@@ -460,15 +460,15 @@ __device__ __forceinline__ void mma_16x8x8(float (&d)[4], unsigned a0, unsigned 
         : "r"(a0), "r"(a1), "r"(b), "f"(0.f));
 }
 
-// A byte per entry of d, in order: 0 where it is negative, 0xff above a
-// hundred denormals (as integers, saturated to eight bits). Two instructions
-// instead of three byte permutations: 1M tank's step 440 us against 447.
-__device__ __forceinline__ unsigned sign_bytes(const float (&d)[4])
+// c moved up by two bytes, below it the signs of hi and lo: 0 where negative, 0xff
+// above a hundred denormals (as integers, saturated to eight bits). Two of these
+// for four products instead of three byte permutations.
+__device__ __forceinline__ unsigned push_signs(unsigned c, float hi, float lo)
 {
     unsigned s;
-    asm("{.reg .b32 t;\n\tcvt.pack.sat.u8.s32.b32 t, %4, %3, 0;\n\tcvt.pack.sat.u8.s32.b32 %0, %2, %1, t;}"
+    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;"
         : "=r"(s)
-        : "r"(__float_as_int(d[0])), "r"(__float_as_int(d[1])), "r"(__float_as_int(d[2])), "r"(__float_as_int(d[3])));
+        : "r"(__float_as_int(hi)), "r"(__float_as_int(lo)), "r"(c));
     return s;
 }
 
@@ -515,11 +515,9 @@ __device__ __forceinline__ int tile_neighbors(const GridDev& g, const float4* __
     unsigned any = 0u;               // those with marks of this lane
     int total = 0;                   // this lane's waiting marks
     // The lane's candidate of a chunk's half, last first, so that bit l of a
-    // ballot and of a word of marks is lane l's and the words are walked from the
-    // top bit down; and its column among the tiles: a word's byte b has the four
-    // tiles' columns b below those of columns b + 4.
+    // ballot and of a word of marks is lane l's and words are walked from the top
+    // bit down.
     const int cand = 31 - lane;
-    const int slot = 4 * ((lane >> 3) + (lane & 4)) + (lane & 3);
 
     int groups = 0;
     while (todo) {
@@ -666,9 +664,9 @@ __device__ __forceinline__ int tile_neighbors(const GridDev& g, const float4* __
                     const float fz = unpack_h2(pack_h2(uz, 0.f)).x;
                     const float n2 = fmaf(fz, fz, fmaf(fxy.y, fxy.y, fxy.x * fxy.x));
                     const unsigned w1 = pack_h2(fz, n2);
-                    sm.frag[h][0][slot] = hxy;
-                    sm.frag[h][1][slot] = w1;
-                    sm.frag[h][2][slot] = pack_h2(n2 - unpack_h2(w1).y, 1.f);
+                    sm.frag[h][0][lane] = hxy;
+                    sm.frag[h][1][lane] = w1;
+                    sm.frag[h][2][lane] = pack_h2(n2 - unpack_h2(w1).y, 1.f);
                     // past the run's end and inactive (in no list): no mark
                     counted[h] = __ballot_sync(kAll, 32 * h + cand < m && !mirror_inactive(q[h]));
                 }
@@ -677,17 +675,20 @@ __device__ __forceinline__ int tile_neighbors(const GridDev& g, const float4* __
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     if (h >= halves) break;
-                    // column j of tile i is the candidate in slot 4 j + i
+                    // column j of tile i is the candidate of lane 4 j + i
                     const uint4 b = *reinterpret_cast<const uint4*>(&sm.frag[h][lane & 3][lane & ~3]);
-                    unsigned acc = 0u;
                     const unsigned bw[4] = {b.x, b.y, b.z, b.w};
+                    // bit 4 j + i of byte g: tile i, column 2 (lane % 4) + j, row lane / 4 + 8 g; 1 where not near
+                    unsigned acc = 0u;
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         float d01[4], d23[4];
                         mma_16x8x8(d01, a0, a1, bw[i]);
                         mma_16x8x8(d23, a2, a3, bw[i]);
-                        acc |= sign_bytes(d01) & (0x01010101u << i);
-                        acc |= sign_bytes(d23) & (0x10101010u << i);
+#pragma unroll
+                        for (int j = 0; j < 2; ++j)
+                            acc |= push_signs(push_signs(0u, d23[2 + j], d23[j]), d01[2 + j], d01[j]) &
+                                   (0x01010101u << (4 * j + i));
                     }
                     sm.bits[h][lane] = acc;
                 }
@@ -697,10 +698,9 @@ __device__ __forceinline__ int tile_neighbors(const GridDev& g, const float4* __
                     if (h >= halves) break;
                     // this lane's row from the four lanes that hold its columns
                     const uint4 v = *reinterpret_cast<const uint4*>(&sm.bits[h][4 * (lane & 7)]);
-                    const unsigned sel = (lane & 8) ? 0x7632u : 0x5410u;
-                    const int sh = (lane & 16) ? 4 : 0;
-                    const unsigned y0 = __byte_perm(v.x, v.y, sel) >> sh, y1 = __byte_perm(v.z, v.w, sel) << (4 - sh);
-                    const unsigned marks = ~((y0 & 0x0f0f0f0fu) | (y1 & 0xf0f0f0f0u)) & (mine ? counted[h] : 0u);
+                    const unsigned sel = 0x4040u + 0x1111u * (unsigned)(lane >> 3);
+                    const unsigned y0 = __byte_perm(v.x, v.y, sel), y1 = __byte_perm(v.z, v.w, sel);
+                    const unsigned marks = ~((y0 & 0xffffu) | (y1 & 0xffff0000u)) & (mine ? counted[h] : 0u);
                     --nw;
                     sm.marks[nw][lane] = marks;
                     if (lane == 0) sm.first[nw] = at + 32 * h + 31;
