@@ -356,6 +356,10 @@ NSPH_API int nsph_sph_segment_adjoint(nsph_sph* solver, const nsph_sph_params* p
  *   the nearer particle hit, if any.
  *   max_steps is at most NSPH_RAYCAST_MAX_STEPS (the reference's cap on the
  *   samples of one ray, sensor_raycast.py:28).
+ *   The call uses the grid's sort buffers. Calls for one grid may come from
+ *   several streams and host threads: each waits on its stream for the one
+ *   before. Captured calls are not ordered so: graphs that raycast one grid
+ *   must not run at the same time.
  * nsph_raycast_clamp_no_hits: depth[i] >= max_distance becomes -1. */
 #define NSPH_RAYCAST_MAX_STEPS (1 << 20)
 

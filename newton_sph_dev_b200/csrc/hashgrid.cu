@@ -1070,6 +1070,7 @@ extern "C" int nsph_grid_destroy(nsph_grid* grid)
     {
         DeviceGuard guard(grid->g.device);
         cudaFree(grid->mirror);
+        if (grid->raycast_done) cudaEventDestroy(grid->raycast_done);
     }
     grid_free(grid->g);
     delete grid;

@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
 #include <string>
 
 #include <nvtx3/nvToolsExt.h>
@@ -415,4 +416,9 @@ struct nsph_grid {
     // ((x, r), (v, inv_mass); or the spheres in grid and in tree order)
     float4* mirror = nullptr;
     int mirror_cap = 0;
+    // The raycasts on this grid share its sort buffers (the tree) and bounds,
+    // whose contents depend on the camera: a call waits for the one before,
+    // whatever its stream, and enqueues as a whole, whatever its host thread.
+    std::mutex raycast_mutex;
+    cudaEvent_t raycast_done = nullptr;
 };

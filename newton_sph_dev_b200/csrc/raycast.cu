@@ -832,43 +832,11 @@ __global__ void k_clamp_no_hits(float* __restrict__ depth, int count, float max_
     if (i < count && depth[i] >= max_distance) depth[i] = -1.f;
 }
 
-}  // namespace
-}  // namespace nsph
-
-using namespace nsph;
-
-extern "C" int nsph_raycast_particles(nsph_grid* grid, const float* x, const float* radius, int n,
-                                      const nsph_raycast_camera* camera, float search_radius, float march_step,
-                                      int max_steps, float* depth, void* stream)
+// the tree and the image of one call, in stream order
+int raycast_enqueue(nsph_grid* grid, const float* x, const float* radius, int n, const nsph_raycast_camera& c,
+                    float search_radius, float march_step, int max_steps, float* depth, cudaStream_t cs)
 {
-    clear_error();
-    NvtxRange nvtx_range("nsph_raycast_particles");
-    if (!grid || !camera) return fail(NSPH_ERR_INVALID_ARG, "null grid or camera");
-    const nsph_raycast_camera& c = *camera;
-    if (c.width < 0 || c.height < 0) return fail(NSPH_ERR_INVALID_ARG, "negative image size");
-    if ((long long)c.width * c.height > 0x7fffffffLL) return fail(NSPH_ERR_INVALID_ARG, "image too large");
-    if (n < 0) return fail(NSPH_ERR_INVALID_ARG, "negative particle count");
-    if (!(march_step > 0.f)) return fail(NSPH_ERR_INVALID_ARG, "march_step must be positive");
-    if (!(search_radius > 0.f) || !isfinite(search_radius))
-        return fail(NSPH_ERR_INVALID_ARG, "search_radius must be positive and finite");
-    if (max_steps < 0 || max_steps > NSPH_RAYCAST_MAX_STEPS)
-        return fail(NSPH_ERR_INVALID_ARG, "max_steps must be in [0, NSPH_RAYCAST_MAX_STEPS]");
-    if (c.width == 0 || c.height == 0 || n == 0 || max_steps == 0) return NSPH_OK;
-    if (!x || !radius || !depth) return fail(NSPH_ERR_INVALID_ARG, "null array");
     Grid& g = grid->g;
-    if (g.world_count > 0) return fail(NSPH_ERR_INVALID_ARG, "the raycast needs a single-world grid");
-    if (!g.built || g.num_points != n)
-        return fail(NSPH_ERR_NOT_BUILT, "the grid must be built on the n particle positions first");
-    DeviceGuard guard(g.device);
-    if (!guard.ok) return fail(NSPH_ERR_CUDA, "cannot select CUDA device");
-    if (grid->mirror_cap < n) {
-        cudaFree(grid->mirror);
-        grid->mirror = nullptr;
-        grid->mirror_cap = 0;
-        NSPH_CUDA_TRY(cudaMalloc(&grid->mirror, sizeof(float4) * 2 * (size_t)g.capacity));
-        grid->mirror_cap = g.capacity;
-    }
-    cudaStream_t cs = (cudaStream_t)stream;
     float4* m = grid->mirror;
     float4* sorted = grid->mirror + grid->mirror_cap;
     unsigned* bounds = g.bounds;
@@ -914,6 +882,58 @@ extern "C" int nsph_raycast_particles(nsph_grid* grid, const float* x, const flo
                                    tiles_x, search_radius, march_step, max_steps, depth));
     NSPH_LAUNCH_CHECK("k_raycast");
     return NSPH_OK;
+}
+
+}  // namespace
+}  // namespace nsph
+
+using namespace nsph;
+
+extern "C" int nsph_raycast_particles(nsph_grid* grid, const float* x, const float* radius, int n,
+                                      const nsph_raycast_camera* camera, float search_radius, float march_step,
+                                      int max_steps, float* depth, void* stream)
+{
+    clear_error();
+    NvtxRange nvtx_range("nsph_raycast_particles");
+    if (!grid || !camera) return fail(NSPH_ERR_INVALID_ARG, "null grid or camera");
+    const nsph_raycast_camera& c = *camera;
+    if (c.width < 0 || c.height < 0) return fail(NSPH_ERR_INVALID_ARG, "negative image size");
+    if ((long long)c.width * c.height > 0x7fffffffLL) return fail(NSPH_ERR_INVALID_ARG, "image too large");
+    if (n < 0) return fail(NSPH_ERR_INVALID_ARG, "negative particle count");
+    if (!(march_step > 0.f)) return fail(NSPH_ERR_INVALID_ARG, "march_step must be positive");
+    if (!(search_radius > 0.f) || !isfinite(search_radius))
+        return fail(NSPH_ERR_INVALID_ARG, "search_radius must be positive and finite");
+    if (max_steps < 0 || max_steps > NSPH_RAYCAST_MAX_STEPS)
+        return fail(NSPH_ERR_INVALID_ARG, "max_steps must be in [0, NSPH_RAYCAST_MAX_STEPS]");
+    if (c.width == 0 || c.height == 0 || n == 0 || max_steps == 0) return NSPH_OK;
+    if (!x || !radius || !depth) return fail(NSPH_ERR_INVALID_ARG, "null array");
+    Grid& g = grid->g;
+    if (g.world_count > 0) return fail(NSPH_ERR_INVALID_ARG, "the raycast needs a single-world grid");
+    if (!g.built || g.num_points != n)
+        return fail(NSPH_ERR_NOT_BUILT, "the grid must be built on the n particle positions first");
+    DeviceGuard guard(g.device);
+    if (!guard.ok) return fail(NSPH_ERR_CUDA, "cannot select CUDA device");
+    std::lock_guard<std::mutex> lock(grid->raycast_mutex);
+    if (grid->mirror_cap < n) {
+        cudaFree(grid->mirror);
+        grid->mirror = nullptr;
+        grid->mirror_cap = 0;
+        NSPH_CUDA_TRY(cudaMalloc(&grid->mirror, sizeof(float4) * 2 * (size_t)g.capacity));
+        grid->mirror_cap = g.capacity;
+    }
+    cudaStream_t cs = (cudaStream_t)stream;
+    // (a captured call is ordered by whoever launches its graph)
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    NSPH_CUDA_TRY(cudaStreamIsCapturing(cs, &capture));
+    const bool ordered = capture == cudaStreamCaptureStatusNone;
+    if (ordered && grid->raycast_done)
+        NSPH_CUDA_TRY(cudaStreamWaitEvent(cs, grid->raycast_done, 0));
+    else if (ordered)
+        NSPH_CUDA_TRY(cudaEventCreateWithFlags(&grid->raycast_done, cudaEventDisableTiming));
+    const int st = raycast_enqueue(grid, x, radius, n, c, search_radius, march_step, max_steps, depth, cs);
+    // (also behind a call that failed half way)
+    if (ordered) NSPH_CUDA_TRY(cudaEventRecord(grid->raycast_done, cs));
+    return st;
 }
 
 extern "C" int nsph_raycast_clamp_no_hits(float* depth, int count, float max_distance, void* stream)
