@@ -331,7 +331,9 @@ __device__ __forceinline__ int group_item(const int4& gr, int u)
 // register (no per-item select, as a reader returning one item at a time
 // needs) and the visits' loads can issue together. kReadOnly: the list was
 // written by an earlier kernel (read-only path); otherwise it is read back by
-// the thread that wrote it (plain loads).
+// the thread that wrote it (plain loads). (The items stay a function of their
+// own: written into the loop, the compiler contracts the surrogate's feature
+// sums another way, and its outputs differ in the last place of a feature.)
 template <bool kReadOnly, class F>
 __device__ __forceinline__ void for_each_listed(const int4* __restrict__ nbr, int n, int k, int cnt, F&& visit)
 {
@@ -344,13 +346,14 @@ __device__ __forceinline__ void for_each_listed(const int4* __restrict__ nbr, in
         const int4 gr = cur;
         cur = nxt;
         if (t + 8 < cnt) nxt = load((t >> 2) + 2);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        auto item = [&](int u) {
             if (t + u < cnt) {
                 const int j = group_item(gr, u);
                 visit(in_bounds(j >= 0 && j < n) ? j : 0);
             }
-        }
+        };
+#pragma unroll
+        for (int u = 0; u < 4; ++u) item(u);
     }
 }
 
