@@ -406,18 +406,18 @@ __device__ __noinline__ int scan_general(const GridDev* g, const float4* xs, con
 // into fp16 hi + lo parts along K). The sign of r2 - T marks a possible
 // neighbour: T exceeds 1 by a bound on the rounding errors, so no neighbour is
 // missed. (fp16 sums, of which only half precision is specified, would save 3 of
-// the 434 us of the 1M tank's step.) A chunk's marks (one 32-bit word per particle) wait in
-// shared memory; then each lane walks its own marks in order, repeats the
-// exact fp32 test of the definition, sums rho and appends to the list. Sets,
-// order and every rounding are therefore those of the general scan.
+// the 434 us of the 1M tank's step.) A chunk's marks (one 32-bit word per
+// particle) wait in shared memory; then each lane walks its own marks in order,
+// repeats the exact fp32 test of the definition, sums rho and appends to the
+// list. Sets, order and every rounding are therefore those of the general scan.
 //
 // Why: per particle about 216 candidates are tested for 30 neighbours. One
 // thread per particle spent three quarters of its 211 warp instructions per
 // particle on the tests and the traversal; a chunk of 1,024 tests costs about
-// 75 warp instructions, 24 of them the matrix part, and the traversal is done
-// once per group. The 1M tank's pass went from 0.291 to 0.243 ms (166 warp
-// instructions per particle, 75% issue active), the 128^3 block's from 0.563
-// to 0.47. What bounds it now is the walk: some 70 instructions for each of a
+// 75 warp instructions, a third of them the matrix part, and the traversal is
+// done once per group. The 1M tank's pass went from 0.291 to 0.246 ms (160 warp
+// instructions per particle, 78% issue active), the 128^3 block's from 0.563
+// to 0.48. What bounds it now is the walk: some 70 instructions for each of a
 // warp's 38 steps. The tiles are 32 x 32 with K = 8 and live in one warp's
 // registers: tcgen05's 128-row tiles would span 16 cells, of whose joint
 // stencil a particle uses a sixth. 64 registers; 48 (five blocks per SM) were
